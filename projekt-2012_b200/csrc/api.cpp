@@ -319,20 +319,32 @@ struct BlockIo {
     int2 *bottom = nullptr, *right = nullptr;
 };
 
+// Words of the control buffer: error, abort, best H, spare; the byte bitmap.
+constexpr int kErrWords = 12;
+
 int run_stage1(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_cols, int64_t n,
                const swb_scoring *sc, uint32_t flags, int64_t sr_interval_rows, int64_t sc_interval,
-               swb::BestRec *best_out, float *ms_out, int64_t *nsr_out, const BlockIo *blk = nullptr) {
+               swb::BestRec *best_out, float *ms_out, int64_t *nsr_out, const BlockIo *blk = nullptr,
+               bool wide = false) {
     using namespace swb;
     cudaError_t e;
-    // TAB mode when the column sequence has at most four distinct bytes and the
-    // shifted scores fit a signed byte
-    bool tab = false;
-    uint8_t lut[256];
+    const int64_t sr_asked = sr_interval_rows;
     c->last_launches = 2;  // wavefront + best-cell reduction
     const int32_t mt1 = sc->match - sc->gap_open, mm1 = sc->mismatch - sc->gap_open;
-    if (mt1 >= -128 && mt1 <= 127 && mm1 >= -128 && mm1 <= 127 && !std::getenv("SWB_STAGE1_CMP")) {
+    // strips in packed 16-bit lanes unless the scoring is too wide for their window
+    // (wide: a window did not hold in a first run)
+    const char *pack_env = std::getenv("SWB_STAGE1_PACK");
+    bool packed = !wide && strip16_fits(*sc, 32, n) && !(pack_env && pack_env[0] == '0');
+    if (blk && n < 256) packed = false;  // E of the right border: packed strips start it from open, see run_strip2
+    // TAB mode of the 32-bit strips when the column sequence has at most four
+    // distinct bytes and the shifted scores fit a signed byte (packed strips
+    // decide on the device, see prepare_kernel)
+    bool tab = packed;
+    uint8_t lut[256];
+    const bool compare = std::getenv("SWB_STAGE1_CMP") != nullptr;
+    if (!packed && mt1 >= -128 && mt1 <= 127 && mm1 >= -128 && mm1 <= 127 && !compare) {
         uint32_t present[256];
-        if ((e = c->flags.ensure(256 * sizeof(uint32_t))) != cudaSuccess ||
+        if ((e = c->flags.ensure(sizeof present)) != cudaSuccess ||
             (e = stage1_presence(d_cols, n, (uint32_t *)c->flags.p, c->stream)) != cudaSuccess ||
             (e = swb::ctx_get(c, present, c->flags.p, sizeof present)) != cudaSuccess)
             return ctx_cuda_fail(c, e, "column alphabet");
@@ -343,7 +355,7 @@ int run_stage1(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_co
     }
     if ((e = c->hbuf.ensure(sizeof(int4) * (size_t)std::max<int64_t>(n, 1))) != cudaSuccess ||
         (e = c->best.ensure(sizeof(BestRec))) != cudaSuccess ||
-        (e = c->errf.ensure(4 * sizeof(int32_t))) != cudaSuccess)
+        (e = c->errf.ensure(kErrWords * sizeof(int32_t))) != cudaSuccess)
         return ctx_cuda_fail(c, e, "stage 1 buffers");
 
     Stage1Args a{};
@@ -356,7 +368,21 @@ int run_stage1(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_co
     a.gx = std::max(sc->gap_open, sc->gap_extend);
     a.mt1 = mt1;
     a.mm1 = mm1;
-    if (tab) {
+    if (packed) {
+        if ((e = c->rcode.ensure((size_t)m + 64)) != cudaSuccess ||
+            (e = c->ctab.ensure(sizeof(uint32_t) * ((size_t)n + 64))) != cudaSuccess)
+            return ctx_cuda_fail(c, e, "stage 1 buffers");
+        a.rcode = (const uint8_t *)c->rcode.p;
+        a.ctab = (const uint32_t *)c->ctab.p;
+        a.present = (const uint32_t *)c->errf.p + 4;
+        // control words and bitmap (all bytes "occur": the compare scores)
+        if ((e = cudaMemsetAsync(c->errf.p, 0, kErrWords * sizeof(int32_t), c->stream)) != cudaSuccess ||
+            (compare && (e = cudaMemsetAsync((uint32_t *)c->errf.p + 4, 0xFF, 32, c->stream)) != cudaSuccess) ||
+            (e = stage1_prepare(d_rows, m, d_cols, n, (uint8_t *)c->rcode.p, (uint32_t *)c->ctab.p, mt1, mm1,
+                                (uint32_t *)c->errf.p + 4, (int4 *)c->hbuf.p, c->stream)) != cudaSuccess)
+            return ctx_cuda_fail(c, e, "stage 1 prepare");
+        c->last_launches += 1;
+    } else if (tab) {
         if ((e = c->lut.ensure(256)) != cudaSuccess || (e = c->rcode.ensure((size_t)m + 64)) != cudaSuccess ||
             (e = c->ctab.ensure(sizeof(uint32_t) * ((size_t)n + 64))) != cudaSuccess ||
             (e = swb::ctx_put(c, c->lut.p, lut, 256)) != cudaSuccess ||
@@ -390,22 +416,24 @@ int run_stage1(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_co
         a.right = blk->right;
     }
 
-    // rows per lane: an override, else the autotuner.  Strips must tile the
-    // special-row spacing when special rows are kept; sr_interval_rows < 0 asks
-    // for a special row at every strip bottom with the strip height left to the
-    // tuner (448 or 512 rows: the walker's block grid follows it).
+    // rows per lane: an override, else the autotuner.  Strips (packed: half strips)
+    // must tile the special-row spacing when special rows are kept;
+    // sr_interval_rows < 0 asks for special rows every 448 or 512 rows, whichever
+    // suits the strip height (the walker's block grid follows it).
     const bool strip_rows = sr_interval_rows < 0;
     const bool stores = sr_interval_rows != 0 || sc_interval > 0;
+    bool probed = false;  // the autotuner ran launches of its own
     int R = 16;
     if (blk && blk->bottom) R = 16;  // the last row must be a strip bottom: 512-row strips
     else if (const char *rv = std::getenv("SWB_STAGE1_R")) R = std::atoi(rv);  // override: 8, 14, 16 or 32
-    else R = autotune_rows_per_lane(c, a, tab, stores, 16, strip_rows, sr_interval_rows > 0 ? sr_interval_rows : 0);
+    else R = autotune_rows_per_lane(c, a, tab, stores, packed, 16, strip_rows, sr_interval_rows > 0 ? sr_interval_rows : 0, &probed);
+    if (R != 8 && R != 14 && R != 16 && R != 32) R = 16;
     if (strip_rows) {
-        if (R != 14 && R != 16) R = 16;
-        sr_interval_rows = 32LL * R;
+        if (!packed && R != 14) R = 16;
+        sr_interval_rows = R == 14 ? 448 : 512;
     }
-    if (sr_interval_rows > 0 && (R > 16 || sr_interval_rows % (32 * R) != 0)) R = 16;
-    Stage1Plan plan = stage1_plan(m, n, c->sms, R, tab);
+    if (sr_interval_rows > 0 && ((!packed && R > 16) || sr_interval_rows % (packed ? 16 * R : 32 * R) != 0)) R = 16;
+    Stage1Plan plan = stage1_plan(m, n, c->sms, R, tab, packed);
     if (c->max_blocks > 0 && plan.blocks > c->max_blocks) plan.blocks = c->max_blocks;
     const int64_t W = (int64_t)plan.blocks * plan.warps_per_block;
     if ((e = c->wbest.ensure(sizeof(BestRec) * (size_t)W)) != cudaSuccess)
@@ -426,9 +454,13 @@ int run_stage1(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_co
     a.sc_every = 1 << 30;
     a.nsc = 0;
     size_t sbytes = 0;
+    int64_t sr_rows = 0;  // rows between special rows
     if (sr_interval_rows > 0) {
-        const int64_t every = std::max<int64_t>(1, sr_interval_rows / plan.strip_rows);
-        const int64_t nsr = (m / plan.strip_rows) / every;
+        const int64_t unit = packed ? plan.strip_rows / 2 : plan.strip_rows;
+        int64_t every = std::max<int64_t>(1, sr_interval_rows / unit);
+        if (sr_interval_rows % unit != 0) every = std::max<int64_t>(1, sr_interval_rows / 512) * (512 / unit);
+        const int64_t nsr = m / (unit * every);
+        sr_rows = unit * every;
         sbytes += sizeof(int2) * (size_t)nsr * (size_t)n;
         if (nsr > 0) {
             a.sr_every = every;
@@ -475,11 +507,11 @@ int run_stage1(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_co
     c->last_scols = a.scols;
     c->last_nsr = a.nsr;
     c->last_n = n;
-    c->last_sr_interval = a.nsr > 0 ? a.sr_every * plan.strip_rows : 0;
+    c->last_sr_interval = a.nsr > 0 ? sr_rows : 0;
     if (nsr_out) *nsr_out = a.nsr;
 
-    if ((e = cudaMemsetAsync(a.hbuf, 0xFF, sizeof(int4) * (size_t)n, c->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(a.err, 0, 4 * sizeof(int32_t), c->stream)) != cudaSuccess)
+    if ((!packed || probed) && ((e = cudaMemsetAsync(a.hbuf, 0xFF, sizeof(int4) * (size_t)n, c->stream)) != cudaSuccess ||
+                                (e = cudaMemsetAsync(a.err, 0, 4 * sizeof(int32_t), c->stream)) != cudaSuccess))
         return ctx_cuda_fail(c, e, "stage 1 reset");
     a.withhold = (flags & SWB_FLAG_TEST_WITHHOLD) ? 1 : 0;  // set after the autotuner's probes
     cudaEventRecord(c->ev0, c->stream);
@@ -489,6 +521,8 @@ int run_stage1(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_co
     if ((e = swb::ctx_get(c, best_out, a.best, sizeof(BestRec))) != cudaSuccess ||
         (e = swb::ctx_get(c, errh, a.err, sizeof errh)) != cudaSuccess)
         return ctx_cuda_fail(c, e, "stage 1");
+    if (errh[0] == kStage1Range)  // a 16-bit window did not hold: the same pass in 32-bit strips
+        return run_stage1(c, d_rows, m, d_cols, n, sc, flags, sr_asked, sc_interval, best_out, ms_out, nsr_out, blk, true);
     if (errh[0] != 0) return ctx_fail(c, SWB_ETIMEOUT, "stage 1: a bounded wait between strips ran out");
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);

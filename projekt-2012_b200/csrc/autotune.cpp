@@ -101,8 +101,18 @@ void tune_record(const std::string &key, int R) {
     store_locked(key, R);
 }
 
-int autotune_rows_per_lane(swb_ctx *c, const Stage1Args &base, bool tab, bool stores, int fallback,
-                           bool strip_rows, int64_t sr_interval) {
+int autotune_rows_per_lane(swb_ctx *c, const Stage1Args &base, bool tab, bool stores, bool packed, int fallback,
+                           bool strip_rows, int64_t sr_interval, bool *probed) {
+    // Packed strips (strip16.cuh).  While every 256-row strip has a scheduler to
+    // itself the strips' latency decides, and the lowest strips are fastest (90 kbp
+    // pair, store pass: 9.8 ms with 256 rows, 10.8 with 448, 11.3 with 512, 17.1 with
+    // 1024); beyond that their fill does, and 448 rows are (172 kbp: 26.8, 20.6, 21.3,
+    // 32.6 ms; 1 Mbp: 341, 298, 322, 323 ms; score only 287, 263, 285, 285 ms).
+    if (packed) {
+        fallback = base.m <= 256LL * 4 * std::max(1, c->sms) ? 8 : 14;
+        if (sr_interval > 0 && sr_interval % (16 * fallback) != 0) fallback = 16;
+        if (stores) return fallback;
+    }
     // pairs below this many cells are not worth a probe
     constexpr double kMinCells = 2e10;
     if ((double)base.m * (double)base.n < kMinCells) return fallback;
@@ -133,7 +143,7 @@ int autotune_rows_per_lane(swb_ctx *c, const Stage1Args &base, bool tab, bool st
         // pair 627 vs 667 ms (fill 0.94 vs 0.82), 10 Mbp pair 46.2 vs 45.7 s
         // (fill 0.94 vs 0.92).
         auto fill = [&](int R) {
-            const int per_sm = stage1_max_blocks_per_sm(R, tab);
+            const int per_sm = stage1_max_blocks_per_sm(R, tab, packed);
             const double slots = (double)std::max(1, c->sms) * std::max(1, per_sm) * 4;
             const double strips = std::ceil((double)base.m / (32.0 * R));
             return strips / (std::ceil(strips / slots) * slots);
@@ -145,10 +155,11 @@ int autotune_rows_per_lane(swb_ctx *c, const Stage1Args &base, bool tab, bool st
         if (has14) return 14;
     }
     const int64_t np = std::min<int64_t>(base.n, 1 << 18);
+    if (probed) *probed = true;
     int bestR = fallback;
     float bestMs = 1e30f;
     for (int R : cands) {
-        Stage1Plan p = stage1_plan(base.m, np, c->sms, R, tab);
+        Stage1Plan p = stage1_plan(base.m, np, c->sms, R, tab, packed);
         p.stores = stores;
         if (c->max_blocks > 0 && p.blocks > c->max_blocks) p.blocks = c->max_blocks;
         const int64_t W = (int64_t)p.blocks * p.warps_per_block;

@@ -114,7 +114,7 @@ extern "C" int swb_score_pair_noalloc(int32_t device, const void *d_rows, int64_
     int sms = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
         return noalloc_fail(SWB_ECUDA, cudaGetErrorString(e));
-    Stage1Plan plan = stage1_plan(rows, cols, sms, 16, false);
+    Stage1Plan plan = stage1_plan(rows, cols, sms, 16, false, false);
     if ((int64_t)plan.blocks * plan.warps_per_block > kMaxWarps) plan.blocks = (int)(kMaxWarps / plan.warps_per_block);
 
     Stage1Args a{};

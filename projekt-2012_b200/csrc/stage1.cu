@@ -45,6 +45,7 @@
 #include <climits>
 
 #include "stage1_core.cuh"
+#include "strip16.cuh"
 
 namespace swb {
 
@@ -107,6 +108,88 @@ __global__ void __launch_bounds__(kWarps * 32, (R <= 16 ? 4 : 2)) stage1_kernel(
     }
 }
 
+// Whether the bytes of a bitmap (8 words) have different codes (byte >> 1) & 3: the
+// letters ACGT do, in either case.  Then the table encodings that prepare_kernel
+// writes with that code tell them apart.
+__device__ __forceinline__ bool codes_differ(const uint32_t *present, int lane) {
+    const uint32_t w = lane < 8 ? present[lane] : 0u;
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) ok &= __reduce_add_sync(0xffffffffu, (unsigned)__popc(w & (0x03030303u << (2 * c)))) <= 1;
+    return ok;
+}
+
+// Before a packed launch, in one pass over the sequences: the table encodings of
+// both, the bitmap of the bytes that occur (zeroed by the caller) and the hand-off
+// entries' reset.
+__global__ void prepare_kernel(const uint8_t *rows, int64_t m, const uint8_t *cols, int64_t n, uint8_t *rcode,
+                               uint32_t *ctab, uint32_t mm4, uint32_t x1, uint32_t *present, int4 *hbuf) {
+    __shared__ uint32_t sh[8];
+    if (threadIdx.x < 8) sh[threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    // few distinct bytes: an atomic only for one that is not in the block's bitmap yet
+    auto see = [&](uint32_t b) {
+        if (!((*(volatile uint32_t *)&sh[b >> 5] >> (b & 31)) & 1u)) atomicOr(&sh[b >> 5], 1u << (b & 31));
+    };
+    for (int64_t i = tid; i < m; i += stride) {
+        const uint32_t b = rows[i];
+        rcode[i] = (uint8_t)((b >> 1) & 3u);
+        see(b);
+    }
+    for (int64_t i = tid; i < n; i += stride) {
+        const uint32_t b = cols[i];
+        ctab[i] = mm4 ^ (x1 << (8 * ((b >> 1) & 3u)));
+        hbuf[i] = make_int4(-1, -1, -1, -1);
+        see(b);
+    }
+    __syncthreads();
+    if (threadIdx.x < 8 && sh[threadIdx.x]) atomicOr(&present[threadIdx.x], sh[threadIdx.x]);
+}
+
+// The same launch with strips in packed 16-bit lanes (strip16.cuh): 2 RH rows per
+// lane, strips of 64 RH rows.  Table or compare scores by the bytes that occur.
+template <int RH, bool STORES>
+__global__ void __launch_bounds__(kWarps * 32, 4) stage1_packed_kernel(Stage1Args a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31;
+    const int wib = threadIdx.x >> 5;
+    WarpMem<RH> *w = reinterpret_cast<WarpMem<RH> *>(smem) + wib;
+    const int64_t B = gridDim.x;
+    init_warp(w, lane, a.open);
+    const bool tab = codes_differ(a.present, lane);
+    int32_t rc = kErrNone;
+    for (int64_t round = 0; rc == kErrNone; ++round) {
+        const int64_t s = blockIdx.x + B * (wib + kWarps * round);
+        if (s >= a.nstrips) break;
+        if (a.trace && lane == 0) {
+            uint32_t smid;
+            asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+            a.trace[3 * s + 2] = (int64_t)smid;
+        }
+        rc = tab ? run_strip2<RH, true, STORES>(a, w, lane, (int32_t)s) : run_strip2<RH, false, STORES>(a, w, lane, (int32_t)s);
+        if (a.trace && lane == 0) {
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            a.trace[3 * s + 1] = (int64_t)t;
+        }
+    }
+    if (lane == 0) {
+        if (rc != kErrNone) {
+            atomicCAS(&a.err[0], kErrNone, rc);
+            atomicExch(&a.err[1], 1);
+        }
+        BestRec r;
+        r.ho = w->best_ho;
+        r.valid = w->best_valid;
+        r.key = w->best_key;
+        r.row = w->best_row;
+        r.col = w->best_col;
+        a.wbest[(int64_t)blockIdx.x * kWarps + wib] = r;
+    }
+}
+
 __global__ void reduce_best_kernel(const BestRec *in, int64_t count, BestRec *out) {
     __shared__ BestRec sh[256];
     BestRec b;
@@ -156,25 +239,33 @@ __global__ void presence_kernel(const uint8_t *seq, int64_t n, uint32_t *flags) 
         if (sh[i]) flags[i] = 1;
 }
 
-template <int R, bool TAB>
-cudaError_t launch_r(Stage1Args &a, const Stage1Plan &p, cudaStream_t st) {
-    void *args[] = {&a};
-    const void *fn = (p.stores || a.srows || a.scols) ? (const void *)stage1_kernel<R, TAB, true>
-                                                      : (const void *)stage1_kernel<R, TAB, false>;
-    cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(p.blocks), dim3(kWarps * 32), args, 0, st);
-    if (e != cudaSuccess) return e;
-    reduce_best_kernel<<<1, 256, 0, st>>>(a.wbest, (int64_t)p.blocks * kWarps, a.best);
-    return cudaGetLastError();
+// Calls f with the kernel of a plan, its dynamic shared memory and whether it is
+// instantiated.
+struct KernelRef {
+    const void *fn = nullptr;
+    size_t smem = 0;
+};
+template <int R, bool TAB, bool STORES>
+KernelRef wide_ref() {
+    return {(const void *)stage1_kernel<R, TAB, STORES>, 0};
 }
-
-template <int R, bool TAB>
-int max_blocks_r() {
-    int nb = 0, ns = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stage1_kernel<R, TAB, false>, kWarps * 32, 0) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ns, stage1_kernel<R, TAB, true>, kWarps * 32, 0) != cudaSuccess)
-        return 0;
-    return nb < ns ? nb : ns;
+template <int R, bool STORES>
+KernelRef packed_ref() {
+    return {(const void *)stage1_packed_kernel<R / 2, STORES>, kWarps * sizeof(WarpMem<R / 2>)};
+}
+template <bool TAB, bool STORES>
+KernelRef kernel_ref(int R, bool packed) {
+    switch (R) {
+        case 8: return packed ? packed_ref<8, STORES>() : wide_ref<8, TAB, STORES>();
+        case 14: return packed ? packed_ref<14, STORES>() : wide_ref<14, TAB, STORES>();
+        case 16: return packed ? packed_ref<16, STORES>() : wide_ref<16, TAB, STORES>();
+        case 32: return packed ? packed_ref<32, STORES>() : wide_ref<32, TAB, STORES>();
+        default: return {};
+    }
+}
+KernelRef kernel_of(int R, bool tab, bool stores, bool packed) {
+    if (tab) return stores ? kernel_ref<true, true>(R, packed) : kernel_ref<true, false>(R, packed);
+    return stores ? kernel_ref<false, true>(R, packed) : kernel_ref<false, false>(R, packed);
 }
 
 }  // namespace
@@ -188,47 +279,55 @@ cudaError_t stage1_configure() {
     const int c = cudaSharedmemCarveoutMaxShared;
     const auto A = cudaFuncAttributePreferredSharedMemoryCarveout;
     cudaError_t e = cudaSuccess;
-    for (cudaError_t x : {cudaFuncSetAttribute((const void *)stage1_kernel<8, false, false>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<8, true, false>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<14, false, false>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<14, true, false>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<14, false, true>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<14, true, true>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<16, false, false>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<16, true, false>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<32, false, false>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<32, true, false>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<8, false, true>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<8, true, true>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<16, false, true>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<16, true, true>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<32, false, true>, A, c),
-                          cudaFuncSetAttribute((const void *)stage1_kernel<32, true, true>, A, c),
-                          cudaFuncSetAttribute((const void *)reduce_best_kernel, A, c),
+    for (int R : {8, 14, 16, 32})
+        for (int v = 0; v < 8; ++v) {
+            const KernelRef k = kernel_of(R, v & 1, v & 2, v & 4);
+            cudaError_t x = cudaFuncSetAttribute(k.fn, A, c);
+            if (x == cudaSuccess && k.smem > 0)
+                x = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+            if (x != cudaSuccess) e = x;
+        }
+    for (cudaError_t x : {cudaFuncSetAttribute((const void *)reduce_best_kernel, A, c),
                           cudaFuncSetAttribute((const void *)encode_kernel, A, c),
+                          cudaFuncSetAttribute((const void *)prepare_kernel, A, c),
                           cudaFuncSetAttribute((const void *)presence_kernel, A, c)})
         if (x != cudaSuccess) e = x;
     return e;
 }
 
-int stage1_max_blocks_per_sm(int R, bool tab) {
-    switch (R) {
-        case 8: return tab ? max_blocks_r<8, true>() : max_blocks_r<8, false>();
-        case 14: return tab ? max_blocks_r<14, true>() : max_blocks_r<14, false>();
-        case 16: return tab ? max_blocks_r<16, true>() : max_blocks_r<16, false>();
-        case 32: return tab ? max_blocks_r<32, true>() : max_blocks_r<32, false>();
-        default: return 0;
+int stage1_max_blocks_per_sm(int R, bool tab, bool packed) {
+    int least = INT_MAX;
+    for (bool stores : {false, true}) {
+        const KernelRef k = kernel_of(R, tab, stores, packed);
+        int nb = 0;
+        if (!k.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn, kWarps * 32, k.smem) != cudaSuccess)
+            return 0;
+        least = std::min(least, nb);
     }
+    return least;
 }
 
-Stage1Plan stage1_plan(int64_t m, int64_t n, int device_sms, int R_hint, bool tab) {
+bool strip16_fits(const swb_scoring &sc, int R, int64_t n) {
+    const int64_t e = std::min(-(int64_t)sc.gap_open, -(int64_t)sc.gap_extend);
+    const int64_t slope = sc.match + e, open = -(int64_t)sc.gap_open;
+    const int64_t mt1 = (int64_t)sc.match + open, mm1 = (int64_t)sc.mismatch + open;
+    // the spread over a warp, the window's margin (window2) and the range of single
+    // scores; half of the window is left for the base to move in.  The step
+    // counter runs to n + 63 and looks two runs of 32 ahead.
+    return (32LL * R + 160) * slope + 2 * open <= 20000 && (R + 96) * slope + 6 * open + 64 <= 6000 &&
+           mt1 - mm1 <= 64 && mt1 <= 127 && mm1 >= -128 && sc.gap_extend >= -1000 && open <= 127 &&
+           n <= (int64_t)INT32_MAX - 256;
+}
+
+Stage1Plan stage1_plan(int64_t m, int64_t n, int device_sms, int R_hint, bool tab, bool packed) {
     Stage1Plan p;
     p.R = (R_hint == 8 || R_hint == 14 || R_hint == 16 || R_hint == 32) ? R_hint : 16;
     p.tab = tab;
+    p.packed = packed;
     p.warps_per_block = kWarps;
     p.strip_rows = 32LL * p.R;
     p.nstrips = (m + p.strip_rows - 1) / p.strip_rows;
-    const int per_sm = stage1_max_blocks_per_sm(p.R, tab);
+    const int per_sm = stage1_max_blocks_per_sm(p.R, tab, packed);
     const int64_t max_blocks = (int64_t)device_sms * (per_sm > 0 ? per_sm : 1);
     // enough blocks that every strip of the first round has a warp, spread over
     // whole multiples of the SM count when there is room
@@ -242,22 +341,13 @@ Stage1Plan stage1_plan(int64_t m, int64_t n, int device_sms, int R_hint, bool ta
 }
 
 cudaError_t stage1_launch(Stage1Args &a, const Stage1Plan &p, cudaStream_t st) {
-    if (p.tab) {
-        switch (p.R) {
-            case 8: return launch_r<8, true>(a, p, st);
-            case 14: return launch_r<14, true>(a, p, st);
-            case 16: return launch_r<16, true>(a, p, st);
-            case 32: return launch_r<32, true>(a, p, st);
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    switch (p.R) {
-        case 8: return launch_r<8, false>(a, p, st);
-        case 14: return launch_r<14, false>(a, p, st);
-        case 16: return launch_r<16, false>(a, p, st);
-        case 32: return launch_r<32, false>(a, p, st);
-        default: return cudaErrorInvalidValue;
-    }
+    const KernelRef k = kernel_of(p.R, p.tab, p.stores || a.srows || a.scols || (p.packed && (a.bottom || a.right || a.left)), p.packed);
+    if (!k.fn) return cudaErrorInvalidValue;
+    void *args[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel(k.fn, dim3(p.blocks), dim3(kWarps * 32), args, k.smem, st);
+    if (e != cudaSuccess) return e;
+    reduce_best_kernel<<<1, 256, 0, st>>>(a.wbest, (int64_t)p.blocks * kWarps, a.best);
+    return cudaGetLastError();
 }
 
 cudaError_t stage1_presence(const uint8_t *seq, int64_t n, uint32_t *flags, cudaStream_t st) {
@@ -265,6 +355,15 @@ cudaError_t stage1_presence(const uint8_t *seq, int64_t n, uint32_t *flags, cuda
     if (e != cudaSuccess || n <= 0) return e;
     int blocks = (int)std::min<int64_t>(1024, (n + 255) / 256);
     presence_kernel<<<blocks, 256, 0, st>>>(seq, n, flags);
+    return cudaGetLastError();
+}
+
+cudaError_t stage1_prepare(const uint8_t *rows, int64_t m, const uint8_t *cols, int64_t n, uint8_t *rcode, uint32_t *ctab,
+                           int32_t mt1, int32_t mm1, uint32_t *present, int4 *hbuf, cudaStream_t st) {
+    const uint32_t mmb = (uint32_t)(uint8_t)(int8_t)mm1;
+    const uint32_t x1 = ((uint32_t)(uint8_t)(int8_t)mt1 ^ mmb) & 0xFFu;
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(2048, (std::max(m, n) + 255) / 256));
+    prepare_kernel<<<blocks, 256, 0, st>>>(rows, m, cols, n, rcode, ctab, mmb * 0x01010101u, x1, present, hbuf);
     return cudaGetLastError();
 }
 

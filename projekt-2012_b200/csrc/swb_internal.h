@@ -44,10 +44,11 @@ struct Stage1Args {
     int32_t mt1, mm1;      // match - open, mismatch - open
     const uint8_t *rcode;  // TAB mode: per-row code (0..3, 7 = matches nothing)
     const uint32_t *ctab;  // TAB mode: per-column word of (s - open) bytes for codes 0..3
+    const uint32_t *present; // packed strips: bitmap of the bytes that occur in rows and cols (8 words)
     uint32_t tab_hi;       // TAB mode: (mismatch - open) in all four bytes (codes 4..7)
     int4 *hbuf;            // n entries {H + open, tag, F of the next row, tag}; 0xFF-filled per launch
     int2 *srows;           // special rows [nsr][n] of (H, F), or nullptr
-    int64_t sr_every;      // a special row every sr_every strips
+    int64_t sr_every;      // a special row every sr_every strips (packed strips: half strips)
     int64_t nsr;           // number of special rows
     int2 *scols;           // special columns [nsc][m] of (H, E), or nullptr
     int32_t sc_every;      // a special column every sc_every columns (power of two)
@@ -74,9 +75,13 @@ struct Stage1Args {
 bool reference_geometry(int64_t rows, int64_t cols, int32_t *G, int32_t *T, int64_t *P1,
                         int64_t *P2);
 
+// Error code of a launch whose 16-bit window did not hold (kErrRange of strip16.cuh).
+constexpr int32_t kStage1Range = 16;
+
 // Stage-1 launch plan (chosen by the host for a pair).
 struct Stage1Plan {
-    bool tab = false;      // PRMT table substitution (column alphabet of <= 4 bytes)
+    bool tab = false;      // PRMT table substitution (column alphabet of <= 4 bytes); packed: decided on the device
+    bool packed = false;   // strips in packed 16-bit lanes (strip16.cuh)
     bool stores = false;   // run the store-mode kernel even without store buffers (autotuner probes)
     int R = 16;            // rows per lane
     int warps_per_block = 4;
@@ -90,10 +95,17 @@ struct Stage1Plan {
 // error (cudaSuccess on success); a bounded-wait timeout is reported through
 // a.err and *timed_out.
 cudaError_t stage1_launch(Stage1Args &a, const Stage1Plan &plan, cudaStream_t st);
-Stage1Plan stage1_plan(int64_t m, int64_t n, int device_sms, int R_hint, bool tab);
-int stage1_max_blocks_per_sm(int R, bool tab);
+Stage1Plan stage1_plan(int64_t m, int64_t n, int device_sms, int R_hint, bool tab, bool packed);
+int stage1_max_blocks_per_sm(int R, bool tab, bool packed);
+// Whether a strip of 32 R rows fits the 16-bit window of packed strips for this
+// scoring (the spread bound of strip16.cuh) and the compare path's score range.
+bool strip16_fits(const swb_scoring &sc, int R, int64_t n);
 // 256 presence flags of the bytes of seq (device), for choosing TAB mode.
 cudaError_t stage1_presence(const uint8_t *seq, int64_t n, uint32_t *flags, cudaStream_t st);
+// Before a packed launch: rcode[m], ctab[n] (code (byte >> 1) & 3), the bitmap of
+// the bytes that occur (8 words, zero before) and the reset of hbuf[n].
+cudaError_t stage1_prepare(const uint8_t *rows, int64_t m, const uint8_t *cols, int64_t n, uint8_t *rcode, uint32_t *ctab,
+                           int32_t mt1, int32_t mm1, uint32_t *present, int4 *hbuf, cudaStream_t st);
 // TAB-mode encodings: rcode[m] and ctab[n] from a device byte->code table.
 cudaError_t stage1_encode(const uint8_t *rows, int64_t m, const uint8_t *cols, int64_t n, const uint8_t *d_lut,
                           uint8_t *rcode, uint32_t *ctab, int32_t mt1, int32_t mm1, uint32_t *tab_hi,
