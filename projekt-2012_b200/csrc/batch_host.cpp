@@ -603,14 +603,14 @@ size_t pow2_at_least(size_t x) {
     return p;
 }
 
-// The instantiated graph for a shape (traced or not, rows per lane, grid cap,
-// size class: grids sized for at most 2^size_class work units and pairs),
+// The instantiated graph for a shape (traced or not, wide block recomputes, rows per
+// lane, grid cap, size class: grids sized for at most 2^size_class work units and pairs),
 // captured on first use.  Its kernels read the call header at c->g_hdr.p, so the
 // graph never changes for a shape; the scoring kernels' parameters are set per
 // replay (graph_set_scoring).
-cudaError_t graph_for(swb_ctx *c, bool traced, int R, int cap, int size_class, swb_ctx::GraphEntry **out) {
+cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, int R, int cap, int size_class, swb_ctx::GraphEntry **out) {
     for (auto &g : c->graphs)
-        if (g.exec && g.traced == (int)traced && g.R == R && g.cap == cap && g.size_class == size_class) {
+        if (g.exec && g.traced == (int)traced && g.wide == (int)wide && g.R == R && g.cap == cap && g.size_class == size_class) {
             *out = &g;
             return cudaSuccess;
         }
@@ -622,7 +622,7 @@ cudaError_t graph_for(swb_ctx *c, bool traced, int R, int cap, int size_class, s
     if ((e = cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
     cudaError_t q = cudaEventRecordWithFlags(c->ev0, c->cap_stream, cudaEventRecordExternal);
     if (q == cudaSuccess) q = batch_graph_enqueue(h, traced, R, c->sms, cap, max_units, c->ev1, c->cap_stream);
-    if (q == cudaSuccess && traced) q = tb::walk_graph_enqueue(h, c->sms, max_units, c->cap_stream);
+    if (q == cudaSuccess && traced) q = tb::walk_graph_enqueue(h, wide, c->sms, max_units, c->cap_stream);
     if (q == cudaSuccess && traced) q = cudaEventRecordWithFlags(c->ev2, c->cap_stream, cudaEventRecordExternal);
     cudaGraph_t graph = nullptr;
     e = cudaStreamEndCapture(c->cap_stream, &graph);
@@ -678,6 +678,7 @@ cudaError_t graph_for(swb_ctx *c, bool traced, int R, int cap, int size_class, s
     }
     slot->args_valid = false;
     slot->traced = traced;
+    slot->wide = wide;
     slot->R = R;
     slot->cap = cap;
     slot->size_class = size_class;
@@ -870,7 +871,7 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
         size_class = std::min(size_class, full);
     }
     swb_ctx::GraphEntry *ge = nullptr;
-    if ((e = graph_for(c, traced, R, c->max_blocks, size_class, &ge)) != cudaSuccess ||
+    if ((e = graph_for(c, traced, traced && !tb::walk16_fits(*sc), R, c->max_blocks, size_class, &ge)) != cudaSuccess ||
         (e = graph_set_scoring(c, ge, g.ba)) != cudaSuccess)
         return ctx_cuda_fail(c, e, "batch graph");
     uint8_t *hout = (uint8_t *)c->h_gout.p;

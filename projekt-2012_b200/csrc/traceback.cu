@@ -14,7 +14,7 @@
 // How: stage 1 keeps special rows (H, F) at every strip bottom (every 448 or 512
 // rows, the strip height) and special columns (H, E) every 256 columns, so every
 // block of that grid (at most 512 x 256) can be recomputed from its stored
-// boundaries alone, with one direction byte per cell.
+// boundaries alone, with four direction bits per cell.
 // A block's directions do not depend on the path, so the walker of a single
 // pair (walk_region) recomputes a predicted corridor of whole blocks at once,
 // one CTA per block across the GPU (the staircase of blocks along the diagonal
@@ -23,7 +23,8 @@
 // diagonal, row or column runs) until it reaches the start or leaves the
 // corridor, where the next round predicts from.  Batches of pairs use one CTA
 // per pair that recomputes the blocks on its path on demand.  Inside a CTA the
-// block recompute is a pipeline of four warps of 128 rows each, handing rows
+// block recompute is a pipeline of two warps of 256 rows each in packed 16-bit
+// halves (four of 128 rows in 32 bits for scoring too wide for them), handing rows
 // down through shared memory with tagged 64-bit words instead of barriers.
 // Pairs whose stores would not fit the HBM budget keep a coarser grid (level 1);
 // each level-1 cell the path enters is recomputed by the stage-1 kernel on that
@@ -45,16 +46,16 @@ namespace {
 
 constexpr int kBR = 512;          // block rows (= stage-1 strip height at R = 16)
 constexpr int kBC = 256;          // block columns (= special-column spacing)
-constexpr int kThreads = 128;     // recompute threads
-constexpr int kRT = kBR / kThreads;  // rows per recompute thread (4)
+constexpr int kRW = 4;            // rows per recompute half lane
+constexpr int kWarpRows = 64 * kRW;          // rows of a recompute warp (64 virtual lanes)
+constexpr int kThreads = kBR / kWarpRows * 32;  // packed recompute threads (two warps)
+constexpr int kThreadsWide = kBR / kRW;      // 32-bit recompute threads (one per four rows)
 
-// Direction byte of a cell: where H comes from (2 bits), whether E and F extend,
-// whether the diagonal predecessor's H is 0, and whether the cell's two bases
-// match (the walk takes the path's substitution scores from it, so it needs
-// no sequence bytes).
-enum : uint8_t {
-    SRC_ZERO = 0, SRC_DIAG = 1, SRC_E = 2, SRC_F = 3, BIT_EEXT = 4, BIT_FEXT = 8, BIT_DZERO = 16, BIT_MATCH = 32
-};
+// Direction bits of a cell (a nibble).  H comes from the diagonal unless ND is set,
+// then from E unless NE is set, then from F; E and F extend unless NEX / NFX is
+// set.  A cell with H = 0 is on no path: the walk knows the path's prefix score
+// and stops at the cell whose diagonal predecessor has none left.
+enum : uint32_t { BIT_ND = 1, BIT_NE = 2, BIT_NEX = 4, BIT_NFX = 8 };
 enum : int32_t { ST_H = 0, ST_E = 1, ST_F = 2 };
 
 struct WalkArgs {
@@ -76,6 +77,7 @@ struct WalkArgs {
     int64_t xp_cap;
     int64_t *st;                   // walker state in/out: see kSt* below
     int32_t br;                    // block rows of the region's grid (the special-row spacing), <= kBR
+    int32_t wide;                  // recompute in 32 bits (walk16_fits does not hold)
 };
 
 // walker state slots
@@ -108,53 +110,75 @@ struct Stage {
     int2 top[kBC + 1];
     uint8_t rb[kBR];
     uint8_t cb[kBC];
+    uint32_t top16[kBC + 8];       // packed recompute: H | F << 16 of row R0 - 1, offsets from base
+    uint16_t col16[64 + kBC + 72]; // packed recompute: column codes, 64 entries of slack in front
 };
 
+// Loads a thread issues together (one at a time they were a chain of global round
+// trips, a sixth of a block's recompute).
+constexpr int kStageBatch = 4;
 __device__ void stage_block(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0, int64_t C1, Stage *s) {
-    const int64_t w = C1 - C0 + 1, h = R1 - R0 + 1;
-    for (int64_t j = (int64_t)threadIdx.x - 1; j < w; j += blockDim.x) {
-        s->top[j + 1] = top_hf(a, R0, C0 + j);
-        if (j >= 0) s->cb[j] = a.cols[C0 + j];
+    const int w = (int)(C1 - C0 + 1), h = (int)(R1 - R0 + 1), nt = (int)blockDim.x;
+    for (int j0 = (int)threadIdx.x - 1; j0 < w; j0 += kStageBatch * nt) {
+        int2 t[kStageBatch];
+        uint8_t b[kStageBatch];
+#pragma unroll
+        for (int q = 0; q < kStageBatch; ++q) {
+            const int j = j0 + q * nt;
+            if (j < w) {
+                t[q] = top_hf(a, R0, C0 + j);
+                b[q] = j >= 0 ? a.cols[C0 + j] : 0;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kStageBatch; ++q) {
+            const int j = j0 + q * nt;
+            if (j < w) {
+                s->top[j + 1] = t[q];
+                if (j >= 0) {
+                    s->cb[j] = b[q];
+                    s->col16[64 + j] = (uint16_t)((uint32_t)b[q] << 6);
+                }
+            }
+        }
     }
-    for (int64_t i = threadIdx.x; i < h; i += blockDim.x) s->rb[i] = a.rows[R0 + i];
+    for (int i0 = (int)threadIdx.x; i0 < h; i0 += 2 * kStageBatch * nt) {
+        uint8_t b[2 * kStageBatch];
+#pragma unroll
+        for (int q = 0; q < 2 * kStageBatch; ++q)
+            if (i0 + q * nt < h) b[q] = a.rows[R0 + i0 + q * nt];
+#pragma unroll
+        for (int q = 0; q < 2 * kStageBatch; ++q)
+            if (i0 + q * nt < h) s->rb[i0 + q * nt] = b[q];
+    }
 }
 
-// Direction bytes of one block in global memory, in the recompute's step order so
-// that every warp store is one coalesced 128-byte line: word (warp, k, lane)
-// holds rows 4t .. 4t + 3 (t = 32 warp + lane) of column k - lane.
-constexpr int kSteps = kBC + 31;
-constexpr int64_t kBlockWords = (int64_t)(kThreads / 32) * kSteps * 32;
-struct GlobalDir {
-    uint32_t *d;
-    __device__ __forceinline__ uint8_t at(int64_t i, int64_t j) const {
-        const int t = (int)(i >> 2), lane = t & 31, warp = t >> 5;
-        const int64_t k = j + lane;
-        return reinterpret_cast<const uint8_t *>(d + ((int64_t)warp * kSteps + k) * 32 + lane)[i & 3];
-    }
-    __device__ __forceinline__ void put(int t, int64_t /*j*/, int64_t k, uint32_t word) const {
-        d[((int64_t)(t >> 5) * kSteps + k) * 32 + (t & 31)] = word;
-    }
-};
-
-// The same layout in shared memory (a block's words copied in from GlobalDir).
-struct SmemDir {
-    const uint32_t *d;
-    __device__ __forceinline__ uint8_t at(int64_t i, int64_t j) const {
-        const int t = (int)(i >> 2), lane = t & 31, warp = t >> 5;
-        const int k = (int)j + lane;
-        return reinterpret_cast<const uint8_t *>(d + (warp * kSteps + k) * 32 + lane)[i & 3];
+// Direction nibbles of one block, in the recompute's step order so that every warp
+// store is one coalesced 128-byte line: word (warp, k, lane) holds rows 4v .. 4v + 3
+// of column k - v for the virtual lanes v = lane (low half) and lane + 32 (high
+// half) of the warp's 256 rows.
+constexpr int kC = 8;  // recompute steps between refills
+constexpr int kSteps = (kBC + 63 + kC - 1) / kC * kC;
+constexpr int64_t kBlockWords = (int64_t)(kBR / kWarpRows) * kSteps * 32;
+__device__ __forceinline__ int dir_index(int i, int j) {  // of the 16-bit half that holds row i, column j
+    const int v = (i >> 2) & 63, warp = i >> 8;
+    return ((warp * kSteps + j + v) * 32 + (v & 31)) * 2 + (v >> 5);
+}
+struct Dir {
+    const uint32_t *d;  // global or shared memory
+    __device__ __forceinline__ uint32_t at(int64_t i, int64_t j) const {
+        return (uint32_t)reinterpret_cast<const uint16_t *>(d)[dir_index((int)i, (int)j)] >> (4 * (i & 3));
     }
 };
-constexpr size_t kDirTileBytes = sizeof(uint32_t) * (size_t)kBlockWords;  // 146,944: a multiple of 16
+constexpr size_t kDirTileBytes = sizeof(uint32_t) * (size_t)kBlockWords;  // 81,920: a multiple of 16
 
-// Hand-off between the warps of a recompute: warp w publishes (H, F) of its last
-// row (block row 128 (w + 1) - 1) column by column in bnd[w][j] as two 64-bit
-// words {H, gen} and {F, gen}, gen being the recompute's generation; warp w + 1
-// reads them as the row above and re-reads until both tags show the current
-// generation.  A 64-bit shared access is single-copy atomic, so the tag proves its
-// value is current without any fence.
+// Hand-off between the warps of a recompute, column by column, as 64-bit words
+// {value, gen}, gen being the recompute's generation; the reader re-reads until the
+// tag shows the current generation.  A 64-bit shared access is single-copy atomic,
+// so the tag proves its value is current without any fence.  Packed recompute:
+// one boundary, H | F << 16 as offsets; 32-bit recompute: three, H and F apart.
 struct Xchg {
-    unsigned long long bnd[kThreads / 32 - 1][kBC][2];
+    unsigned long long bnd[kThreadsWide / 32 - 1][kBC][2];
     int32_t err;
     uint32_t gen;  // generations used so far by this CTA (tags start at 1; entries start at 0)
 };
@@ -162,7 +186,7 @@ struct Xchg {
 // Zeroes the hand-off tags and the generation count (once per CTA).
 __device__ void xchg_init(Xchg *x) {
     unsigned long long *p = &x->bnd[0][0][0];
-    for (int i = threadIdx.x; i < (kThreads / 32 - 1) * kBC * 2; i += blockDim.x) p[i] = 0ULL;
+    for (int i = threadIdx.x; i < (kThreadsWide / 32 - 1) * kBC * 2; i += blockDim.x) p[i] = 0ULL;
     if (threadIdx.x == 0) {
         x->err = 0;
         x->gen = 0;
@@ -173,26 +197,23 @@ __device__ void xchg_init(Xchg *x) {
 // writer is a warp of the same CTA, so this only guards against a defect.
 constexpr long long kXchgWaitCycles = 2LL * 1000 * 1000 * 1000;
 
-__device__ __forceinline__ unsigned long long pack(int32_t v, uint32_t gen) {
-    return ((unsigned long long)gen << 32) | (uint32_t)v;
+__device__ __forceinline__ unsigned long long pack(uint32_t v, uint32_t gen) {
+    return ((unsigned long long)gen << 32) | v;
 }
 __device__ __forceinline__ unsigned long long ld_shared_volatile(const unsigned long long *p) {
     return *reinterpret_cast<const volatile unsigned long long *>(p);
 }
 
-// Waits until entry j of boundary b carries generation gen; returns (H, F).  After
-// one wait ran out (x->err set) it no longer waits: the warp finishes its loop on
-// whatever values it reads and the caller discards the block.
-__device__ __forceinline__ int2 take(Xchg *x, int b, int64_t j, uint32_t gen, bool &fail) {
-    if (fail) return make_int2(0, 0);
-    unsigned long long h = ld_shared_volatile(&x->bnd[b][j][0]);
-    unsigned long long f = ld_shared_volatile(&x->bnd[b][j][1]);
-    if ((uint32_t)(h >> 32) != gen || (uint32_t)(f >> 32) != gen) {
+// Waits until *p carries generation gen and returns its value.  After one wait ran
+// out (x->err set) it no longer waits: the warp finishes its loop on whatever
+// values it reads and the caller discards the block.
+__device__ __forceinline__ uint32_t take(Xchg *x, const unsigned long long *p, uint32_t gen, bool &fail) {
+    unsigned long long v = ld_shared_volatile(p);
+    if ((uint32_t)(v >> 32) != gen && !fail) {
         const long long t0 = clock64();
         for (;;) {
-            h = ld_shared_volatile(&x->bnd[b][j][0]);
-            f = ld_shared_volatile(&x->bnd[b][j][1]);
-            if ((uint32_t)(h >> 32) == gen && (uint32_t)(f >> 32) == gen) break;
+            v = ld_shared_volatile(p);
+            if ((uint32_t)(v >> 32) == gen) break;
             if (clock64() - t0 > kXchgWaitCycles) {
                 fail = true;
                 x->err = 1;
@@ -200,27 +221,27 @@ __device__ __forceinline__ int2 take(Xchg *x, int b, int64_t j, uint32_t gen, bo
             }
         }
     }
-    return make_int2((int32_t)(uint32_t)h, (int32_t)(uint32_t)f);
+    return (uint32_t)v;
 }
 
-// Recomputes block rows [R0, R1] x cols [C0, C1] into dir.  Expects
-// stage_block() to have filled `s`, x->err zeroed, and a barrier after both;
-// `gen` must differ from every earlier recompute of this CTA.  Thread t owns
-// rows R0 + 4t .. R0 + 4t + 3: each warp is a 128-row wavefront (lane l computes
-// column k - l at step k, rows passed down by shuffles) and the four warps form
-// a pipeline through x, so no CTA barrier is needed inside the column loop.
-template <class D>
-__device__ void recompute(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0, int64_t C1, const D &dir,
-                          Xchg *x, const Stage *s, uint32_t gen) {
+// Recomputes block rows [R0, R1] x cols [C0, C1] into d in 32 bits.  Expects
+// stage_block() to have filled `s`, x->err zeroed, and a barrier after both; `gen`
+// must differ from every earlier recompute of this CTA.  Thread t owns rows
+// R0 + 4t .. R0 + 4t + 3: each warp is a 128-row wavefront (lane l computes column
+// k - l at step k, rows passed down by shuffles) and the four warps form a pipeline
+// through x, so no CTA barrier is needed inside the column loop.  For scoring whose
+// values do not fit 16 bits over a block.
+__device__ void recompute_wide(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0, int64_t C1, uint32_t *d, Xchg *x,
+                               const Stage *s, uint32_t gen) {
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
     const int64_t w = C1 - C0 + 1;
-    const int64_t r0 = R0 + (int64_t)t * kRT;  // my first row
-    if (R0 + (int64_t)warp * 32 * kRT > R1) return;  // this warp (and every warp below it) has no rows
-    int32_t Hl[kRT], El[kRT];
-    uint8_t ra[kRT];
+    const int64_t r0 = R0 + (int64_t)t * kRW;  // my first row
+    if (R0 + (int64_t)warp * 32 * kRW > R1) return;  // this warp (and every warp below it) has no rows
+    int32_t Hl[kRW], El[kRW];
+    uint8_t ra[kRW];
 #pragma unroll
-    for (int i = 0; i < kRT; ++i) {
+    for (int i = 0; i < kRW; ++i) {
         const int64_t r = r0 + i;
         if (r <= R1) {
             const int2 v = left_he(a, C0, r);
@@ -238,20 +259,22 @@ __device__ void recompute(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0,
     if (t == 0) hdiag0 = s->top[0].x;
     else hdiag0 = (r0 - 1 <= R1) ? left_he(a, C0, r0 - 1).x : 0;
     bool fail = false;
-    // warps below the first start with a few columns of slack behind the warp above
-    if (warp > 0 && lane == 0) take(x, warp - 1, w - 1 < 15 ? w - 1 : 15, gen, fail);
     __syncwarp();
     int32_t upH = 0, upF = 0;  // (H, F) from the row above at my current column
     int32_t prevUpH = hdiag0;  // H of the row above at the previous column
-    const bool publish = (lane == 31) && warp < kThreads / 32 - 1 && (r0 + kRT - 1 <= R1);
+    const bool publish = (lane == 31) && warp < kThreadsWide / 32 - 1 && (r0 + kRW - 1 <= R1);
     const int64_t steps = w + 31;
     for (int64_t k = 0; k < steps; ++k) {
         const int64_t j = k - lane;  // my column offset
         const bool act = (j >= 0 && j < w && r0 <= R1);
         if (lane == 0 && j < w) {
-            const int2 tv = (warp == 0) ? s->top[j + 1] : take(x, warp - 1, j, gen, fail);
-            upH = tv.x;
-            upF = tv.y;
+            if (warp == 0) {
+                upH = s->top[j + 1].x;
+                upF = s->top[j + 1].y;
+            } else {
+                upH = (int32_t)take(x, &x->bnd[warp - 1][j][0], gen, fail);
+                upF = (int32_t)take(x, &x->bnd[warp - 1][j][1], gen, fail);
+            }
         }
         int32_t oH = 0, oF = 0;
         if (act) {
@@ -260,20 +283,16 @@ __device__ void recompute(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0,
             int32_t hu = upH, fu = upF;
             uint32_t word = 0;
 #pragma unroll
-            for (int i = 0; i < kRT; ++i) {
+            for (int i = 0; i < kRW; ++i) {
                 if (r0 + i <= R1) {
                     const int32_t eext = El[i] + a.ext, eopen = Hl[i] + a.open;
                     const int32_t fext = fu + a.ext, fopen = hu + a.open;
                     const int32_t e = max(eext, eopen), f = max(fext, fopen);
-                    const bool same = ra[i] == cb;
-                    const int32_t dg = hd + (same ? a.match : a.mismatch);
+                    const int32_t dg = hd + (ra[i] == cb ? a.match : a.mismatch);
                     const int32_t hv = max(max(0, e), max(f, dg));
-                    uint32_t v = hv == 0 ? SRC_ZERO : (hv == dg ? SRC_DIAG : (hv == e ? SRC_E : SRC_F));
-                    if (same) v |= BIT_MATCH;
-                    if (eext == e) v |= BIT_EEXT;
-                    if (fext == f) v |= BIT_FEXT;
-                    if (hd == 0) v |= BIT_DZERO;
-                    word |= v << (8 * i);
+                    word |= ((hv != dg ? BIT_ND : 0u) | (hv != e ? BIT_NE : 0u) | (eext != e ? BIT_NEX : 0u) |
+                             (fext != f ? BIT_NFX : 0u))
+                            << (4 * i);
                     hd = Hl[i];
                     Hl[i] = hv;
                     El[i] = e;
@@ -281,12 +300,12 @@ __device__ void recompute(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0,
                     fu = f;
                 }
             }
-            dir.put(t, j, k, word);
+            reinterpret_cast<uint16_t *>(d)[dir_index(t * kRW, (int)j)] = (uint16_t)word;
             oH = hu;
             oF = fu;
             if (publish) {
-                x->bnd[warp][j][0] = pack(oH, gen);
-                x->bnd[warp][j][1] = pack(oF, gen);
+                x->bnd[warp][j][0] = pack((uint32_t)oH, gen);
+                x->bnd[warp][j][1] = pack((uint32_t)oF, gen);
             }
         }
         prevUpH = upH;
@@ -301,11 +320,179 @@ __device__ void recompute(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0,
     }
 }
 
-// Warp 0 walks the path through the block [R0, R1] x [C0, C1].
-// Row and column indices fit 32 bits (pairs are limited to 2^31 - 64 rows), so
-// the crosspoint tests use 32-bit remainders.
-template <class D>
-__device__ void walk(const WalkArgs &a, int64_t R0, int64_t C0, const D &dir, int64_t *S) {
+// The same in packed 16-bit halves, two warps of 256 rows: as in strip16.cuh the low
+// halves of a warp are virtual lanes 0..31 (four rows each) and the high halves
+// virtual lanes 32..63, and lane 31 turns its slot of the shuffle around.  A
+// block's cells lie within 12,000 of its corner (walk16_fits), so offsets from
+// base = max(0, corner - 12000) fit, and with base > 0 no H comes down to it, where
+// the relu would differ from the recurrence's floor at 0.
+// Unrolled by 4: a block walks through its code once, and by 8 a block alone takes
+// 35% longer for instruction fetch (600 bp pair's stage 2: 0.176 against 0.129 ms).
+// What bounds it: 19 ALU ops a row pair (each direction bit is an exclusive or and
+// an unsigned minimum with 1, gathered by a multiply-add) at 64 lanes per SM and cycle,
+// and for a block alone the chain of 400 steps.  Stage 2 of the 600 bp pair (one or
+// two blocks) 0.26 -> 0.13 ms against the 32-bit recompute, a batch of 24 pairs'
+// walker 8.2 -> 2.8 ms.
+constexpr int32_t kCornerOffset = 12000;
+__device__ __forceinline__ uint32_t dup16(int32_t v) { return (uint32_t)(uint16_t)(int16_t)v * 0x00010001u; }
+__device__ __forceinline__ uint32_t pair16(int32_t lo, int32_t hi) {
+    return ((uint32_t)(uint16_t)(int16_t)lo) | ((uint32_t)(uint16_t)(int16_t)hi << 16);
+}
+__device__ __forceinline__ uint32_t prmt(uint32_t lo, uint32_t hi, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(lo), "r"(hi), "r"(sel));
+    return r;
+}
+
+// 1 in each half that differs.
+__device__ __forceinline__ uint32_t differs(uint32_t a, uint32_t b) { return __vminu2(a ^ b, 0x00010001u); }
+
+struct Lane4 {
+    uint32_t H[kRW], E[kRW], ra[kRW];
+    uint32_t inH, inF, hd;  // (H, F) of the row above at this column, its H at the previous one
+};
+struct Scores4 {
+    uint32_t open2, ext2, gx2, mt1, mm;
+};
+
+// One step: returns the lane's direction word; fl is F of its last rows.  PRED:
+// halves whose column is left of the block keep their values (mask).
+template <bool PRED>
+__device__ __forceinline__ uint32_t step4(Lane4 &L, const Scores4 &c, uint32_t col, uint32_t rv, uint32_t selH,
+                                          uint32_t selF, int src, uint32_t mask, uint32_t &fl) {
+    uint32_t t[kRW], e[kRW], dg[kRW], word = 0;
+    uint32_t hd = L.hd;
+#pragma unroll
+    for (int i = 0; i < kRW; ++i) {
+        const uint32_t s = __viaddmax_s16x2(~(L.ra[i] ^ col), c.mt1, c.mm);
+        const uint32_t x = __vadd2(L.E[i], c.ext2);
+        e[i] = __viaddmax_s16x2(L.H[i], c.open2, x);
+        dg[i] = __vadd2(hd, s);
+        t[i] = __vimax_s16x2_relu(dg[i], e[i]);
+        word += differs(e[i], x) * (BIT_NEX << (4 * i));
+        hd = L.H[i];
+    }
+    uint32_t y = __vadd2(L.inF, c.ext2);
+    uint32_t f = __viaddmax_s16x2(L.inH, c.open2, y);
+#pragma unroll
+    for (int i = 0; i < kRW; ++i) {
+        const uint32_t h = __vmaxs2(t[i], f);
+        word += differs(f, y) * (BIT_NFX << (4 * i)) +
+                differs(h, dg[i]) * (BIT_ND << (4 * i)) +
+                differs(h, e[i]) * (BIT_NE << (4 * i));
+        fl = f;
+        y = __vadd2(f, c.ext2);
+        f = __viaddmax_s16x2(f, c.gx2, __vadd2(t[i], c.open2));
+        L.H[i] = PRED ? ((h & mask) | (L.H[i] & ~mask)) : h;
+        L.E[i] = PRED ? ((e[i] & mask) | (L.E[i] & ~mask)) : e[i];
+    }
+    const uint32_t nH = prmt(rv, L.H[kRW - 1], selH), nF = prmt(rv, fl, selF);
+    L.hd = L.inH;
+    L.inH = __shfl_sync(0xffffffffu, nH, src);
+    L.inF = __shfl_sync(0xffffffffu, nF, src);
+    return word;
+}
+
+// As recompute_wide; kThreads threads.
+__device__ void recompute16(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0, int64_t C1, uint32_t *d, Xchg *x,
+                            Stage *s, uint32_t gen) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int w = (int)(C1 - C0 + 1), h = (int)(R1 - R0 + 1), r_warp = warp * kWarpRows;
+    if (r_warp >= h) return;  // this warp has no rows
+    const int32_t corner = s->top[0].x, base = max(0, corner - kCornerOffset);
+    Scores4 c;
+    c.open2 = dup16(a.open);
+    c.ext2 = dup16(a.ext);
+    c.gx2 = dup16(max(a.open, a.ext));
+    c.mt1 = dup16(a.match + 1);
+    c.mm = dup16(a.mismatch);
+    auto off = [&](int32_t v) { return max(v - base, -16384); };
+    if (warp == 0) {
+        for (int j = lane; j < w; j += 32) s->top16[j] = pair16(off(s->top[j + 1].x), off(s->top[j + 1].y));
+        __syncwarp();
+    }
+    Lane4 L;
+#pragma unroll
+    for (int i = 0; i < kRW; ++i) {
+        int2 lv[2];
+        uint32_t code[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int r = r_warp + (lane + 32 * q) * kRW + i;  // rows past the end: the last row's boundary, no match
+            lv[q] = left_he(a, C0, R0 + min(r, h - 1));
+            code[q] = (r < h ? (uint32_t)s->rb[r] : 256u) << 6;
+        }
+        L.H[i] = pair16(off(lv[0].x), off(lv[1].x));
+        L.E[i] = pair16(off(lv[0].y), off(lv[1].y));
+        L.ra[i] = code[0] | (code[1] << 16);
+    }
+    const int src = (lane + 31) & 31;
+    const uint32_t selH = lane == 31 ? 0x5410u : 0x7654u, selF = lane == 31 ? 0x5432u : 0x7654u;
+    bool fail = false;
+    auto above = [&](int j) -> uint32_t {  // (H, F) of the row above the warp at column j
+        if (j >= w) j = w - 1;
+        return warp == 0 ? s->top16[j] : take(x, &x->bnd[warp - 1][j][0], gen, fail);
+    };
+    {
+        // what the shuffles of the step before column 0 would have brought
+        const uint32_t up = __shfl_sync(0xffffffffu, prmt(0u, L.H[kRW - 1], selH), src);
+        const int32_t first = warp == 0 ? corner : left_he(a, C0, R0 + r_warp - 1).x;
+        const uint32_t v = above(0);
+        L.hd = lane == 0 ? prmt((uint32_t)off(first), up, 0x7610u) : up;
+        L.inH = lane == 0 ? prmt(v, up, 0x7610u) : up;
+        L.inF = v >> 16;
+    }
+    const bool publish = lane == 31 && r_warp + kWarpRows < h;
+    const uint16_t *pc = s->col16 + 64 - lane;
+    uint32_t *pd = d + (int64_t)warp * kSteps * 32 + lane;
+    unsigned long long(*pub)[2] = x->bnd[warp < kThreads / 32 - 1 ? warp : 0];
+    const int steps = w + 63;
+    uint32_t col = (uint32_t)pc[0] | ((uint32_t)pc[-32] << 16);
+    // chunks of kC steps: one lane per column of the row above; the next step's
+    // column codes are loaded ahead.  The last chunk's steps past `steps` write
+    // words that no walk reads (kSteps is a multiple of kC).
+    for (int k = 0; k < 64; k += kC) {
+        const uint32_t ab = above(k + 1 + (lane & (kC - 1)));
+        __syncwarp();
+#pragma unroll 4
+        for (int u = 0; u < kC; ++u) {
+            const uint32_t next = (uint32_t)pc[k + u + 1] | ((uint32_t)pc[k + u - 31] << 16);
+            const uint32_t rv = __shfl_sync(0xffffffffu, ab, u);
+            const uint32_t mask = (k + u >= lane ? 0x0000FFFFu : 0u) | (k + u >= lane + 32 ? 0xFFFF0000u : 0u);
+            uint32_t fl;
+            pd[(k + u) * 32] = step4<true>(L, c, col, rv, selH, selF, src, mask, fl);
+            if (publish && k + u == 63) pub[0][0] = pack(prmt(L.H[kRW - 1], fl, 0x7632u), gen);
+            col = next;
+        }
+    }
+    for (int k = 64; k < steps; k += kC) {
+        const uint32_t ab = above(k + 1 + (lane & (kC - 1)));
+        __syncwarp();
+#pragma unroll 4
+        for (int u = 0; u < kC; ++u) {
+            const uint32_t next = (uint32_t)pc[k + u + 1] | ((uint32_t)pc[k + u - 31] << 16);
+            const uint32_t rv = __shfl_sync(0xffffffffu, ab, u);
+            uint32_t fl;
+            pd[(k + u) * 32] = step4<false>(L, c, col, rv, selH, selF, src, ~0u, fl);
+            if (publish && k + u - 63 < w) pub[k + u - 63][0] = pack(prmt(L.H[kRW - 1], fl, 0x7632u), gen);
+            col = next;
+        }
+    }
+}
+
+// Either recompute; wide is the same for all blocks of a launch.
+template <bool WIDE>
+__device__ __forceinline__ void recompute(const WalkArgs &a, int64_t R0, int64_t R1, int64_t C0, int64_t C1, uint32_t *d,
+                                          Xchg *x, Stage *s, uint32_t gen) {
+    if constexpr (WIDE) recompute_wide(a, R0, R1, C0, C1, d, x, s, gen);
+    else recompute16(a, R0, R1, C0, C1, d, x, s, gen);
+}
+
+// Warp 0 walks the path through the block that starts at (R0, C0); rb, cb: the
+// block's bytes.  Row and column indices fit 32 bits (pairs are limited to
+// 2^31 - 64 rows), so the crosspoint tests use 32-bit remainders.
+__device__ void walk(const WalkArgs &a, int64_t R0, int64_t C0, const Dir &dir, const uint8_t *rb, const uint8_t *cb,
+                     int64_t *S) {
     const int lane = threadIdx.x & 31;
     int64_t r = S[kStR], c = S[kStC];
     int32_t state = (int32_t)S[kStState];
@@ -314,22 +501,25 @@ __device__ void walk(const WalkArgs &a, int64_t R0, int64_t C0, const D &dir, in
     bool done = false, err = false;
     while (!done && !err && r >= R0 && c >= C0) {
         if (state == ST_H) {
-            // run of diagonal moves that are not the start
+            // run of diagonal moves: cells whose H comes from the diagonal, up to the
+            // one whose diagonal predecessor has no score left, the start cell
             const int64_t rr = r - lane, cc = c - lane;
             const bool in = rr >= R0 && cc >= C0;
-            const uint8_t v = in ? dir.at(rr - R0, cc - C0) : 0;
-            const bool ok = in && (v & 3) == SRC_DIAG && !(v & BIT_DZERO);
-            const uint32_t bal = __ballot_sync(0xffffffffu, ok);
-            const int nrun = (bal == 0xffffffffu) ? 32 : __ffs(~bal) - 1;
-            // inclusive prefix over lanes of the run's substitution scores (the
-            // suffix after lane i's cell), from one ballot of the matching cells
-            const bool mt = lane < nrun && (v & BIT_MATCH);
-            const uint32_t mb = __ballot_sync(0xffffffffu, mt);
-            const int nle = min(lane + 1, nrun);
-            const int mle = __popc(mb & (0xffffffffu >> (31 - lane)));
-            const int32_t ps = mle * a.match + (nle - mle) * a.mismatch;
+            const uint32_t v = in ? dir.at(rr - R0, cc - C0) : BIT_ND;
+            // inclusive prefix over lanes of the substitution scores (the suffix after
+            // lane i's cell), from one ballot of the matching cells
+            const uint32_t mb = __ballot_sync(0xffffffffu, in && rb[rr - R0] == cb[cc - C0]);
+            const uint32_t upto = 0xffffffffu >> (31 - lane);
+            const int mle = __popc(mb & upto);
+            const int32_t ps = mle * a.match + (lane + 1 - mle) * a.mismatch;
+            const uint32_t db = __ballot_sync(0xffffffffu, (v & BIT_ND) == 0);
+            const int ndiag = (db == 0xffffffffu) ? 32 : __ffs(~db) - 1;
+            const uint32_t sb = __ballot_sync(0xffffffffu, lane < ndiag && (int64_t)a.score == suffix + ps);
+            const bool start = sb != 0;
+            const int nrun = start ? __ffs(sb) : ndiag;  // cells taken; the start cell is the last
             // crosspoint: moving from (rr, cc) to (rr-1, cc-1) enters row rr-1 from below
-            const bool xp = lane < nrun && rr - 1 >= 0 && ((int32_t)rr % X) == 0;
+            // (not from the start cell)
+            const bool xp = lane < nrun - (start ? 1 : 0) && rr - 1 >= 0 && ((int32_t)rr % X) == 0;
             const uint32_t xbal = __ballot_sync(0xffffffffu, xp);
             if (xp) {
                 const int64_t slot = nxp + __popc(xbal & ((1u << lane) - 1));
@@ -342,36 +532,28 @@ __device__ void walk(const WalkArgs &a, int64_t R0, int64_t C0, const D &dir, in
                 }
             }
             if (lane < nrun && nops + lane < a.ops_cap) a.ops[nops + lane] = 'M';
-            const int32_t tot = __popc(mb) * a.match + (nrun - __popc(mb)) * a.mismatch;
-            nops += nrun;
-            suffix += tot;
-            nxp += __popc(xbal);
-            r -= nrun;
-            c -= nrun;
-            if (nrun < 32 && r >= R0 && c >= C0) {
-                const uint8_t w = dir.at(r - R0, c - C0);
-                const int src = w & 3;
-                if (src == SRC_DIAG) {  // the start cell
-                    if (lane == 0 && nops < a.ops_cap) a.ops[nops] = 'M';
-                    nops += 1;
-                    suffix += (w & BIT_MATCH) ? a.match : a.mismatch;
-                    S[kStStartR] = r;
-                    S[kStStartC] = c;
-                    done = true;
-                } else if (src == SRC_E) {
-                    state = ST_E;
-                } else if (src == SRC_F) {
-                    state = ST_F;
-                } else {
-                    err = true;
-                }
+            if (nrun > 0) {
+                nops += nrun;
+                suffix += __shfl_sync(0xffffffffu, ps, nrun - 1);
+                nxp += __popc(xbal);
+                r -= nrun;
+                c -= nrun;
+            }
+            if (start) {
+                S[kStStartR] = r + 1;
+                S[kStStartC] = c + 1;
+                done = true;
+            } else if (nrun < 32 && r >= R0 && c >= C0) {
+                const uint32_t q = dir.at(r - R0, c - C0);
+                if (!(q & BIT_ND)) err = true;  // cannot be: the run stopped here
+                state = (q & BIT_NE) ? ST_F : ST_E;
             }
         } else if (state == ST_E) {
             // horizontal run: 'I' for every cell until the gap opens
             const int64_t cc = c - lane;
             const bool in = cc >= C0;
-            const uint8_t v = in ? dir.at(r - R0, cc - C0) : 0;
-            const bool ext = in && (v & BIT_EEXT);
+            const uint32_t v = in ? dir.at(r - R0, cc - C0) : BIT_NEX;
+            const bool ext = !(v & BIT_NEX);
             const uint32_t bal = __ballot_sync(0xffffffffu, ext);
             const uint32_t inb = __ballot_sync(0xffffffffu, in);
             int nrun;                                  // cells consumed
@@ -393,8 +575,8 @@ __device__ void walk(const WalkArgs &a, int64_t R0, int64_t C0, const D &dir, in
             // vertical run: 'D' for every cell until the gap opens
             const int64_t rr = r - lane;
             const bool in = rr >= R0;
-            const uint8_t v = in ? dir.at(rr - R0, c - C0) : 0;
-            const bool ext = in && (v & BIT_FEXT);
+            const uint32_t v = in ? dir.at(rr - R0, c - C0) : BIT_NFX;
+            const bool ext = !(v & BIT_NFX);
             const uint32_t bal = __ballot_sync(0xffffffffu, ext);
             const uint32_t inb = __ballot_sync(0xffffffffu, in);
             const int firstno = (bal == 0xffffffffu) ? 32 : __ffs(~bal) - 1;
@@ -446,8 +628,8 @@ __device__ void walk(const WalkArgs &a, int64_t R0, int64_t C0, const D &dir, in
 
 // Block after block until the start is reached or the path leaves the region
 // [rr0, .) x [cc0, .); the state is read from and written back to a.st.
-template <class D>
-__device__ void walk_body(const WalkArgs &a, const D &dir, Xchg *xc, Stage *sg, int64_t *S) {
+template <bool WIDE>
+__device__ void walk_body(const WalkArgs &a, uint32_t *dir, Xchg *xc, Stage *sg, int64_t *S) {
     if (threadIdx.x < kStN) S[threadIdx.x] = a.st[threadIdx.x];
     __syncthreads();
     int guard = 0;
@@ -458,14 +640,14 @@ __device__ void walk_body(const WalkArgs &a, const D &dir, Xchg *xc, Stage *sg, 
         const int64_t C0 = a.cc0 + ((c - a.cc0) / kBC) * kBC;
         stage_block(a, R0, r, C0, c, sg);
         __syncthreads();
-        recompute(a, R0, r, C0, c, dir, xc, sg, xc->gen + (uint32_t)guard + 1u);
+        recompute<WIDE>(a, R0, r, C0, c, dir, xc, sg, xc->gen + (uint32_t)guard + 1u);
         __syncthreads();
         if (xc->err) {
             if (threadIdx.x == 0) S[kStErr] = 1;
             __syncthreads();
             break;
         }
-        if (threadIdx.x < 32) walk(a, R0, C0, dir, S);
+        if (threadIdx.x < 32) walk(a, R0, C0, Dir{dir}, sg->rb, sg->cb, S);
         __syncthreads();
     }
     if (threadIdx.x < kStN) a.st[threadIdx.x] = S[threadIdx.x];
@@ -477,8 +659,10 @@ __device__ void walk_body(const WalkArgs &a, const D &dir, Xchg *xc, Stage *sg, 
 // of a region into gdir + b * kBlockWords (one CTA per block at a time).  A block
 // depends only on the stored boundaries, not on the path, so any set of blocks
 // can run at once.
-__global__ void __launch_bounds__(kThreads) precompute_kernel(WalkArgs a, const int64_t *blk, int64_t nblk,
-                                                              uint32_t *gdir, int32_t *err) {
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? kThreadsWide : kThreads) precompute_kernel(WalkArgs a, const int64_t *blk,
+                                                                                   int64_t nblk, uint32_t *gdir,
+                                                                                   int32_t *err) {
     __shared__ Xchg xc;
     __shared__ Stage sg;
     xchg_init(&xc);
@@ -489,13 +673,12 @@ __global__ void __launch_bounds__(kThreads) precompute_kernel(WalkArgs a, const 
         __syncthreads();
         stage_block(a, R0, R1, C0, C1, &sg);
         __syncthreads();
-        recompute(a, R0, R1, C0, C1, GlobalDir{gdir + b * kBlockWords}, &xc, &sg, ++gen);
+        recompute<WIDE>(a, R0, R1, C0, C1, gdir + b * kBlockWords, &xc, &sg, ++gen);
     }
     __syncthreads();
     if (threadIdx.x == 0 && xc.err) atomicExch(err, 1);
 }
 
-// Sequence bytes of a block for the walk's diagonal scores.
 // One warp walks the path through precomputed blocks: block (bi, bj) of the
 // region (relative to rr0, cc0) is slot map[(bi - bi0) * mw + (bj - bj0)] of
 // gdir, or absent (-1).  Stops where the path enters an absent block, at the
@@ -517,15 +700,17 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
 
 // The walk of each block reads the block's direction words from shared memory:
 // on entering a block the warp copies the part the path can still reach (the
-// 128-row chunks at or above the current row, the steps up to the current
-// column + 31) from gdir with one bulk asynchronous copy (cp.async.bulk, the
+// 256-row chunks at or above the current row, the steps up to the current
+// column + 63) from gdir with one bulk asynchronous copy (cp.async.bulk, the
 // TMA engine) per chunk, completing on an mbarrier; every step of the walk is
-// then a shared-memory read instead of a dependent L2 round trip.  The
-// direction bytes carry the match bit, so no sequence bytes are read.
+// then a shared-memory read instead of a dependent L2 round trip.  The block's
+// sequence bytes, for the path's scores, are fetched as aligned words while the
+// copy is on its way.
 __global__ void __launch_bounds__(32) corridor_walk_kernel(WalkArgs a, const uint32_t *gdir, const int32_t *map,
                                                            int64_t bi0, int64_t bj0, int64_t mh, int64_t mw,
                                                            const int32_t *err) {
     extern __shared__ __align__(16) uint32_t dtile[];  // kBlockWords words
+    __shared__ uint32_t seq_r[kBR / 4 + 2], seq_c[kBC / 4 + 2];
     __shared__ int64_t S[kStN];
     __shared__ __align__(8) uint64_t bar_mem;
     const int lane = threadIdx.x;
@@ -551,8 +736,8 @@ __global__ void __launch_bounds__(32) corridor_walk_kernel(WalkArgs a, const uin
         const int32_t slot = map[(bi - bi0) * mw + (bj - bj0)];
         if (slot < 0) break;
         const int64_t R0 = a.rr0 + bi * a.br, C0 = a.cc0 + bj * kBC;
-        const int wmax = (int)((r - R0) >> 7);
-        const int kn = (int)(c - C0 + 32 < (int64_t)kSteps ? c - C0 + 32 : (int64_t)kSteps);
+        const int wmax = (int)((r - R0) / kWarpRows);
+        const int kn = (int)(c - C0) + 64;
         const uint32_t chunk = (uint32_t)kn * 32u * 4u;
         __syncwarp();  // the previous block's reads of dtile are done
         if (lane == 0) {
@@ -569,6 +754,25 @@ __global__ void __launch_bounds__(32) corridor_walk_kernel(WalkArgs a, const uin
                     : "memory");
         }
         in_flight = true;
+        // bytes R0..r and C0..c, as the aligned words that hold them
+        const uintptr_t pr = reinterpret_cast<uintptr_t>(a.rows + R0), pc = reinterpret_cast<uintptr_t>(a.cols + C0);
+        const int nr = (int)((pr & 3) + (r - R0)) / 4 + 1, nc = (int)((pc & 3) + (c - C0)) / 4 + 1;
+        {
+            uint32_t v[kBR / 128 + 1 + kBC / 128 + 1];
+            constexpr int kNR = kBR / 128 + 1, kNC = kBC / 128 + 1;
+#pragma unroll
+            for (int q = 0; q < kNR; ++q)
+                if (lane + 32 * q < nr) v[q] = reinterpret_cast<const uint32_t *>(pr & ~(uintptr_t)3)[lane + 32 * q];
+#pragma unroll
+            for (int q = 0; q < kNC; ++q)
+                if (lane + 32 * q < nc) v[kNR + q] = reinterpret_cast<const uint32_t *>(pc & ~(uintptr_t)3)[lane + 32 * q];
+#pragma unroll
+            for (int q = 0; q < kNR; ++q)
+                if (lane + 32 * q < nr) seq_r[lane + 32 * q] = v[q];
+#pragma unroll
+            for (int q = 0; q < kNC; ++q)
+                if (lane + 32 * q < nc) seq_c[lane + 32 * q] = v[kNR + q];
+        }
         const bool ok = __all_sync(0xffffffffu, bar_wait(bar, phase & 1));
         if (!ok) {
             if (lane == 0) S[kStErr] = 1;
@@ -578,7 +782,8 @@ __global__ void __launch_bounds__(32) corridor_walk_kernel(WalkArgs a, const uin
         in_flight = false;
         ++phase;
         __syncwarp();
-        walk(a, R0, C0, SmemDir{dtile}, S);
+        walk(a, R0, C0, Dir{dtile}, reinterpret_cast<const uint8_t *>(seq_r) + (pr & 3),
+             reinterpret_cast<const uint8_t *>(seq_c) + (pc & 3), S);
         __syncwarp();
     }
     // A copy still in flight after its wait ran out writes this CTA's shared
@@ -596,13 +801,14 @@ __global__ void __launch_bounds__(32) corridor_walk_kernel(WalkArgs a, const uin
 // matrix is its region), recomputing the blocks on its path on demand into its
 // own region of gdir (kBlockWords words per CTA).
 // One CTA per pair at a time, pairs p = blockIdx.x, + gridDim.x, ...
+template <bool WIDE>
 __device__ __forceinline__ void walk_pairs(const WalkArgs *args, int64_t n, uint32_t *gdir) {
     __shared__ Xchg xc;
     __shared__ Stage sg;
     __shared__ int64_t S[kStN];
     __shared__ WalkArgs sa;
     xchg_init(&xc);
-    const GlobalDir dir{gdir + (int64_t)blockIdx.x * kBlockWords};
+    uint32_t *dir = gdir + (int64_t)blockIdx.x * kBlockWords;
     for (int64_t p = blockIdx.x; p < n; p += gridDim.x) {
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -610,12 +816,14 @@ __device__ __forceinline__ void walk_pairs(const WalkArgs *args, int64_t n, uint
             xc.err = 0;
         }
         __syncthreads();
-        walk_body(sa, dir, &xc, &sg, S);
+        walk_body<WIDE>(sa, dir, &xc, &sg, S);
     }
 }
 
-__global__ void __launch_bounds__(kThreads) walk_batch_kernel(const WalkArgs *args, int64_t n, uint32_t *gdir) {
-    walk_pairs(args, n, gdir);
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? kThreadsWide : kThreads) walk_batch_kernel(const WalkArgs *args, int64_t n,
+                                                                                   uint32_t *gdir) {
+    walk_pairs<WIDE>(args, n, gdir);
 }
 
 // Graphed batches: every pair's walk starts at the best cell the scoring kernel
@@ -639,8 +847,9 @@ __global__ void walk_graph_init_kernel(const GraphHdr *h) {
     }
 }
 
-__global__ void __launch_bounds__(kThreads) walk_graph_kernel(const GraphHdr *h) {
-    walk_pairs((const WalkArgs *)h->walk_args, h->npairs, h->walk_dir);
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? kThreadsWide : kThreads) walk_graph_kernel(const GraphHdr *h) {
+    walk_pairs<WIDE>((const WalkArgs *)h->walk_args, h->npairs, h->walk_dir);
 }
 
 }  // namespace
@@ -649,12 +858,15 @@ cudaError_t walker_configure() {
     const int c = cudaSharedmemCarveoutMaxShared;
     const auto A = cudaFuncAttributePreferredSharedMemoryCarveout;
     cudaError_t e = cudaSuccess;
-    for (cudaError_t x : {cudaFuncSetAttribute((const void *)precompute_kernel, A, c),
+    for (cudaError_t x : {cudaFuncSetAttribute((const void *)precompute_kernel<false>, A, c),
+                          cudaFuncSetAttribute((const void *)precompute_kernel<true>, A, c),
                           cudaFuncSetAttribute((const void *)corridor_walk_kernel, A, c),
                           cudaFuncSetAttribute((const void *)corridor_walk_kernel,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDirTileBytes),
-                          cudaFuncSetAttribute((const void *)walk_batch_kernel, A, c),
-                          cudaFuncSetAttribute((const void *)walk_graph_kernel, A, c)})
+                          cudaFuncSetAttribute((const void *)walk_batch_kernel<false>, A, c),
+                          cudaFuncSetAttribute((const void *)walk_batch_kernel<true>, A, c),
+                          cudaFuncSetAttribute((const void *)walk_graph_kernel<false>, A, c),
+                          cudaFuncSetAttribute((const void *)walk_graph_kernel<true>, A, c)})
         if (x != cudaSuccess) e = x;
     return e;
 }
@@ -700,6 +912,16 @@ Plan plan_for(const swb_options &opts, int64_t m, int64_t n, int64_t br) {
 // Block rows of a region's grid: in.br, or the full block height when unset.
 static int64_t block_rows_of(const WalkInputs &in) { return in.br > 0 && in.br <= kBR ? in.br : kBR; }
 
+// Whether a block's cells stay within kCornerOffset of its corner (the spread bound
+// of strip16.cuh over the block's rows and columns) and the scores fit the packed
+// recompute.
+bool walk16_fits(const swb_scoring &sc) {
+    const int64_t e = std::min(-(int64_t)sc.gap_open, -(int64_t)sc.gap_extend);
+    const int64_t slope = sc.match + e, open = -(int64_t)sc.gap_open;
+    return (kBR + kBC + 2) * slope + 3 * open - sc.gap_extend <= kCornerOffset - 256 && sc.match - sc.mismatch <= 64 &&
+           sc.gap_extend >= -1000 && open <= 1000 && sc.mismatch >= -1000;
+}
+
 static WalkArgs to_args(const WalkInputs &in) {
     WalkArgs a{};
     a.rows = in.rows;
@@ -726,6 +948,7 @@ static WalkArgs to_args(const WalkInputs &in) {
     a.xp_cap = in.xp_cap;
     a.st = in.dstate;
     a.br = (int32_t)block_rows_of(in);
+    a.wide = walk16_fits(in.sc) ? 0 : 1;
     return a;
 }
 
@@ -815,7 +1038,8 @@ int walk_region(cudaStream_t st, int sms, const WalkInputs &in, int64_t *host_st
             err = std::string("walker corridor: ") + cudaGetErrorString(e);
             return SWB_ECUDA;
         }
-        precompute_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(a, d_blk, nblk, gdir, d_err);
+        if (a.wide) precompute_kernel<true><<<(unsigned)nblk, kThreadsWide, 0, st>>>(a, d_blk, nblk, gdir, d_err);
+        else precompute_kernel<false><<<(unsigned)nblk, kThreads, 0, st>>>(a, d_blk, nblk, gdir, d_err);
         corridor_walk_kernel<<<1, 32, kDirTileBytes, st>>>(a, gdir, d_map, bi0, bj0, mh, mw, d_err);
         *launches += 2;
         if ((e = cudaGetLastError()) != cudaSuccess ||
@@ -855,7 +1079,8 @@ int walk_batch(cudaStream_t st, int sms, const WalkInputs *in, int64_t n, void *
         err = std::string("batched walker set-up: ") + cudaGetErrorString(e);
         return SWB_ECUDA;
     }
-    walk_batch_kernel<<<(unsigned)grid, kThreads, 0, st>>>((const WalkArgs *)d_args, n, (uint32_t *)d_dir);
+    if (args[0].wide) walk_batch_kernel<true><<<(unsigned)grid, kThreadsWide, 0, st>>>((const WalkArgs *)d_args, n, (uint32_t *)d_dir);
+    else walk_batch_kernel<false><<<(unsigned)grid, kThreads, 0, st>>>((const WalkArgs *)d_args, n, (uint32_t *)d_dir);
     if ((e = cudaGetLastError()) != cudaSuccess ||
         (e = scr.get(scr.owner, host_states, d_states, sizeof(int64_t) * kStN * (size_t)n)) != cudaSuccess) {
         err = std::string("batched walker: ") + cudaGetErrorString(e);
@@ -878,10 +1103,12 @@ void pack_walk_args(const WalkInputs *in, int64_t n, int64_t *d_states, void *ds
     }
 }
 
-cudaError_t walk_graph_enqueue(const GraphHdr *d_hdr, int sms, int64_t max_pairs, cudaStream_t st) {
+cudaError_t walk_graph_enqueue(const GraphHdr *d_hdr, bool wide, int sms, int64_t max_pairs, cudaStream_t st) {
     const int64_t p = std::max<int64_t>(1, max_pairs);
     walk_graph_init_kernel<<<(unsigned)std::min<int64_t>(std::max(1, sms), (p + 255) / 256), 256, 0, st>>>(d_hdr);
-    walk_graph_kernel<<<(unsigned)std::min<int64_t>(walk_graph_ctas(sms), p), kThreads, 0, st>>>(d_hdr);
+    const unsigned grid = (unsigned)std::min<int64_t>(walk_graph_ctas(sms), p);
+    if (wide) walk_graph_kernel<true><<<grid, kThreadsWide, 0, st>>>(d_hdr);
+    else walk_graph_kernel<false><<<grid, kThreads, 0, st>>>(d_hdr);
     return cudaGetLastError();
 }
 
