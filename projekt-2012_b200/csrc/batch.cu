@@ -26,6 +26,7 @@
 
 #include "batch.h"
 #include "stage1_core.cuh"
+#include "strip16.cuh"
 
 namespace swb {
 namespace {
@@ -82,6 +83,40 @@ struct PairView : S {
     static constexpr int64_t *trace = nullptr;
 };
 
+// The view of pair d; units: what one of d.sr_every's 512-row strips is in the
+// units of v.sr_every (1, or half strips of packed strips).
+template <class S>
+__device__ __forceinline__ void make_view(const BatchArgs &g, const BatchPair &d, bool tab, int units, PairView<S> &v) {
+    v.open = g.open;
+    v.ext = g.ext;
+    v.gx = g.gx;
+    v.mt1 = g.mt1;
+    v.mm1 = g.mm1;
+    v.tab_hi = g.tab_hi;
+    v.err = g.ctl + 1;
+    v.rows = g.seq + d.row_off;
+    v.cols = g.cseq + d.col_off;
+    v.rcode = tab ? g.rcode + d.row_off : nullptr;
+    v.ctab = tab ? g.ctab + d.col_off : nullptr;
+    v.m = d.m;
+    v.n = d.n;
+    v.hbuf = g.hbuf + d.hbuf_off;
+    v.gbest = g.gbest + d.slot;
+    v.tie = d.tie;
+    v.wait_limit = g.wait_limit;
+    if constexpr (!std::is_same<S, NoStores>::value) {
+        v.srows = g.srows + d.sr_off;
+        v.sr_every = (int64_t)d.sr_every * units;
+        v.scols = g.scols + d.sc_off;
+        v.sc_every = d.sc_every;
+    }
+    if constexpr (std::is_same<S, WithBounds>::value) {
+        v.top = d.top;
+        v.left = d.left;
+        v.corner = (d.top && d.left) ? d.top[-1].x : 0;
+    }
+}
+
 // Claims units until the queue is empty and runs each as one strip.
 template <int R, bool TAB, class S>
 __device__ __forceinline__ void batch_body(const BatchArgs &g) {
@@ -99,34 +134,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs &g) {
         if (u >= nunits || ld_volatile(&g.ctl[2]) != 0) break;
         const BatchPair d = g.pairs[g.unit_pair[u]];
         PairView<S> v;
-        v.open = g.open;
-        v.ext = g.ext;
-        v.gx = g.gx;
-        v.mt1 = g.mt1;
-        v.mm1 = g.mm1;
-        v.tab_hi = g.tab_hi;
-        v.err = g.ctl + 1;
-        v.rows = g.seq + d.row_off;
-        v.cols = g.cseq + d.col_off;
-        v.rcode = TAB ? g.rcode + d.row_off : nullptr;
-        v.ctab = TAB ? g.ctab + d.col_off : nullptr;
-        v.m = d.m;
-        v.n = d.n;
-        v.hbuf = g.hbuf + d.hbuf_off;
-        v.gbest = g.gbest + d.slot;
-        v.tie = d.tie;
-        v.wait_limit = g.wait_limit;
-        if constexpr (!std::is_same<S, NoStores>::value) {
-            v.srows = g.srows + d.sr_off;
-            v.sr_every = d.sr_every;
-            v.scols = g.scols + d.sc_off;
-            v.sc_every = d.sc_every;
-        }
-        if constexpr (std::is_same<S, WithBounds>::value) {
-            v.top = d.top;
-            v.left = d.left;
-            v.corner = (d.top && d.left) ? d.top[-1].x : 0;
-        }
+        make_view(g, d, TAB, 1, v);
         Best b;
         init_best(b, g.open);
         int32_t bho = b.ho;
@@ -162,6 +170,56 @@ __device__ __forceinline__ void batch_body(const BatchArgs &g) {
             g.ubest[d.ufirst + strip] = r;
         }
     }
+}
+
+// The same with packed 16-bit strips of 64 RH rows (strip16.cuh).
+template <int RH, class S>
+__device__ __forceinline__ void packed_body(const BatchArgs &g, bool tab) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr bool STORES = !std::is_same<S, NoStores>::value;
+    const int lane = threadIdx.x & 31;
+    WarpMem<RH> *w = reinterpret_cast<WarpMem<RH> *>(smem) + (threadIdx.x >> 5);
+    for (;;) {
+        __syncwarp();
+        int32_t u = 0;
+        if (lane == 0) u = atomicAdd(&g.ctl[0], 1);
+        u = __shfl_sync(0xffffffffu, u, 0);
+        const int64_t nunits = g.nunits_dev ? *g.nunits_dev : g.nunits;
+        if (u >= nunits || ld_volatile(&g.ctl[2]) != 0) break;
+        const BatchPair d = g.pairs[g.unit_pair[u]];
+        PairView<S> v;
+        make_view(g, d, tab, 512 / (32 * RH), v);
+        init_warp(w, lane, g.open);
+        const int32_t strip = g.unit_strip ? g.unit_strip[u] : u - d.unit0;
+        const int32_t rc = tab ? run_strip2<RH, true, STORES>(v, w, lane, strip) : run_strip2<RH, false, STORES>(v, w, lane, strip);
+        if (rc != kErrNone) {
+            if (lane == 0) {
+                atomicCAS(&g.ctl[1], kErrNone, rc);
+                atomicExch(&g.ctl[2], 1);
+            }
+            break;
+        }
+        if (lane == 0) {
+            BestRec r;
+            r.ho = w->best_ho;
+            r.valid = w->best_valid;
+            r.key = w->best_key;
+            r.row = w->best_row;
+            r.col = w->best_col;
+            g.ubest[d.ufirst + strip] = r;
+        }
+    }
+}
+
+template <int RH, class S>
+__global__ void __launch_bounds__(kWarps * 32, 4) batch_packed_kernel(BatchArgs g, int tab) {
+    packed_body<RH, S>(g, tab != 0);
+}
+
+// The graphed form (see batch_graph_kernel below); the mode is read from the header.
+template <int RH, class S>
+__global__ void __launch_bounds__(kWarps * 32, 4) batch_packed_graph_kernel(BatchArgs g, const GraphHdr *h) {
+    packed_body<RH, S>(g, h->tab != 0);
 }
 
 template <int R, bool TAB, class S>
@@ -346,23 +404,54 @@ __global__ void batch_encode_kernel(const uint8_t *seq, int64_t bytes, const uin
     }
 }
 
-template <int R, bool TAB, class S>
-int max_blocks() {
+// The kernel of a launch: rows per lane R, table or compare scores, packed or 32-bit
+// strips, direct or graphed form.
+struct KernelRef {
+    const void *fn = nullptr;
+    size_t smem = 0;
+};
+template <class S>
+KernelRef kernel_ref(int R, bool tab, bool packed, bool graph) {
+    if (packed) {
+        if constexpr (std::is_same<S, WithBounds>::value) {  // level-1 recompute: direct, 512-row strips
+            return {(const void *)batch_packed_kernel<8, S>, kWarps * sizeof(WarpMem<8>)};
+        } else {
+            if (R == 8)
+                return {graph ? (const void *)batch_packed_graph_kernel<4, S> : (const void *)batch_packed_kernel<4, S>,
+                        kWarps * sizeof(WarpMem<4>)};
+            return {graph ? (const void *)batch_packed_graph_kernel<8, S> : (const void *)batch_packed_kernel<8, S>,
+                    kWarps * sizeof(WarpMem<8>)};
+        }
+    }
+    if constexpr (std::is_same<S, NoStores>::value) {
+        if (R == 8) {
+            if (graph) return {tab ? (const void *)batch_graph_kernel<8, true, S> : (const void *)batch_graph_kernel<8, false, S>, 0};
+            return {tab ? (const void *)batch_kernel<8, true, S> : (const void *)batch_kernel<8, false, S>, 0};
+        }
+    }
+    if constexpr (!std::is_same<S, WithBounds>::value) {
+        if (graph) return {tab ? (const void *)batch_graph_kernel<16, true, S> : (const void *)batch_graph_kernel<16, false, S>, 0};
+    }
+    return {tab ? (const void *)batch_kernel<16, true, S> : (const void *)batch_kernel<16, false, S>, 0};
+}
+KernelRef kernel_of(BatchMode mode, int R, bool tab, bool packed, bool graph) {
+    if (mode == kBatchBounds) return kernel_ref<WithBounds>(R, tab, packed, false);
+    if (mode == kBatchStores) return kernel_ref<WithStores>(R, tab, packed, graph);
+    return kernel_ref<NoStores>(R, tab, packed, graph);
+}
+
+int max_blocks(const KernelRef &k) {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_kernel<R, TAB, S>, kWarps * 32, 0) != cudaSuccess)
-        return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn, kWarps * 32, k.smem) != cudaSuccess) return 0;
     return nb;
 }
 
-template <int R, bool TAB, class S>
-cudaError_t launch(const BatchArgs &a, int sms, int cap, cudaStream_t st) {
-    const int per_sm = std::max(1, max_blocks<R, TAB, S>());
-    const int64_t need = (a.nunits + kWarps - 1) / kWarps;
-    int64_t limit = (int64_t)per_sm * sms;
+// Blocks of a launch of at most `units` units.
+int grid_for(const KernelRef &k, int sms, int cap, int64_t units) {
+    int64_t limit = (int64_t)std::max(1, max_blocks(k)) * sms;
     if (cap > 0 && cap < limit) limit = cap;
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(need, limit));
-    batch_kernel<R, TAB, S><<<blocks, kWarps * 32, 0, st>>>(a);
-    return cudaGetLastError();
+    const int64_t need = (units + kWarps - 1) / kWarps;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(need, limit));
 }
 
 }  // namespace
@@ -371,58 +460,22 @@ cudaError_t batch_configure() {
     const int c = cudaSharedmemCarveoutMaxShared;
     const auto A = cudaFuncAttributePreferredSharedMemoryCarveout;
     cudaError_t e = cudaSuccess;
-    for (cudaError_t x : {cudaFuncSetAttribute((const void *)batch_kernel<8, false, NoStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_kernel<8, true, NoStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_kernel<16, false, NoStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_kernel<16, true, NoStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_kernel<16, false, WithStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_kernel<16, true, WithStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_kernel<16, false, WithBounds>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_kernel<16, true, WithBounds>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_graph_kernel<8, false, NoStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_graph_kernel<8, true, NoStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_graph_kernel<16, false, NoStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_graph_kernel<16, true, NoStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_graph_kernel<16, false, WithStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_graph_kernel<16, true, WithStores>, A, c),
-                          cudaFuncSetAttribute((const void *)batch_reduce_kernel, A, c),
+    for (BatchMode mode : {kBatchScore, kBatchStores, kBatchBounds})
+        for (int R : {8, 16})
+            for (int v = 0; v < 8; ++v) {
+                const KernelRef k = kernel_of(mode, R, v & 1, v & 2, v & 4);
+                cudaError_t x = cudaFuncSetAttribute(k.fn, A, c);
+                if (x == cudaSuccess && k.smem > 0)
+                    x = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+                if (x != cudaSuccess) e = x;
+            }
+    for (cudaError_t x : {cudaFuncSetAttribute((const void *)batch_reduce_kernel, A, c),
                           cudaFuncSetAttribute((const void *)batch_encode_kernel, A, c)})
         if (x != cudaSuccess) e = x;
     return e;
 }
 
-namespace {
-
-template <int R, bool TAB, class S>
-int graph_grid(int sms, int cap) {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_graph_kernel<R, TAB, S>, kWarps * 32, 0) != cudaSuccess)
-        nb = 1;
-    int64_t g = (int64_t)std::max(1, nb) * sms;
-    if (cap > 0 && cap < g) g = cap;
-    return (int)std::max<int64_t>(1, g);
-}
-
-template <int R, class S>
-cudaError_t graph_scoring(const GraphHdr *h, int sms, int cap, int64_t max_units, cudaStream_t st) {
-    const BatchArgs placeholder{};  // replaced before the first replay
-    const int64_t need = std::max<int64_t>(1, (max_units + kWarps - 1) / kWarps);
-    const int gt = (int)std::min<int64_t>(graph_grid<R, true, S>(sms, cap), need);
-    const int gc = (int)std::min<int64_t>(graph_grid<R, false, S>(sms, cap), need);
-    batch_graph_kernel<R, true, S><<<gt, kWarps * 32, 0, st>>>(placeholder, h);
-    batch_graph_kernel<R, false, S><<<gc, kWarps * 32, 0, st>>>(placeholder, h);
-    return cudaGetLastError();
-}
-
-template <int R, class S>
-void scoring_funcs(const void **f) {
-    f[0] = (const void *)batch_graph_kernel<R, true, S>;
-    f[1] = (const void *)batch_graph_kernel<R, false, S>;
-}
-
-}  // namespace
-
-cudaError_t batch_graph_enqueue(const GraphHdr *d_hdr, bool traced, int R, int sms, int max_blocks,
+cudaError_t batch_graph_enqueue(const GraphHdr *d_hdr, bool traced, bool packed, int R, int sms, int max_blocks,
                                 int64_t max_units, cudaEvent_t ev_mid, cudaStream_t st) {
     // grid-stride kernels: up to 4 blocks of 256 threads per SM, fewer for small batches
     const int wide = (int)std::min<int64_t>(4LL * std::max(1, sms), std::max<int64_t>(std::max(1, sms) / 4, max_units / 8));
@@ -430,10 +483,12 @@ cudaError_t batch_graph_enqueue(const GraphHdr *d_hdr, bool traced, int R, int s
     graph_decide_kernel<<<1, 256, 0, st>>>(const_cast<GraphHdr *>(d_hdr));
     graph_encode_kernel<<<wide, 256, 0, st>>>(d_hdr);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (traced) e = graph_scoring<16, WithStores>(d_hdr, sms, max_blocks, max_units, st);
-    else if (R == 8) e = graph_scoring<8, NoStores>(d_hdr, sms, max_blocks, max_units, st);
-    else e = graph_scoring<16, NoStores>(d_hdr, sms, max_blocks, max_units, st);
+    BatchArgs placeholder{};  // replaced before the first replay
+    void *args[] = {&placeholder, &d_hdr};
+    for (int k = 0; k < (packed ? 1 : 2) && e == cudaSuccess; ++k) {
+        const KernelRef f = kernel_of(traced ? kBatchStores : kBatchScore, R, k == 0, packed, true);
+        e = cudaLaunchKernel(f.fn, dim3(grid_for(f, sms, max_blocks, max_units)), dim3(kWarps * 32), args, f.smem, st);
+    }
     if (e != cudaSuccess) return e;
     graph_reduce_kernel<<<wide, 256, 0, st>>>(d_hdr);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -441,10 +496,8 @@ cudaError_t batch_graph_enqueue(const GraphHdr *d_hdr, bool traced, int R, int s
     return e;
 }
 
-void batch_graph_scoring_funcs(bool traced, int R, const void **f) {
-    if (traced) scoring_funcs<16, WithStores>(f);
-    else if (R == 8) scoring_funcs<8, NoStores>(f);
-    else scoring_funcs<16, NoStores>(f);
+void batch_graph_scoring_funcs(bool traced, bool packed, int R, const void **f) {
+    for (int k = 0; k < 2; ++k) f[k] = kernel_of(traced ? kBatchStores : kBatchScore, R, k == 0, packed, true).fn;
 }
 
 int batch_score_rows_per_lane() {
@@ -456,33 +509,25 @@ int batch_score_rows_per_lane() {
     return 16;
 }
 
-int batch_max_blocks_per_sm(bool tab, BatchMode mode) {
-    if (mode == kBatchBounds) return tab ? max_blocks<16, true, WithBounds>() : max_blocks<16, false, WithBounds>();
-    if (mode == kBatchStores) return tab ? max_blocks<16, true, WithStores>() : max_blocks<16, false, WithStores>();
-    return tab ? max_blocks<16, true, NoStores>() : max_blocks<16, false, NoStores>();
+int batch_max_blocks_per_sm(bool tab, BatchMode mode, bool packed) {
+    return max_blocks(kernel_of(mode, kBatchR, tab, packed, false));
 }
 
-int batch_resident_warps(bool tab, BatchMode mode, int sms, int max_blocks) {
-    int64_t blocks = (int64_t)std::max(1, batch_max_blocks_per_sm(tab, mode)) * sms;
-    if (max_blocks > 0 && max_blocks < blocks) blocks = max_blocks;
+int batch_resident_warps(bool tab, BatchMode mode, bool packed, int sms, int cap) {
+    int64_t blocks = (int64_t)std::max(1, batch_max_blocks_per_sm(tab, mode, packed)) * sms;
+    if (cap > 0 && cap < blocks) blocks = cap;
     return (int)(blocks * kWarps);
 }
 
-cudaError_t batch_launch(const BatchArgs &a, bool tab, BatchMode mode, int R, int sms, int max_blocks, int64_t npairs,
+cudaError_t batch_launch(const BatchArgs &a, bool tab, BatchMode mode, bool packed, int R, int sms, int cap, int64_t npairs,
                          BestRec *pbest, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     if (a.nunits > 0) {
-        if (mode == kBatchBounds)
-            e = tab ? launch<16, true, WithBounds>(a, sms, max_blocks, st)
-                    : launch<16, false, WithBounds>(a, sms, max_blocks, st);
-        else if (mode == kBatchStores)
-            e = tab ? launch<16, true, WithStores>(a, sms, max_blocks, st)
-                    : launch<16, false, WithStores>(a, sms, max_blocks, st);
-        else if (R == 8)
-            e = tab ? launch<8, true, NoStores>(a, sms, max_blocks, st) : launch<8, false, NoStores>(a, sms, max_blocks, st);
-        else
-            e = tab ? launch<16, true, NoStores>(a, sms, max_blocks, st)
-                    : launch<16, false, NoStores>(a, sms, max_blocks, st);
+        const KernelRef k = kernel_of(mode, R, tab, packed, false);
+        BatchArgs args = a;
+        int table = tab ? 1 : 0;
+        void *params[] = {&args, &table};
+        e = cudaLaunchKernel(k.fn, dim3(grid_for(k, sms, cap, a.nunits)), dim3(kWarps * 32), params, k.smem, st);
         if (e != cudaSuccess) return e;
     }
     if (npairs > 0) {

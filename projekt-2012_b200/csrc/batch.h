@@ -137,29 +137,32 @@ struct GraphHdr {
 // the scoring kernel keeps every pair's special rows and columns.  Grids are
 // sized for calls of at most max_units work units (and pairs).  ev_mid, if
 // non-null, is recorded (as an external event) after the merge.
-cudaError_t batch_graph_enqueue(const GraphHdr *d_hdr, bool traced, int R, int sms, int max_blocks,
+cudaError_t batch_graph_enqueue(const GraphHdr *d_hdr, bool traced, bool packed, int R, int sms, int max_blocks,
                                 int64_t max_units, cudaEvent_t ev_mid, cudaStream_t st);
-// The two scoring kernels of such a graph (table path, compare path): their
+// The scoring kernels of such a graph (table path, compare path; the same one for
+// both with packed strips): their
 // parameters (BatchArgs, header address) are set on the instantiated graph
 // before every replay.
-void batch_graph_scoring_funcs(bool traced, int R, const void **f);
+void batch_graph_scoring_funcs(bool traced, bool packed, int R, const void **f);
 
 // Launches the batched wavefront over units [0, a.nunits) (a.ctl must be zeroed
 // first), then merges the strips' best cells of pairs [0, npairs) of a.pairs
 // into pbest[slot] (which holds the pair's best so far, or an invalid record).
 // Every strip a launch runs must have its predecessor strip either earlier in the
 // same launch's unit order or finished by an earlier launch.  `mode` selects
-// what is stored.  max_blocks > 0 caps the grid (the rest of the GPU stays free
+// what is stored.  packed: strips of 32 R rows in packed 16-bit lanes (strip16_fits
+// must hold; an error code of kStage1Range asks for the launch again without).
+// max_blocks > 0 caps the grid (the rest of the GPU stays free
 // for other work).
-cudaError_t batch_launch(const BatchArgs &a, bool tab, BatchMode mode, int R, int sms, int max_blocks,
+cudaError_t batch_launch(const BatchArgs &a, bool tab, BatchMode mode, bool packed, int R, int sms, int max_blocks,
                          int64_t npairs, BestRec *pbest, cudaStream_t st);
 // Byte presence flags over a buffer (TAB-mode choice) and the TAB encodings of
 // every byte of seq (rcode[i] = lut[seq[i]], ctab[i] = table word of seq[i]).
 cudaError_t batch_encode(const uint8_t *seq, int64_t bytes, const uint8_t *d_lut, uint8_t *rcode, uint32_t *ctab,
                          int32_t mt1, int32_t mm1, uint32_t *tab_hi, cudaStream_t st);
-int batch_max_blocks_per_sm(bool tab, BatchMode mode);
+int batch_max_blocks_per_sm(bool tab, BatchMode mode, bool packed);
 // Warps of a full batched launch of that mode (the grid batch_launch uses at most).
-int batch_resident_warps(bool tab, BatchMode mode, int sms, int max_blocks);
+int batch_resident_warps(bool tab, BatchMode mode, bool packed, int sms, int max_blocks);
 // Rows per lane of score-only batched launches (16 unless SWB_BATCH_R overrides).
 int batch_score_rows_per_lane();
 

@@ -21,6 +21,10 @@
 namespace swb {
 namespace {
 
+// Internal result of a pass with packed strips whose 16-bit window did not hold:
+// the batch runs again with 32-bit strips.
+constexpr int kRangeAgain = -1;
+
 struct PairInfo {
     int64_t row_off, col_off;
     int64_t m, n;
@@ -134,8 +138,8 @@ void claim_order(const std::vector<int32_t> &nstrips, const std::vector<int32_t>
 // one record per entry of bp (slot k).  strip_major: claim the strips in
 // claim_order instead of pair by pair.
 int run_launch(swb_ctx *c, const uint8_t *d_seq, bool tab, const BatchArgs &base, std::vector<BatchPair> &bp,
-               std::vector<int32_t> &unit_pair, int64_t hbuf_entries, bool stores, int R, std::vector<BestRec> &pbest,
-               float *ms, bool strip_major = false) {
+               std::vector<int32_t> &unit_pair, int64_t hbuf_entries, bool stores, bool packed, int R,
+               std::vector<BestRec> &pbest, float *ms, bool strip_major = false) {
     cudaError_t e;
     const int64_t np = (int64_t)bp.size(), nu = (int64_t)unit_pair.size();
     std::vector<int32_t> us;
@@ -147,7 +151,7 @@ int run_launch(swb_ctx *c, const uint8_t *d_seq, bool tab, const BatchArgs &base
             nc[(size_t)k] = bp[(size_t)k].n;
             rect += (double)bp[(size_t)k].m * (double)bp[(size_t)k].n;
         }
-        const int warps = std::max(1, batch_resident_warps(tab, stores ? kBatchStores : kBatchScore, c->sms,
+        const int warps = std::max(1, batch_resident_warps(tab, stores ? kBatchStores : kBatchScore, packed, c->sms,
                                                           c->max_blocks));
         up.reserve((size_t)nu);
         us.reserve((size_t)nu);
@@ -189,7 +193,7 @@ int run_launch(swb_ctx *c, const uint8_t *d_seq, bool tab, const BatchArgs &base
         (e = cudaMemsetAsync(a.ctl, 0, 4 * sizeof(int32_t), c->stream)) != cudaSuccess)
         return ctx_cuda_fail(c, e, "batch set-up");
     cudaEventRecord(c->ev0, c->stream);
-    if ((e = batch_launch(a, tab, stores ? kBatchStores : kBatchScore, R, c->sms, c->max_blocks, np,
+    if ((e = batch_launch(a, tab, stores ? kBatchStores : kBatchScore, packed, R, c->sms, c->max_blocks, np,
                           (BestRec *)c->b_pbest.p, c->stream)) !=
         cudaSuccess)
         return ctx_cuda_fail(c, e, "batch launch");
@@ -203,6 +207,7 @@ int run_launch(swb_ctx *c, const uint8_t *d_seq, bool tab, const BatchArgs &base
         (e = cudaStreamSynchronize(c->stream)) != cudaSuccess)
         return ctx_cuda_fail(c, e, "batch");
     std::memcpy(ctl, hctl, sizeof ctl);
+    if (ctl[1] == kStage1Range) return kRangeAgain;
     if (ctl[1] != 0) return ctx_fail(c, SWB_ETIMEOUT, "batch: a bounded wait between strips ran out");
     std::memcpy(pbest.data(), hs, sizeof(BestRec) * (size_t)np);
     float t = 0.f;
@@ -597,20 +602,32 @@ struct PhaseLog {
 
 size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
 
+// Rows per lane of a packed batched pass over the pairs `order`: 256-row strips (8)
+// while every one of them has a scheduler to itself (their step is the shortest and
+// latency decides), 512-row strips (16) beyond that.
+int packed_strip_rows(swb_ctx *c, const std::vector<PairInfo> &info, const std::vector<int64_t> &order, bool stores) {
+    if (!stores && std::getenv("SWB_BATCH_R")) return batch_score_rows_per_lane();
+    const int64_t slots = 4LL * (c->max_blocks > 0 ? std::min(c->max_blocks, c->sms) : c->sms);
+    int64_t strips = 0;
+    for (int64_t i : order)
+        if ((strips += (info[(size_t)i].m + 255) / 256) > slots) return 16;
+    return 8;
+}
+
 size_t pow2_at_least(size_t x) {
     size_t p = 1 << 16;
     while (p < x) p <<= 1;
     return p;
 }
 
-// The instantiated graph for a shape (traced or not, wide block recomputes, rows per
-// lane, grid cap, size class: grids sized for at most 2^size_class work units and pairs),
+// The instantiated graph for a shape (traced or not, wide block recomputes, packed or
+// 32-bit strips, rows per lane, grid cap, size class: grids sized for at most 2^size_class work units and pairs),
 // captured on first use.  Its kernels read the call header at c->g_hdr.p, so the
 // graph never changes for a shape; the scoring kernels' parameters are set per
 // replay (graph_set_scoring).
-cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, int R, int cap, int size_class, swb_ctx::GraphEntry **out) {
+cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, bool packed, int R, int cap, int size_class, swb_ctx::GraphEntry **out) {
     for (auto &g : c->graphs)
-        if (g.exec && g.traced == (int)traced && g.wide == (int)wide && g.R == R && g.cap == cap && g.size_class == size_class) {
+        if (g.exec && g.traced == (int)traced && g.wide == (int)wide && g.packed == (int)packed && g.R == R && g.cap == cap && g.size_class == size_class) {
             *out = &g;
             return cudaSuccess;
         }
@@ -621,7 +638,7 @@ cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, int R, int cap, int si
     const GraphHdr *h = (const GraphHdr *)c->g_hdr.p;
     if ((e = cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
     cudaError_t q = cudaEventRecordWithFlags(c->ev0, c->cap_stream, cudaEventRecordExternal);
-    if (q == cudaSuccess) q = batch_graph_enqueue(h, traced, R, c->sms, cap, max_units, c->ev1, c->cap_stream);
+    if (q == cudaSuccess) q = batch_graph_enqueue(h, traced, packed, R, c->sms, cap, max_units, c->ev1, c->cap_stream);
     if (q == cudaSuccess && traced) q = tb::walk_graph_enqueue(h, wide, c->sms, max_units, c->cap_stream);
     if (q == cudaSuccess && traced) q = cudaEventRecordWithFlags(c->ev2, c->cap_stream, cudaEventRecordExternal);
     cudaGraph_t graph = nullptr;
@@ -632,7 +649,7 @@ cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, int R, int cap, int si
     cudaKernelNodeParams skp[2] = {};
     if (e == cudaSuccess) {
         const void *f[2];
-        batch_graph_scoring_funcs(traced, R, f);
+        batch_graph_scoring_funcs(traced, packed, R, f);
         size_t nn = 0;
         e = cudaGraphGetNodes(graph, nullptr, &nn);
         std::vector<cudaGraphNode_t> nodes(nn);
@@ -679,6 +696,7 @@ cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, int R, int cap, int si
     slot->args_valid = false;
     slot->traced = traced;
     slot->wide = wide;
+    slot->packed = packed;
     slot->R = R;
     slot->cap = cap;
     slot->size_class = size_class;
@@ -731,10 +749,10 @@ struct GraphPass {
 // score), and one copy brings the results back.
 int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::vector<PairInfo> &info,
                const std::vector<int64_t> &order, const swb_scoring *sc, uint32_t flags, bool traced,
-               swb_batch_result *out, GraphPass &gp) {
+               bool packed, swb_batch_result *out, GraphPass &gp) {
     cudaError_t e;
     PhaseLog ph(c);
-    const int R = traced ? kBatchR : batch_score_rows_per_lane();
+    const int R = packed ? packed_strip_rows(c, info, order, traced) : (traced ? kBatchR : batch_score_rows_per_lane());
     std::vector<int32_t> unit_pair;
     int64_t hb = 0, srn = 0, scn = 0, ops_total = 0, xp_total = 0;
     layout_units(info, order, flags, 32 * R, gp.bp, unit_pair, &hb);
@@ -871,7 +889,7 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
         size_class = std::min(size_class, full);
     }
     swb_ctx::GraphEntry *ge = nullptr;
-    if ((e = graph_for(c, traced, traced && !tb::walk16_fits(*sc), R, c->max_blocks, size_class, &ge)) != cudaSuccess ||
+    if ((e = graph_for(c, traced, traced && !tb::walk16_fits(*sc), packed, R, c->max_blocks, size_class, &ge)) != cudaSuccess ||
         (e = graph_set_scoring(c, ge, g.ba)) != cudaSuccess)
         return ctx_cuda_fail(c, e, "batch graph");
     uint8_t *hout = (uint8_t *)c->h_gout.p;
@@ -883,6 +901,7 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
         return ctx_cuda_fail(c, e, "batch graph replay");
     ph.mark("graph: copies + replay");
     const int32_t *ctl = (const int32_t *)(hout + o_ctl);
+    if (ctl[1] == kStage1Range) return kRangeAgain;
     if (ctl[1] != 0) return ctx_fail(c, SWB_ETIMEOUT, "batch: a bounded wait between strips ran out");
     gp.tab = ctl[4] != 0;
     gp.d_seq = g.ba.seq;
@@ -905,9 +924,9 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
     return SWB_OK;
 }
 
-int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t seq_bytes, const swb_pair_ref *pairs,
-              int64_t npairs, const swb_scoring *sc, uint32_t flags, double trace_frac, swb_batch_result *out,
-              bool stores_first) {
+int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t seq_bytes,
+                     const swb_pair_ref *pairs, int64_t npairs, const swb_scoring *sc, uint32_t flags, double trace_frac,
+                     swb_batch_result *out, bool stores_first, bool wide) {
     const auto t0 = std::chrono::steady_clock::now();
     PhaseLog ph(c);
     std::memset(out, 0, sizeof *out);
@@ -941,6 +960,9 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
                                   (long double)(maxlen + 2);
         if (worst > 2.0e9L) return ctx_fail(c, SWB_EUNSUPPORTED, "scores would leave the int32 range");
     }
+    // strips in packed 16-bit lanes unless the scoring is too wide for their window
+    const char *pack_env = std::getenv("SWB_STAGE1_PACK");
+    const bool packed = !wide && strip16_fits(*sc, kBatchR, maxlen) && !(pack_env && pack_env[0] == '0');
     out->npairs = npairs;
     out->cells = cells;
     out->items = (swb_batch_item *)std::calloc((size_t)std::max<int64_t>(1, npairs), sizeof(swb_batch_item));
@@ -974,7 +996,7 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
     GraphPass gp;
     ph.mark("orient + order");
     if (use_graph) {
-        int rc = graph_pass(c, h_seq, seq_bytes, info, order, sc, flags, stores_first, out, gp);
+        int rc = graph_pass(c, h_seq, seq_bytes, info, order, sc, flags, stores_first, packed, out, gp);
         if (rc != SWB_OK) return rc;
     }
 
@@ -1025,7 +1047,7 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
             base.ctab = gp.ctab;
             base.tab_hi = (uint32_t)(uint8_t)(int8_t)base.mm1 * 0x01010101u;
         }
-        launches += stores_first ? 8 : 6;
+        launches += (stores_first ? 8 : 6) - (packed ? 1 : 0);
     } else if (!order.empty() && base.mt1 >= -128 && base.mt1 <= 127 && base.mm1 >= -128 && base.mm1 <= 127) {
         // TAB mode when the whole buffer holds at most four distinct bytes
         uint32_t present[256];
@@ -1067,7 +1089,8 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
     int64_t hb = 0, srn = 0, scn = 0, ops_total = 0, xp_total = 0;
     float ms1 = 0.f;
     const bool first_stores = stores_first && !order.empty();
-    const int R1 = first_stores ? kBatchR : batch_score_rows_per_lane();
+    const int R1 = packed ? packed_strip_rows(c, info, order, first_stores)
+                          : (first_stores ? kBatchR : batch_score_rows_per_lane());
     if (use_graph) {
         bp = gp.bp;
         pbest = gp.pbest;
@@ -1100,7 +1123,7 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
             std::vector<BestRec> pb2;
             int64_t hb2 = 0;
             layout_units(info, sub, flags, 32 * R1, bp2, up2, &hb2);
-            rc = run_launch(c, d_seq, tab, base, bp2, up2, hb2, false, R1, pb2, &ms1, true);
+            rc = run_launch(c, d_seq, tab, base, bp2, up2, hb2, false, packed, R1, pb2, &ms1, true);
             if (rc != SWB_OK) return rc;
             launches += 2;
             for (size_t i = 0; i < rest.size(); ++i) pbest[(size_t)rest[i]] = pb2[i];
@@ -1114,7 +1137,7 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
             a1.srows = (int2 *)c->b_srows.p;
             a1.scols = (int2 *)c->b_scols.p;
         }
-        int rc = run_launch(c, d_seq, tab, a1, bp, unit_pair, hb, first_stores, R1, pbest, &ms1, true);
+        int rc = run_launch(c, d_seq, tab, a1, bp, unit_pair, hb, first_stores, packed, R1, pbest, &ms1, true);
         if (rc != SWB_OK) return rc;
         launches += 2;
     }
@@ -1172,7 +1195,8 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
             std::vector<std::pair<int64_t, int64_t>> ext(tr.size());
             for (size_t k = 0; k < tr.size(); ++k)
                 ext[k] = {out->items[tr[k]].end_row + 1, out->items[tr[k]].end_col + 1};
-            layout_units(info, tr, flags, kBatchStripRows, bpw, up2, &hb2, &ext);
+            const int R2 = packed ? packed_strip_rows(c, info, tr, true) : kBatchR;
+            layout_units(info, tr, flags, 32 * R2, bpw, up2, &hb2, &ext);
             layout_stores(bpw, out->items, tr, &srn, &scn, &ops_total, &xp_total);
             int rc = ensure_stores(srn, scn);
             if (rc != SWB_OK) return rc;
@@ -1181,7 +1205,7 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
             b2.scols = (int2 *)c->b_scols.p;
             std::vector<BestRec> pb2;
             float ms2 = 0.f;
-            rc = run_launch(c, d_seq, tab, b2, bpw, up2, hb2, true, kBatchR, pb2, &ms2, true);
+            rc = run_launch(c, d_seq, tab, b2, bpw, up2, hb2, true, packed, R2, pb2, &ms2, true);
             if (rc != SWB_OK) return rc;
             launches += 2;
             for (size_t k = 0; k < tr.size(); ++k) {
@@ -1346,6 +1370,18 @@ int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, int64_t
 }
 
 }  // namespace
+
+// Packed strips first, 32-bit ones if a window did not hold.
+static int batch_run(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq, int64_t seq_bytes, const swb_pair_ref *pairs,
+                     int64_t npairs, const swb_scoring *sc, uint32_t flags, double trace_frac, swb_batch_result *out,
+                     bool stores_first) {
+    int rc = batch_run_strips(c, h_seq, d_seq, seq_bytes, pairs, npairs, sc, flags, trace_frac, out, stores_first, false);
+    if (rc == kRangeAgain) {
+        swb_batch_result_free(out);
+        rc = batch_run_strips(c, h_seq, d_seq, seq_bytes, pairs, npairs, sc, flags, trace_frac, out, stores_first, true);
+    }
+    return rc;
+}
 
 int batch_align_all_traced(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const swb_pair_ref *pairs,
                            int64_t npairs, const swb_scoring *sc, uint32_t flags, swb_batch_result *out) {

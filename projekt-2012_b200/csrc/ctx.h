@@ -72,7 +72,7 @@ struct swb_ctx {
         cudaKernelNodeParams kp[2] = {};     // their launch shapes
         unsigned char set_args[256] = {};    // the BatchArgs last set on them
         bool args_valid = false;
-        int traced = 0, wide = 0, R = 0, cap = 0, size_class = 0;
+        int traced = 0, wide = 0, packed = 0, R = 0, cap = 0, size_class = 0;
     };
     GraphEntry graphs[16];
     int graph_next = 0;                  // round-robin replacement when all entries are taken

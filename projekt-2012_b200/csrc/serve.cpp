@@ -329,7 +329,7 @@ int swb_server_create(const swb_server_options *opts, const swb_scoring *sc, swb
     }
     s->sms = s->cs->sms;
     if (s->o.reserve_sms >= s->sms) s->o.reserve_sms = std::max(1, s->sms / 8);
-    s->per_sm = std::max(1, swb::batch_max_blocks_per_sm(true, swb::kBatchStores));
+    s->per_sm = std::max(1, swb::batch_max_blocks_per_sm(true, swb::kBatchStores, true));
     s->ts = std::thread([s] { s->short_lane(); });
     s->tl = std::thread([s] { s->long_lane(); });
     *out = s;

@@ -77,6 +77,7 @@ int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const 
         // once by one batched launch that writes each cell's 512 x 256 stores,
         // then walked cell by cell
         const int64_t cap = level1_corridor_cells(plan, sms);
+        bool packed = strip16_fits(*sc, kBatchR, n);
         std::vector<int64_t> cells;  // (RR0, CC0) pairs
         std::vector<BatchPair> bp;
         std::vector<int32_t> up;
@@ -182,7 +183,7 @@ int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const 
                 (e = cudaMemsetAsync(dg, 0, sizeof(int32_t) * (size_t)ncell, st)) != cudaSuccess ||
                 (e = cudaMemsetAsync(dpb, 0, sizeof(BestRec) * (size_t)ncell, st)) != cudaSuccess ||
                 (e = cudaMemsetAsync(dc, 0, 4 * sizeof(int32_t), st)) != cudaSuccess ||
-                (e = batch_launch(ba, false, kBatchBounds, kBatchR, sms, 0, ncell, dpb, st)) != cudaSuccess) {
+                (e = batch_launch(ba, false, kBatchBounds, packed, kBatchR, sms, 0, ncell, dpb, st)) != cudaSuccess) {
                 err = std::string("level-1 recompute: ") + cudaGetErrorString(e);
                 return SWB_ECUDA;
             }
@@ -191,6 +192,11 @@ int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const 
             if ((e = scr.get(scr.owner, ctl, dc, sizeof ctl)) != cudaSuccess) {
                 err = std::string("level-1 recompute: ") + cudaGetErrorString(e);
                 return SWB_ECUDA;
+            }
+            if (ctl[1] == kStage1Range && packed) {  // a 16-bit window did not hold: this round again in 32 bits
+                packed = false;
+                --round;
+                continue;
             }
             if (ctl[1] != 0) {
                 err = "level-1 recompute: a bounded wait between strips ran out";
