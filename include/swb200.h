@@ -71,11 +71,9 @@ typedef struct {
  * returns SWB_ETIMEOUT with the context still usable.  Pairs of one strip (at
  * most 448 rows) have no wait and are unaffected. */
 #define SWB_FLAG_TEST_WITHHOLD 0x80000000u
-/* Test hook of swb_batch_align[_device]: the packed 16-bit scoring pass takes
- * every pair, also those whose best score may not fit 16 bits; a pair that
- * reaches the limit is detected and scored again in int32, so results do not
- * change.  Without it only pairs whose score is bounded below the limit are
- * packed. */
+/* Accepted by swb_batch_align[_device] and without effect: packed strips hold
+ * 32-bit scores (a base and 16-bit offsets), so no pair has to be kept out of
+ * them. */
 #define SWB_FLAG_TEST_PACK_ANY 0x40000000u
 
 typedef struct {

@@ -201,7 +201,6 @@ int swb_ctx_create(const swb_options *opts, swb_ctx **out) {
         (e = cudaEventCreate(&c->ev0)) != cudaSuccess || (e = cudaEventCreate(&c->ev1)) != cudaSuccess ||
         (e = cudaEventCreate(&c->ev2)) != cudaSuccess ||
         (e = swb::stage1_configure()) != cudaSuccess || (e = swb::batch_configure()) != cudaSuccess ||
-        (e = swb::batch16_configure()) != cudaSuccess ||
         (e = swb::tb::walker_configure()) != cudaSuccess) {
         int rc = ctx_cuda_fail(nullptr, e, "swb_ctx_create");
         // release what was created before the failure

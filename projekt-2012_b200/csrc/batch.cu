@@ -189,24 +189,32 @@ __device__ __forceinline__ void packed_body(const BatchArgs &g, bool tab) {
         const BatchPair d = g.pairs[g.unit_pair[u]];
         PairView<S> v;
         make_view(g, d, tab, 512 / (32 * RH), v);
-        init_warp(w, lane, g.open);
-        const int32_t strip = g.unit_strip ? g.unit_strip[u] : u - d.unit0;
-        const int32_t rc = tab ? run_strip2<RH, true, STORES>(v, w, lane, strip) : run_strip2<RH, false, STORES>(v, w, lane, strip);
+        // one strip, or every strip of a whole pair in turn (the strip above is always
+        // complete, so no wait spins)
+        const int32_t first = g.unit_strip ? g.unit_strip[u] : u - d.unit0;
+        const int32_t s0 = first == kWholePair ? 0 : first, s1 = first == kWholePair ? d.nstrips : first + 1;
+        int32_t rc = kErrNone;
+#pragma unroll 1
+        for (int32_t strip = s0; strip < s1 && rc == kErrNone; ++strip) {
+            init_warp(w, lane, g.open);
+            rc = tab ? run_strip2<RH, true, STORES>(v, w, lane, strip) : run_strip2<RH, false, STORES>(v, w, lane, strip);
+            if (rc == kErrNone && lane == 0) {
+                BestRec r;
+                r.ho = w->best_ho;
+                r.valid = w->best_valid;
+                r.key = w->best_key;
+                r.row = w->best_row;
+                r.col = w->best_col;
+                g.ubest[d.ufirst + strip] = r;
+            }
+            __syncwarp();
+        }
         if (rc != kErrNone) {
             if (lane == 0) {
                 atomicCAS(&g.ctl[1], kErrNone, rc);
                 atomicExch(&g.ctl[2], 1);
             }
             break;
-        }
-        if (lane == 0) {
-            BestRec r;
-            r.ho = w->best_ho;
-            r.valid = w->best_valid;
-            r.key = w->best_key;
-            r.row = w->best_row;
-            r.col = w->best_col;
-            g.ubest[d.ufirst + strip] = r;
         }
     }
 }
@@ -416,6 +424,8 @@ KernelRef kernel_ref(int R, bool tab, bool packed, bool graph) {
         if constexpr (std::is_same<S, WithBounds>::value) {  // level-1 recompute: direct, 512-row strips
             return {(const void *)batch_packed_kernel<8, S>, kWarps * sizeof(WarpMem<8>)};
         } else {
+            if constexpr (std::is_same<S, NoStores>::value)
+                if (R == 14) return {(const void *)batch_packed_kernel<7, S>, kWarps * sizeof(WarpMem<7>)};  // direct only
             if (R == 8)
                 return {graph ? (const void *)batch_packed_graph_kernel<4, S> : (const void *)batch_packed_kernel<4, S>,
                         kWarps * sizeof(WarpMem<4>)};
@@ -461,7 +471,7 @@ cudaError_t batch_configure() {
     const auto A = cudaFuncAttributePreferredSharedMemoryCarveout;
     cudaError_t e = cudaSuccess;
     for (BatchMode mode : {kBatchScore, kBatchStores, kBatchBounds})
-        for (int R : {8, 16})
+        for (int R : {8, 14, 16})
             for (int v = 0; v < 8; ++v) {
                 const KernelRef k = kernel_of(mode, R, v & 1, v & 2, v & 4);
                 cudaError_t x = cudaFuncSetAttribute(k.fn, A, c);
@@ -509,12 +519,12 @@ int batch_score_rows_per_lane() {
     return 16;
 }
 
-int batch_max_blocks_per_sm(bool tab, BatchMode mode, bool packed) {
-    return max_blocks(kernel_of(mode, kBatchR, tab, packed, false));
+int batch_max_blocks_per_sm(bool tab, BatchMode mode, bool packed, int R) {
+    return max_blocks(kernel_of(mode, R, tab, packed, false));
 }
 
-int batch_resident_warps(bool tab, BatchMode mode, bool packed, int sms, int cap) {
-    int64_t blocks = (int64_t)std::max(1, batch_max_blocks_per_sm(tab, mode, packed)) * sms;
+int batch_resident_warps(bool tab, BatchMode mode, bool packed, int R, int sms, int cap) {
+    int64_t blocks = (int64_t)std::max(1, batch_max_blocks_per_sm(tab, mode, packed, R)) * sms;
     if (cap > 0 && cap < blocks) blocks = cap;
     return (int)(blocks * kWarps);
 }

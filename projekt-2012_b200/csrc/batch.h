@@ -35,6 +35,9 @@ enum BatchMode : int32_t {
     kBatchBounds = 2,      // special rows / columns of sub-rectangles with top / left boundaries
 };
 
+// A work unit of packed strips that is every strip of its pair, run in turn by one warp.
+constexpr int32_t kWholePair = -1;
+
 // Uniform arguments of one batched launch.
 struct BatchArgs {
     const uint8_t *seq;        // sequence bytes of the rows (CMP mode)
@@ -45,7 +48,7 @@ struct BatchArgs {
     uint32_t tab_hi;
     const BatchPair *pairs;
     const int32_t *unit_pair;  // work unit -> index into pairs; units are claimed in this order
-    const int32_t *unit_strip; // if set, work unit -> strip of its pair; else the strip is u - unit0
+    const int32_t *unit_strip; // if set, work unit -> strip of its pair, or kWholePair; else the strip is u - unit0
     int64_t nunits;
     const int64_t *nunits_dev; // if set, the unit count is read here (graphed launches) instead
     int4 *hbuf;
@@ -56,51 +59,10 @@ struct BatchArgs {
     int64_t wait_limit;        // bound of each wait for the strip above, in SM clock cycles; 0 = default
 };
 
-// Two pairs scored side by side in packed 16-bit lanes (batch16.cu): half 0 is
-// pair a (low 16 bits of every lane register), half 1 pair b.  Both have the
-// same strip count; the packed rectangle is M = max(m) rows x N = max(n) columns.
-struct PackedPair {
-    int64_t row_off[2], col_off[2];  // byte offsets of each pair's rows / cols in the sequence buffer
-    int64_t hbuf_off;                // first of the N hand-off entries (packs of more than one strip)
-    int32_t m[2], n[2];              // m = n = 0: an empty half
-    int32_t M, N;
-    int32_t unit0, nstrips;          // strip s keeps its two best records at ubest[2 (unit0 + s) + half]
-    int32_t whole, pad_;             // 1: one work item, one warp runs every strip in turn;
-                                     // 0: one work item per strip, chained across warps
-    int32_t slot[2];                 // pbest / gbest / saturation slot of each half
-    TieGeom tie[2];
-};
-
-// Uniform arguments of one packed launch (TAB mode only: table words and row codes).
-struct Batch16Args {
-    const uint8_t *rcode;
-    const uint32_t *ctab;
-    uint32_t open2, ext2, gx2;  // gap_open, gap_extend, max of both in both halves
-    int32_t open;
-    uint32_t mm4;               // the table word of a column past a pair's end (a mismatch for every code)
-    int32_t sat_lim;            // a half's column maximum (H + open) at or above this flags its pair
-    const PackedPair *pairs;
-    const int2 *items;          // work item -> (packed pair, strip); claimed in this order
-    int64_t nunits;             // work items
-    int4 *hbuf;
-    int32_t *gbest;             // per slot: best H seen so far
-    BestRec *ubest;             // per strip of every packed pair: two records (half 0, half 1)
-    int32_t *ctl;               // [0] unit counter, [1] error code, [2] abort flag
-    int32_t *sat;               // per slot: 1 when the pair reached the 16-bit limit
-    int64_t wait_limit;
-};
-
-// Rows per lane of the packed kernel: 14 (448-row strips) unless the batch
-// autotuner picks 8 (256-row strips, less padding below short pairs).
+// Rows per lane of the large score-only pass's strips: 14 (448 rows) unless the
+// batch autotuner picks 8 (256 rows, less padding below short pairs).
 constexpr int kBatch16R = 14;
 constexpr int kBatch16RShort = 8;
-
-cudaError_t batch16_configure();
-// Warps of a full packed launch (the grid batch16_launch uses at most).
-int batch16_resident_warps(int R, int sms, int max_blocks);
-// R: kBatch16R or kBatch16RShort; the packed pairs' strip counts must use it.
-cudaError_t batch16_launch(const Batch16Args &a, int R, int sms, int max_blocks, int64_t npacked, BestRec *pbest,
-                           cudaStream_t st);
 
 // Rows per lane of the batched kernel's store passes (their strips are 512 rows,
 // the walker's block height); score-only passes may use 8 (256-row strips).
@@ -160,9 +122,9 @@ cudaError_t batch_launch(const BatchArgs &a, bool tab, BatchMode mode, bool pack
 // every byte of seq (rcode[i] = lut[seq[i]], ctab[i] = table word of seq[i]).
 cudaError_t batch_encode(const uint8_t *seq, int64_t bytes, const uint8_t *d_lut, uint8_t *rcode, uint32_t *ctab,
                          int32_t mt1, int32_t mm1, uint32_t *tab_hi, cudaStream_t st);
-int batch_max_blocks_per_sm(bool tab, BatchMode mode, bool packed);
+int batch_max_blocks_per_sm(bool tab, BatchMode mode, bool packed, int R = 16);
 // Warps of a full batched launch of that mode (the grid batch_launch uses at most).
-int batch_resident_warps(bool tab, BatchMode mode, bool packed, int sms, int max_blocks);
+int batch_resident_warps(bool tab, BatchMode mode, bool packed, int R, int sms, int max_blocks);
 // Rows per lane of score-only batched launches (16 unless SWB_BATCH_R overrides).
 int batch_score_rows_per_lane();
 

@@ -62,6 +62,26 @@ void sort_desc(std::vector<int64_t> &idx, Key key) {
     }
 }
 
+// The descriptor of pair p in a launch with H-row strips, of its top-left em x en
+// cells; the tie rule keeps the whole pair's geometry.
+void set_pair(BatchPair &d, const PairInfo &p, int64_t em, int64_t en, int64_t H, int32_t slot, uint32_t flags) {
+    d.row_off = p.row_off;
+    d.col_off = p.col_off;
+    d.m = (int32_t)em;
+    d.n = (int32_t)en;
+    d.nstrips = (int32_t)((em + H - 1) / H);
+    d.slot = slot;
+    d.sr_every = 1;
+    d.sc_every = 1 << 30;
+    int32_t G = 0, T = 0;
+    int64_t P1 = 0, P2 = 0;
+    const bool refok = reference_geometry(p.m, p.n, &G, &T, &P1, &P2);
+    d.tie.mode = ((flags & SWB_FLAG_TIE_ROWMAJOR) || !refok) ? kTieRowMajor : kTieReference;
+    d.tie.G = G;
+    d.tie.T = T;
+    d.tie.C = refok ? P2 / G : 1;
+}
+
 // Lays out the units of `order` (indices into info, already sorted) as one
 // launch: unit0 / ufirst / ucount / hbuf offsets; returns the unit count.
 // extent (optional, one per entry of order): compute only the top-left
@@ -76,29 +96,15 @@ int64_t layout_units(const std::vector<PairInfo> &info, const std::vector<int64_
         const PairInfo &p = info[(size_t)order[k]];
         BatchPair &d = bp[k];
         std::memset(&d, 0, sizeof d);
-        d.row_off = p.row_off;
-        d.col_off = p.col_off;
         const int64_t em = extent ? (*extent)[k].first : p.m, en = extent ? (*extent)[k].second : p.n;
-        d.m = (int32_t)em;
-        d.n = (int32_t)en;
-        d.nstrips = (int32_t)((em + strip_rows - 1) / strip_rows);
+        set_pair(d, p, em, en, strip_rows, (int32_t)k, flags);
         d.unit0 = (int32_t)units;
         d.ufirst = (int32_t)units;
         d.ucount = d.nstrips;
-        d.slot = (int32_t)k;
-        d.sr_every = 1;
-        d.sc_every = 1 << 30;
         if (d.nstrips > 1) {
             d.hbuf_off = hb;
             hb += en;
         }
-        int32_t G = 0, T = 0;
-        int64_t P1 = 0, P2 = 0;
-        const bool refok = reference_geometry(p.m, p.n, &G, &T, &P1, &P2);
-        d.tie.mode = ((flags & SWB_FLAG_TIE_ROWMAJOR) || !refok) ? kTieRowMajor : kTieReference;
-        d.tie.G = G;
-        d.tie.T = T;
-        d.tie.C = refok ? P2 / G : 1;
         for (int32_t s = 0; s < d.nstrips; ++s) unit_pair.push_back((int32_t)k);
         units += d.nstrips;
     }
@@ -136,13 +142,16 @@ void claim_order(const std::vector<int32_t> &nstrips, const std::vector<int32_t>
 
 // Runs one scoring launch (optionally the store pass) over bp; pbest receives
 // one record per entry of bp (slot k).  strip_major: claim the strips in
-// claim_order instead of pair by pair.
+// claim_order instead of pair by pair; unit_strip (with `strips` in all): unit_pair
+// is in claim order already and these are its strips.
 int run_launch(swb_ctx *c, const uint8_t *d_seq, bool tab, const BatchArgs &base, std::vector<BatchPair> &bp,
                std::vector<int32_t> &unit_pair, int64_t hbuf_entries, bool stores, bool packed, int R,
-               std::vector<BestRec> &pbest, float *ms, bool strip_major = false) {
+               std::vector<BestRec> &pbest, float *ms, bool strip_major = false,
+               const std::vector<int32_t> *unit_strip = nullptr, int64_t strips = 0) {
     cudaError_t e;
     const int64_t np = (int64_t)bp.size(), nu = (int64_t)unit_pair.size();
-    std::vector<int32_t> us;
+    std::vector<int32_t> claimed;
+    const std::vector<int32_t> &us = unit_strip ? *unit_strip : claimed;
     if (strip_major && np > 0) {
         std::vector<int32_t> ns((size_t)np), nc((size_t)np), up;
         double rect = 0.0;
@@ -151,18 +160,18 @@ int run_launch(swb_ctx *c, const uint8_t *d_seq, bool tab, const BatchArgs &base
             nc[(size_t)k] = bp[(size_t)k].n;
             rect += (double)bp[(size_t)k].m * (double)bp[(size_t)k].n;
         }
-        const int warps = std::max(1, batch_resident_warps(tab, stores ? kBatchStores : kBatchScore, packed, c->sms,
+        const int warps = std::max(1, batch_resident_warps(tab, stores ? kBatchStores : kBatchScore, packed, R, c->sms,
                                                           c->max_blocks));
         up.reserve((size_t)nu);
-        us.reserve((size_t)nu);
-        claim_order(ns, nc, rect / warps / (32.0 * R), up, us);
+        claimed.reserve((size_t)nu);
+        claim_order(ns, nc, rect / warps / (32.0 * R), up, claimed);
         unit_pair.swap(up);
     }
     const size_t bp_bytes = sizeof(BatchPair) * (size_t)np, up_bytes = sizeof(int32_t) * (size_t)nu * (us.empty() ? 1 : 2);
     if ((e = c->b_pairs.ensure(bp_bytes)) != cudaSuccess || (e = c->b_units.ensure(up_bytes)) != cudaSuccess ||
         (e = c->b_hbuf.ensure(sizeof(int4) * (size_t)std::max<int64_t>(1, hbuf_entries))) != cudaSuccess ||
         (e = c->b_gbest.ensure(sizeof(int32_t) * (size_t)np)) != cudaSuccess ||
-        (e = c->b_ubest.ensure(sizeof(BestRec) * (size_t)std::max<int64_t>(1, nu))) != cudaSuccess ||
+        (e = c->b_ubest.ensure(sizeof(BestRec) * (size_t)std::max<int64_t>(1, std::max(nu, strips)))) != cudaSuccess ||
         (e = c->b_pbest.ensure(sizeof(BestRec) * (size_t)np)) != cudaSuccess ||
         (e = c->b_ctl.ensure(4 * sizeof(int32_t))) != cudaSuccess ||
         (e = c->h_stage.ensure(std::max(bp_bytes + up_bytes, sizeof(BestRec) * (size_t)np + 64) + 64)) != cudaSuccess)
@@ -262,9 +271,9 @@ bool graphs_enabled() {
     return !(v && v[0] == '0');
 }
 
-// The packed 16-bit scoring pass (batch16.cu) serves score-only passes of
-// batches with at least this many pairs in the table (<= 4 letter) mode; the
-// smaller batches of the serving loop keep the replayed graph.
+// Score-only passes of batches with at least this many pairs are laid out and tuned
+// as a large pass (run_packed); the smaller batches of the serving loop keep the
+// replayed graph.
 constexpr int64_t kPackMinPairs = 2048;
 
 bool packing_enabled() {
@@ -272,229 +281,93 @@ bool packing_enabled() {
     return !(v && v[0] == '0');
 }
 
-// Highest H + open a half of a packed lane may reach before its pair is scored
-// again in int32; a pair whose best score is bounded by match * n + 256 below
-// it is packed without that risk.
-constexpr int32_t kSatLimit = 32767 - 256;
-
-// Which packed pairs run on one warp, strip after strip, instead of one strip
-// per warp chained through the hand-off buffer.  With far more pairs than
-// resident warps a short pair needs no pipeline across warps (whose strips
-// would each spin while the strip above gets ahead); a long one keeps it, so
-// that no single warp holds the batch's tail.  A pair runs whole when its
-// packed rectangle is at most a tenth of one warp's share of the launch's
-// cells: on the 100,000-pair batch that is about 8 strips of 448 rows
-// (packed kernel 195.4 -> 176.2 ms; whole up to 16 strips, 206.0 ms).
-// SWB_BATCH16_WHOLE=k instead runs pairs of at most k strips whole (0: none).
+// Which pairs of a large pass run on one warp, strip after strip, instead of one
+// strip per warp chained through the hand-off buffer.  With far more pairs than
+// resident warps a short pair needs no pipeline across warps (whose strips would
+// each spin while the strip above gets ahead); a long one keeps it, so that no
+// single warp holds the batch's tail.  A pair runs whole when its cells are at most
+// a tenth of one warp's share of the launch's.  SWB_BATCH16_WHOLE=k instead runs
+// pairs of at most k strips whole (0: none).
 constexpr int64_t kWholeShareDiv = 10;
 int32_t packed_whole_strips() {
     if (const char *v = std::getenv("SWB_BATCH16_WHOLE")) return std::max(0, std::atoi(v));
     return -1;
 }
 
-// Positions of `order` whose pair may run packed (its best score is bounded
-// below the 16-bit limit, or the test flag packs every pair) and the others.
-void split_packable(const std::vector<PairInfo> &info, const std::vector<int64_t> &order, const swb_scoring *sc,
-                    uint32_t flags, std::vector<int64_t> &ppos, std::vector<int64_t> &rest) {
-    for (size_t k = 0; k < order.size(); ++k) {
-        const PairInfo &p = info[(size_t)order[k]];
-        const bool fits = (int64_t)sc->match * p.n + 256 <= kSatLimit;
-        if (fits || (flags & SWB_FLAG_TEST_PACK_ANY)) ppos.push_back((int64_t)k);
-        else rest.push_back((int64_t)k);
-    }
-}
-
-// The host half of a packed pass (see layout_packed).
+// The host half of a large pass (see layout_packed).
 struct PackedLayout {
     int R = 0;                    // rows per lane it was laid out for (0: none)
     std::vector<int64_t> pos;     // the positions of `order` it covers, as given
-    std::vector<PackedPair> pp;   // packed pairs
-    std::vector<int2> up;         // work items (packed pair, strip)
-    int64_t units = 0, hb = 0;    // strips (best records) and hand-off entries
+    std::vector<BatchPair> bp;    // one per position; slot = its index
+    std::vector<int32_t> up, us;  // work units: pair, strip (or kWholePair)
+    int64_t strips = 0, hb = 0;   // strips (best records) and hand-off entries
 };
 
-// The host half of the packed pass over the positions `pos` of `order` with R
-// rows per lane: pairs sorted by strip count and width and taken two at a time
-// (a pair whose neighbour has another strip count gets an empty partner), each
-// packed pair whole or chained, and the work items in their claim order.
+// The host half of the large pass over the positions `pos` of `order` with R rows
+// per lane: each pair whole or chained, and the work units in their claim order:
+// chained pairs as claim_order says, then the whole ones, largest first (`order`
+// is), which fill the tail.
 void layout_packed(swb_ctx *c, const std::vector<PairInfo> &info, const std::vector<int64_t> &order,
-                   std::vector<int64_t> pos, uint32_t flags, int R, PackedLayout &L) {
+                   const std::vector<int64_t> &pos, uint32_t flags, int R, PackedLayout &L) {
     L.R = R;
     L.pos = pos;
     const int64_t H = 32LL * R;
     const int32_t whole_max = packed_whole_strips();  // -1: by the cell share
-    auto strips = [&](int64_t k) { return (info[(size_t)order[(size_t)k]].m + H - 1) / H; };
-    // strip count, then width, both descending
-    sort_desc(pos, [&](int64_t x) {
-        return ((uint64_t)strips(x) << 32) | (uint64_t)info[(size_t)order[(size_t)x]].n;
-    });
-    const int32_t dummy = (int32_t)order.size();  // slot of an empty half
-    std::vector<PackedPair> &pp = L.pp;
-    std::vector<int2> &up = L.up;  // work items
-    pp.clear();
-    up.clear();
-    int64_t units = 0, hb = 0;
-    for (size_t i = 0; i < pos.size();) {
-        const int64_t ka = pos[i];
-        const int64_t kb = (i + 1 < pos.size() && strips(pos[i + 1]) == strips(ka)) ? pos[i + 1] : -1;
-        i += kb >= 0 ? 2 : 1;
-        PackedPair d;
-        std::memset(&d, 0, sizeof d);
-        const int64_t ks[2] = {ka, kb};
-        for (int h = 0; h < 2; ++h) {
-            if (ks[h] < 0) {
-                d.slot[h] = dummy;
-                d.tie[h].mode = kTieRowMajor;
-                continue;
-            }
-            const PairInfo &p = info[(size_t)order[(size_t)ks[h]]];
-            d.row_off[h] = p.row_off;
-            d.col_off[h] = p.col_off;
-            d.m[h] = (int32_t)p.m;
-            d.n[h] = (int32_t)p.n;
-            d.slot[h] = (int32_t)ks[h];
-            int32_t G = 0, T = 0;
-            int64_t P1 = 0, P2 = 0;
-            const bool refok = reference_geometry(p.m, p.n, &G, &T, &P1, &P2);
-            d.tie[h].mode = ((flags & SWB_FLAG_TIE_ROWMAJOR) || !refok) ? kTieRowMajor : kTieReference;
-            d.tie[h].G = G;
-            d.tie[h].T = T;
-            d.tie[h].C = refok ? P2 / G : 1;
-        }
-        d.M = std::max(d.m[0], d.m[1]);
-        d.N = std::max(d.n[0], d.n[1]);
-        d.nstrips = (int32_t)((d.M + H - 1) / H);
-        d.unit0 = (int32_t)units;
+    double cells = 0.0;
+    for (int64_t k : pos) cells += (double)info[(size_t)order[(size_t)k]].m * (double)info[(size_t)order[(size_t)k]].n;
+    const double share = cells / std::max(1, batch_resident_warps(true, kBatchScore, true, R, c->sms, c->max_blocks));
+    L.bp.resize(pos.size());
+    L.up.clear();
+    L.us.clear();
+    L.strips = L.hb = 0;
+    std::vector<int32_t> chained, ns, nc;
+    std::vector<int32_t> whole;
+    for (size_t q = 0; q < pos.size(); ++q) {
+        const PairInfo &p = info[(size_t)order[(size_t)pos[q]]];
+        BatchPair &d = L.bp[q];
+        d = BatchPair{};
+        set_pair(d, p, p.m, p.n, H, (int32_t)q, flags);
+        d.unit0 = d.ufirst = (int32_t)L.strips;
+        d.ucount = d.nstrips;
+        L.strips += d.nstrips;
         if (d.nstrips > 1) {
-            d.hbuf_off = hb;
-            hb += d.N;
+            d.hbuf_off = L.hb;
+            L.hb += p.n;
         }
-        units += d.nstrips;
-        pp.push_back(d);
+        const bool w = whole_max >= 0 ? d.nstrips <= whole_max
+                                      : (double)p.m * (double)p.n * (double)kWholeShareDiv <= share;
+        if (w) {
+            whole.push_back((int32_t)q);
+        } else {
+            chained.push_back((int32_t)q);
+            ns.push_back(d.nstrips);
+            nc.push_back(d.n);
+        }
     }
-    // whole pairs and the work items (pairs stay in the order above)
-    double rect = 0.0;
-    for (const PackedPair &d : pp) rect += (double)d.M * (double)d.N;
-    const double share = rect / std::max(1, batch16_resident_warps(R, c->sms, c->max_blocks));
-    std::vector<int32_t> chained;  // strip counts descending, as pp
-    for (size_t q = 0; q < pp.size(); ++q) {
-        PackedPair &d = pp[q];
-        d.whole = whole_max >= 0 ? (d.nstrips <= whole_max ? 1 : 0)
-                                 : ((double)d.M * (double)d.N * (double)kWholeShareDiv <= share ? 1 : 0);
-        if (!d.whole) chained.push_back((int32_t)q);
+    claim_order(ns, nc, share / (double)H, L.up, L.us);
+    for (int32_t &u : L.up) u = chained[(size_t)u];
+    for (int32_t q : whole) {
+        L.up.push_back(q);
+        L.us.push_back(kWholePair);
     }
-    // Claim order.  A chained pair's strip s waits until strip s - 1 is about
-    // kLagSteps steps ahead; claimed pair by pair, the warps that take strips
-    // 0..s of a pair start together and strip s spins s times that long (16% of
-    // the packed pass on the 100,000-pair batch).  So the chained pairs go
-    // strip-major (strip 0 of each, then strip 1, ...), and each strip is
-    // claimed long after the one above it.  A pair whose own chain (N columns
-    // plus the lag of every strip) is at least half of one warp's share of the
-    // launch would then finish late and hold the tail: those go first, pair by
-    // pair.  Whole pairs follow, largest first, and fill the tail.  Every strip
-    // is claimed after the strip it waits for.
-    constexpr double kLagSteps = 84.0;
-    const double share_steps = share / (double)H;
-    std::vector<int32_t> flow;  // non-critical chained pairs, strip counts descending
-    for (int32_t q : chained) {
-        const PackedPair &d = pp[(size_t)q];
-        if (2.0 * ((double)d.N + (d.nstrips - 1) * kLagSteps) >= share_steps)
-            for (int32_t s = 0; s < d.nstrips; ++s) up.push_back(make_int2(q, s));
-        else
-            flow.push_back(q);
-    }
-    // (pp is sorted by strip count, so the pairs of `flow` with more than s
-    // strips are a prefix of it)
-    for (int32_t s = 0; !flow.empty() && s < pp[(size_t)flow[0]].nstrips; ++s)
-        for (size_t i = 0; i < flow.size() && pp[(size_t)flow[i]].nstrips > s; ++i)
-            up.push_back(make_int2(flow[i], s));
-    for (size_t q = 0; q < pp.size(); ++q)
-        if (pp[q].whole) up.push_back(make_int2((int32_t)q, 0));
-    L.units = units;
-    L.hb = hb;
 }
 
-// The packed scoring pass over the positions `pos` of `order` with R rows per
-// lane (the layout `pre` when it was made for the same R and positions).  Fills
-// pbest[k] for every k in pos and appends to `redo` the positions whose pair
-// reached the 16-bit limit.
-int run_packed(swb_ctx *c, const BatchArgs &base, const std::vector<PairInfo> &info,
+// The large pass over the positions `pos` of `order` with R rows per lane (the
+// layout `pre` when it was made for the same R and positions).  Fills pbest[k] for
+// every k in pos.
+int run_packed(swb_ctx *c, const uint8_t *d_seq, bool tab, const BatchArgs &base, const std::vector<PairInfo> &info,
                const std::vector<int64_t> &order, const std::vector<int64_t> &pos, uint32_t flags, int R,
-               std::vector<BestRec> &pbest, std::vector<int64_t> &redo, float *ms,
-               const PackedLayout *pre = nullptr) {
-    cudaError_t e;
+               std::vector<BestRec> &pbest, float *ms, PackedLayout *pre = nullptr) {
     PackedLayout local;
-    const PackedLayout *L = pre;
+    PackedLayout *L = pre;
     if (!L || L->R != R || L->pos != pos) {
         layout_packed(c, info, order, pos, flags, R, local);
         L = &local;
     }
-    const std::vector<PackedPair> &pp = L->pp;
-    const std::vector<int2> &up = L->up;
-    const int64_t units = L->units, hb = L->hb;
-    const int64_t np = (int64_t)pp.size(), nslots = (int64_t)order.size() + 1, items = (int64_t)up.size();
-    const size_t pp_bytes = sizeof(PackedPair) * (size_t)np, up_bytes = sizeof(int2) * (size_t)items;
-    const size_t back = sizeof(BestRec) * (size_t)nslots + sizeof(int32_t) * (size_t)nslots + 64;
-    if ((e = c->b_pairs.ensure(pp_bytes)) != cudaSuccess || (e = c->b_units.ensure(up_bytes)) != cudaSuccess ||
-        (e = c->b_hbuf.ensure(sizeof(int4) * (size_t)std::max<int64_t>(1, hb))) != cudaSuccess ||
-        (e = c->b_gbest.ensure(sizeof(int32_t) * (size_t)nslots)) != cudaSuccess ||
-        (e = c->b_ubest.ensure(2 * sizeof(BestRec) * (size_t)std::max<int64_t>(1, units))) != cudaSuccess ||
-        (e = c->b_pbest.ensure(sizeof(BestRec) * (size_t)nslots)) != cudaSuccess ||
-        (e = c->b_sat.ensure(sizeof(int32_t) * (size_t)nslots)) != cudaSuccess ||
-        (e = c->b_ctl.ensure(4 * sizeof(int32_t))) != cudaSuccess ||
-        (e = c->h_stage.ensure(std::max(pp_bytes + up_bytes, back) + 64)) != cudaSuccess)
-        return ctx_cuda_fail(c, e, "packed batch buffers");
-    uint8_t *hs = (uint8_t *)c->h_stage.p;
-    std::memcpy(hs, pp.data(), pp_bytes);
-    std::memcpy(hs + pp_bytes, up.data(), up_bytes);
-    Batch16Args a{};
-    a.rcode = base.rcode;
-    a.ctab = base.ctab;
-    a.open = base.open;
-    a.open2 = (uint32_t)(uint16_t)(int16_t)base.open * 0x00010001u;
-    a.ext2 = (uint32_t)(uint16_t)(int16_t)base.ext * 0x00010001u;
-    a.gx2 = (uint32_t)(uint16_t)(int16_t)base.gx * 0x00010001u;
-    a.mm4 = base.tab_hi;
-    a.sat_lim = kSatLimit;
-    a.pairs = (const PackedPair *)c->b_pairs.p;
-    a.items = (const int2 *)c->b_units.p;
-    a.nunits = items;
-    a.hbuf = (int4 *)c->b_hbuf.p;
-    a.gbest = (int32_t *)c->b_gbest.p;
-    a.ubest = (BestRec *)c->b_ubest.p;
-    a.ctl = (int32_t *)c->b_ctl.p;
-    a.sat = (int32_t *)c->b_sat.p;
-    a.wait_limit = c->wait_cycles;
-    if ((e = cudaMemcpyAsync(c->b_pairs.p, hs, pp_bytes, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(c->b_units.p, hs + pp_bytes, up_bytes, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess ||
-        (hb > 0 && (e = cudaMemsetAsync(a.hbuf, 0xFF, sizeof(int4) * (size_t)hb, c->stream)) != cudaSuccess) ||
-        (e = cudaMemsetAsync(a.gbest, 0, sizeof(int32_t) * (size_t)nslots, c->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(c->b_pbest.p, 0, sizeof(BestRec) * (size_t)nslots, c->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(a.sat, 0, sizeof(int32_t) * (size_t)nslots, c->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(a.ctl, 0, 4 * sizeof(int32_t), c->stream)) != cudaSuccess)
-        return ctx_cuda_fail(c, e, "packed batch set-up");
-    cudaEventRecord(c->ev0, c->stream);
-    if ((e = batch16_launch(a, R, c->sms, c->max_blocks, np, (BestRec *)c->b_pbest.p, c->stream)) != cudaSuccess)
-        return ctx_cuda_fail(c, e, "packed batch launch");
-    cudaEventRecord(c->ev1, c->stream);
-    BestRec *hb_best = (BestRec *)hs;
-    int32_t *hsat = (int32_t *)(hs + sizeof(BestRec) * (size_t)nslots);
-    int32_t *hctl = hsat + nslots;
-    if ((e = cudaMemcpyAsync(hb_best, c->b_pbest.p, sizeof(BestRec) * (size_t)nslots, cudaMemcpyDeviceToHost,
-                             c->stream)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(hsat, a.sat, sizeof(int32_t) * (size_t)nslots, cudaMemcpyDeviceToHost, c->stream)) !=
-            cudaSuccess ||
-        (e = cudaMemcpyAsync(hctl, a.ctl, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(c->stream)) != cudaSuccess)
-        return ctx_cuda_fail(c, e, "packed batch");
-    if (hctl[1] != 0) return ctx_fail(c, SWB_ETIMEOUT, "batch: a bounded wait between strips ran out");
-    for (int64_t k : pos) {
-        if (hsat[k]) redo.push_back(k);
-        else pbest[(size_t)k] = hb_best[k];
-    }
-    float t = 0.f;
-    cudaEventElapsedTime(&t, c->ev0, c->ev1);
-    if (ms) *ms += t;
+    std::vector<BestRec> pb;
+    const int rc = run_launch(c, d_seq, tab, base, L->bp, L->up, L->hb, false, true, R, pb, ms, false, &L->us, L->strips);
+    if (rc != SWB_OK) return rc;
+    for (size_t q = 0; q < pos.size(); ++q) pbest[(size_t)pos[q]] = pb[q];
     return SWB_OK;
 }
 
@@ -549,10 +422,9 @@ int packed_rows_known(swb_ctx *c, const std::vector<PairInfo> &info, const std::
     return (int64_t)ppos.size() < kTuneMinPairs ? kBatch16R : 0;
 }
 
-int tune_packed(swb_ctx *c, const BatchArgs &base, const std::vector<PairInfo> &info,
+int tune_packed(swb_ctx *c, const uint8_t *d_seq, bool tab, const BatchArgs &base, const std::vector<PairInfo> &info,
                 const std::vector<int64_t> &order, std::vector<int64_t> &ppos, uint32_t flags,
-                std::vector<BestRec> &pbest, std::vector<int64_t> &redo, float *ms, int32_t *launches, int *R,
-                const char **how) {
+                std::vector<BestRec> &pbest, float *ms, int32_t *launches, int *R, const char **how) {
     std::string key;
     const int known = packed_rows_known(c, info, order, ppos, how, &key);
     *R = known > 0 ? known : kBatch16R;
@@ -568,7 +440,7 @@ int tune_packed(swb_ctx *c, const BatchArgs &base, const std::vector<PairInfo> &
             cells += (double)p.m * (double)p.n;
         }
         float t = 0.f;
-        const int rc = run_packed(c, base, info, order, sample, flags, cands[i], pbest, redo, &t);
+        const int rc = run_packed(c, d_seq, tab, base, info, order, sample, flags, cands[i], pbest, &t);
         if (rc != SWB_OK) return rc;
         *launches += 2;
         if (ms) *ms += t;
@@ -962,7 +834,8 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
     }
     // strips in packed 16-bit lanes unless the scoring is too wide for their window
     const char *pack_env = std::getenv("SWB_STAGE1_PACK");
-    const bool packed = !wide && strip16_fits(*sc, kBatchR, maxlen) && !(pack_env && pack_env[0] == '0');
+    const bool packed =
+        !wide && strip16_fits(*sc, kBatchR, maxlen) && !(pack_env && pack_env[0] == '0') && packing_enabled();
     out->npairs = npairs;
     out->cells = cells;
     out->items = (swb_batch_item *)std::calloc((size_t)std::max<int64_t>(1, npairs), sizeof(swb_batch_item));
@@ -987,11 +860,9 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
     // host batches run as one replayed graph (sequences and descriptors in one
     // copy, results in one copy); device batches and the store pass of a
     // partially traced batch launch their kernels directly
-    // large score-only batches take the packed 16-bit pass (direct launches); the
-    // rest of host batches run as one replayed graph
-    const int32_t mt1 = sc->match - sc->gap_open, mm1 = sc->mismatch - sc->gap_open;
-    const bool pack_candidate = !stores_first && (int64_t)order.size() >= kPackMinPairs && packing_enabled() &&
-                                mt1 >= -128 && mt1 <= 127 && mm1 >= -128 && mm1 <= 127;
+    // large score-only batches take their own pass (direct launches); the rest of
+    // host batches run as one replayed graph
+    const bool pack_candidate = !stores_first && packed && (int64_t)order.size() >= kPackMinPairs;
     const bool use_graph = h_seq != nullptr && !order.empty() && graphs_enabled() && !pack_candidate;
     GraphPass gp;
     ph.mark("orient + order");
@@ -1018,12 +889,11 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
 
     // The packed pass's host layout (sorting, packing, claim order: several ms
     // for 100,000 pairs) is built now, while the sequences are still on their
-    // way to the device, whenever its strip height needs no probe.  If the
-    // batch then turns out not to be in the table mode, it goes unused.
+    // way to the device, whenever its strip height needs no probe.
     PackedLayout early;
     if (pack_candidate && !order.empty() && !use_graph) {
-        std::vector<int64_t> ppos, rest;
-        split_packable(info, order, sc, flags, ppos, rest);
+        std::vector<int64_t> ppos(order.size());
+        std::iota(ppos.begin(), ppos.end(), 0);
         const char *how = "";
         const int R = packed_rows_known(c, info, order, ppos, &how, nullptr);
         if (R > 0 && !ppos.empty()) layout_packed(c, info, order, ppos, flags, R, early);
@@ -1095,39 +965,24 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
         bp = gp.bp;
         pbest = gp.pbest;
         ms1 = gp.ms1;
-    } else if (!(pack_candidate && tab)) {
+    } else if (!pack_candidate) {
         layout_units(info, order, flags, 32 * R1, bp, unit_pair, &hb);
     }
-    if (!order.empty() && !use_graph && pack_candidate && tab) {
-        // pairs whose best score is bounded below the 16-bit limit run packed two
-        // per warp; the others, and any pair that reached the limit, in int32
-        std::vector<int64_t> ppos, rest;
-        split_packable(info, order, sc, flags, ppos, rest);
+    if (!order.empty() && !use_graph && pack_candidate) {
+        std::vector<int64_t> ppos(order.size());
+        std::iota(ppos.begin(), ppos.end(), 0);
         pbest.assign(order.size(), BestRec{});
         int Rp = kBatch16R;
         const char *how = "";
-        int rc = tune_packed(c, base, info, order, ppos, flags, pbest, rest, &ms1, &launches, &Rp, &how);
+        int rc = tune_packed(c, d_seq, tab, base, info, order, ppos, flags, pbest, &ms1, &launches, &Rp, &how);
         if (rc != SWB_OK) return rc;
         if (ph.on) std::fprintf(stderr, "swb batch: packed rows per lane %d (%s)\n", Rp, how);
         if (!ppos.empty()) {
-            rc = run_packed(c, base, info, order, ppos, flags, Rp, pbest, rest, &ms1, &early);
+            rc = run_packed(c, d_seq, tab, base, info, order, ppos, flags, Rp, pbest, &ms1, &early);
             if (rc != SWB_OK) return rc;
             launches += 2;
         }
         ph.mark("packed pass");
-        if (!rest.empty()) {
-            std::vector<int64_t> sub(rest.size());
-            for (size_t i = 0; i < rest.size(); ++i) sub[i] = order[(size_t)rest[i]];
-            std::vector<BatchPair> bp2;
-            std::vector<int32_t> up2;
-            std::vector<BestRec> pb2;
-            int64_t hb2 = 0;
-            layout_units(info, sub, flags, 32 * R1, bp2, up2, &hb2);
-            rc = run_launch(c, d_seq, tab, base, bp2, up2, hb2, false, packed, R1, pb2, &ms1, true);
-            if (rc != SWB_OK) return rc;
-            launches += 2;
-            for (size_t i = 0; i < rest.size(); ++i) pbest[(size_t)rest[i]] = pb2[i];
-        }
     } else if (!order.empty() && !use_graph) {
         BatchArgs a1 = base;
         if (first_stores) {
