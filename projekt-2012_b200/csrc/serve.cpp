@@ -37,6 +37,10 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
+// A burst of 48 requests in one or two iterations instead of three or more: see
+// short_lane.
+constexpr int64_t kGatherUs = 100, kGatherMaxUs = 500;
+
 double ms_since(Clock::time_point t0, Clock::time_point t1) {
     return std::chrono::duration<double, std::milli>(t1 - t0).count();
 }
@@ -75,7 +79,7 @@ uint64_t long_footprint(int64_t m, int64_t n, uint64_t store_budget, int sms) {
     const uint64_t level2 = p.level1 ? (uint64_t)swb::tb::level1_corridor_cells(p, sms) *
                                            (uint64_t)swb::tb::level1_cell_store_bytes(p)
                                      : 0;
-    const uint64_t walker = (uint64_t)4 * 148 * 4 * (256 + 31) * 32 * 4;  // precomputed direction blocks
+    const uint64_t walker = (uint64_t)8 * 148 * 81920;  // direction blocks of the walker's CTAs
     return 6ULL * (uint64_t)(m + n) + 16ULL * (uint64_t)n + stores + level2 + walker + (uint64_t)(m + n + 8) +
            (64ULL << 20);
 }
@@ -123,6 +127,15 @@ struct swb_server {
                 std::unique_lock<std::mutex> lk(mu);
                 cv_work.wait(lk, [&] { return stop || !qs.empty(); });
                 if (stop && qs.empty()) return;
+                // An iteration of one or two pairs costs about as much as one of fifty, so
+                // while requests keep coming in, a moment's wait serves them together: up to
+                // kGatherUs after the newest request, kGatherMaxUs in all.
+                const auto gather_end = Clock::now() + std::chrono::microseconds(kGatherMaxUs);
+                while (!stop && (int)qs.size() < o.max_batch) {
+                    const auto until = std::min(gather_end, qs.back()->t_submit + std::chrono::microseconds(kGatherUs));
+                    if (Clock::now() >= until) break;
+                    cv_work.wait_until(lk, until);
+                }
                 while (!qs.empty() && (int)it.size() < o.max_batch) {
                     Request *r = qs.front();
                     if (reserved + r->foot > o.hbm_budget_bytes && !it.empty()) break;
