@@ -84,6 +84,10 @@ struct GraphHdr {
     void *walk_args;          // traced graphs: walker arguments per pair (traceback.cu's layout)
     int64_t *walk_states;     // traced graphs: walker state per pair
     uint32_t *walk_dir;       // traced graphs: walker direction scratch (8 CTAs per SM)
+    const int2 *seg_items;    // traced graphs walked in segments: (pair, segment), their number,
+    int64_t seg_nitems;       // per pair its first segment or -1, and their records and outputs
+    const int32_t *seg_base;
+    void *seg_rec;
     uint8_t *lut;             // byte -> code (written by the decide kernel)
     uint32_t *presence;       // 256-bit byte bitmap (all zero between calls)
     int32_t *out;             // [0..3] the launch's control words, [4] the decided mode

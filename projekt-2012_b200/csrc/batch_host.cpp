@@ -497,9 +497,10 @@ size_t pow2_at_least(size_t x) {
 // captured on first use.  Its kernels read the call header at c->g_hdr.p, so the
 // graph never changes for a shape; the scoring kernels' parameters are set per
 // replay (graph_set_scoring).
-cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, bool packed, int R, int cap, int size_class, swb_ctx::GraphEntry **out) {
+cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, bool packed, bool segments, int R, int cap, int size_class, swb_ctx::GraphEntry **out) {
     for (auto &g : c->graphs)
-        if (g.exec && g.traced == (int)traced && g.wide == (int)wide && g.packed == (int)packed && g.R == R && g.cap == cap && g.size_class == size_class) {
+        if (g.exec && g.traced == (int)traced && g.wide == (int)wide && g.packed == (int)packed &&
+            g.segments == (int)segments && g.R == R && g.cap == cap && g.size_class == size_class) {
             *out = &g;
             return cudaSuccess;
         }
@@ -511,7 +512,7 @@ cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, bool packed, int R, in
     if ((e = cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
     cudaError_t q = cudaEventRecordWithFlags(c->ev0, c->cap_stream, cudaEventRecordExternal);
     if (q == cudaSuccess) q = batch_graph_enqueue(h, traced, packed, R, c->sms, cap, max_units, c->ev1, c->cap_stream);
-    if (q == cudaSuccess && traced) q = tb::walk_graph_enqueue(h, wide, c->sms, max_units, c->cap_stream);
+    if (q == cudaSuccess && traced) q = tb::walk_graph_enqueue(h, wide, segments, c->sms, max_units, max_units, c->cap_stream);
     if (q == cudaSuccess && traced) q = cudaEventRecordWithFlags(c->ev2, c->cap_stream, cudaEventRecordExternal);
     cudaGraph_t graph = nullptr;
     e = cudaStreamEndCapture(c->cap_stream, &graph);
@@ -569,6 +570,7 @@ cudaError_t graph_for(swb_ctx *c, bool traced, bool wide, bool packed, int R, in
     slot->traced = traced;
     slot->wide = wide;
     slot->packed = packed;
+    slot->segments = segments;
     slot->R = R;
     slot->cap = cap;
     slot->size_class = size_class;
@@ -603,7 +605,7 @@ cudaError_t graph_set_scoring(swb_ctx *c, swb_ctx::GraphEntry *g, const BatchArg
 struct GraphPass {
     std::vector<BatchPair> bp;
     std::vector<BestRec> pbest;
-    bool tab = false;
+    bool tab = false, segments = false;
     const uint8_t *d_seq = nullptr;
     const uint8_t *rcode = nullptr;
     const uint32_t *ctab = nullptr;
@@ -652,11 +654,20 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
         ops_total = oo;
         xp_total = xo;
     }
+    std::vector<int32_t> seg_base, seg_items;
+    int64_t nseg = 0;
+    if (traced) {
+        std::vector<int64_t> rows((size_t)np);
+        for (int64_t k = 0; k < np; ++k) rows[(size_t)k] = gp.bp[(size_t)k].m;
+        nseg = tb::seg_plan(rows.data(), np, c->sms, seg_base, seg_items);
+    }
     // device layouts (16-byte aligned sections)
     const size_t wa_bytes = tb::walk_args_bytes();
     const size_t in_pairs = 0, in_units = al16(in_pairs + sizeof(BatchPair) * (size_t)np);
     const size_t in_walk = al16(in_units + sizeof(int32_t) * (size_t)nu);
-    const size_t in_seq = al16(in_walk + (traced ? wa_bytes * (size_t)np : 0));
+    const size_t in_seg = al16(in_walk + (traced ? wa_bytes * (size_t)np : 0));
+    const size_t in_segb = al16(in_seg + sizeof(int32_t) * (nseg > 0 ? seg_items.size() : 0));
+    const size_t in_seq = al16(in_segb + sizeof(int32_t) * (nseg > 0 ? seg_base.size() : 0));
     const size_t in_bytes = al16(in_seq + (size_t)seq_bytes + 64);
     const size_t w_hbuf = 0, w_gbest = al16(w_hbuf + sizeof(int4) * (size_t)hb);
     const size_t w_ubest = al16(w_gbest + sizeof(int32_t) * (size_t)np);
@@ -675,6 +686,7 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
     if ((e = c->g_hdr.ensure(hdr_all)) != cudaSuccess || (e = c->g_in.ensure(in_bytes)) != cudaSuccess ||
         (e = c->g_work.ensure(work_bytes)) != cudaSuccess || (e = c->g_out.ensure(out_bytes)) != cudaSuccess ||
         (traced && (e = c->g_dir.ensure(tb::walk_batch_dir_bytes(c->sms, tb::walk_graph_ctas(c->sms)))) != cudaSuccess) ||
+        (nseg > 0 && (e = c->g_seg.ensure(pow2_at_least(tb::seg_scratch_bytes(nseg)))) != cudaSuccess) ||
         (e = c->h_gin.ensure(pow2_at_least(hdr_bytes + in_bytes))) != cudaSuccess ||
         (e = c->h_gout.ensure(pow2_at_least(out_bytes))) != cudaSuccess)
         return ctx_cuda_fail(c, e, "graphed batch buffers");
@@ -717,6 +729,10 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
     g.walk_args = traced ? (void *)(din + in_walk) : nullptr;
     g.walk_states = traced ? (int64_t *)(dout + o_states) : nullptr;
     g.walk_dir = traced ? (uint32_t *)c->g_dir.p : nullptr;
+    g.seg_nitems = nseg;
+    g.seg_items = (const int2 *)(din + in_seg);
+    g.seg_base = (const int32_t *)(din + in_segb);
+    g.seg_rec = c->g_seg.p;
     g.lut = dh + hdr_bytes;
     g.presence = (uint32_t *)(dh + hdr_bytes + 256);
     g.out = (int32_t *)(dout + o_ctl);
@@ -748,6 +764,10 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
         }
         tb::pack_walk_args(win.data(), np, g.walk_states, hin + in_walk);
     }
+    if (nseg > 0) {
+        std::memcpy(hin + in_seg, seg_items.data(), sizeof(int32_t) * seg_items.size());
+        std::memcpy(hin + in_segb, seg_base.data(), sizeof(int32_t) * seg_base.size());
+    }
     ph.mark("graph: descriptors");
     copy_parallel(hin + in_seq, h_seq, (size_t)seq_bytes);
     ph.mark("graph: sequences staged");
@@ -761,7 +781,7 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
         size_class = std::min(size_class, full);
     }
     swb_ctx::GraphEntry *ge = nullptr;
-    if ((e = graph_for(c, traced, traced && !tb::walk16_fits(*sc), packed, R, c->max_blocks, size_class, &ge)) != cudaSuccess ||
+    if ((e = graph_for(c, traced, traced && !tb::walk16_fits(*sc), packed, nseg > 0, R, c->max_blocks, size_class, &ge)) != cudaSuccess ||
         (e = graph_set_scoring(c, ge, g.ba)) != cudaSuccess)
         return ctx_cuda_fail(c, e, "batch graph");
     uint8_t *hout = (uint8_t *)c->h_gout.p;
@@ -776,6 +796,7 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
     if (ctl[1] == kStage1Range) return kRangeAgain;
     if (ctl[1] != 0) return ctx_fail(c, SWB_ETIMEOUT, "batch: a bounded wait between strips ran out");
     gp.tab = ctl[4] != 0;
+    gp.segments = nseg > 0;
     gp.d_seq = g.ba.seq;
     gp.rcode = g.ba.rcode;
     gp.ctab = g.ba.ctab;
@@ -917,7 +938,7 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
             base.ctab = gp.ctab;
             base.tab_hi = (uint32_t)(uint8_t)(int8_t)base.mm1 * 0x01010101u;
         }
-        launches += (stores_first ? 8 : 6) - (packed ? 1 : 0);
+        launches += (stores_first ? 8 : 6) - (packed ? 1 : 0) + (gp.segments ? 2 : 0);
     } else if (!order.empty() && base.mt1 >= -128 && base.mt1 <= 127 && base.mm1 >= -128 && base.mm1 <= 127) {
         // TAB mode when the whole buffer holds at most four distinct bytes
         uint32_t present[256];
@@ -1148,10 +1169,13 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
                 scr.put = [](void *owner, void *dst, const void *src, size_t bytes) -> cudaError_t {
                     return ctx_put((swb_ctx *)owner, dst, src, bytes);
                 };
+                scr.ensure = [](void *owner, int which, size_t bytes) -> void * {
+                    swb_ctx *cx = (swb_ctx *)owner;
+                    return cx->tb[which].ensure(bytes) == cudaSuccess ? cx->tb[which].p : nullptr;
+                };
                 int rc = tb::walk_batch(c->stream, c->sms, win.data(), (int64_t)win.size(), c->b_walk.p,
-                                        (int64_t *)c->b_state.p, c->b_gdir.p, st.data(), scr, err);
+                                        (int64_t *)c->b_state.p, c->b_gdir.p, st.data(), scr, err, &launches);
                 if (rc != SWB_OK) return ctx_fail(c, rc, "%s", err.c_str());
-                launches += 1;
                 hops.resize((size_t)std::max<int64_t>(1, oo));
                 hxp.resize((size_t)std::max<int64_t>(4, 4 * xo));
                 if ((e = ctx_get(c, hops.data(), c->b_ops.p, (size_t)oo)) != cudaSuccess ||

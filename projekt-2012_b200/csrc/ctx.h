@@ -51,7 +51,7 @@ struct swb_ctx {
     int64_t wait_cycles = 0;  // opts.wait_limit_ms in SM clock cycles (0: the kernels' default)
     std::string err;
     swb::DevBuf rows, cols, hbuf, wbest, best, errf, srows, scols, work, flags, lut, rcode, ctab, trace;
-    swb::DevBuf tb[24];  // traceback scratch (ops, crosspoints, state, level-2 stores, recompute and walker buffers)
+    swb::DevBuf tb[32];  // traceback scratch (ops, crosspoints, state, level-2 stores, recompute and walker buffers)
     // batched path: sequences, encodings, descriptors, per-unit / per-pair records, stores
     swb::DevBuf b_seq, b_rcode, b_ctab, b_pairs, b_units, b_hbuf, b_gbest, b_ubest, b_pbest, b_ctl, b_srows,
         b_scols, b_walk, b_ops, b_xps, b_state, b_gdir;
@@ -63,7 +63,7 @@ struct swb_ctx {
     // graphed batches: the call header (allocated once: the graphs hold its
     // address), packed inputs, work buffers, packed results, walker scratch, their
     // pinned staging, and the instantiated graphs by shape
-    swb::DevBuf g_hdr, g_in, g_work, g_out, g_dir;
+    swb::DevBuf g_hdr, g_in, g_work, g_out, g_dir, g_seg;
     swb::HostBuf h_gin, h_gout;
     struct GraphEntry {
         cudaGraph_t graph = nullptr;        // kept: its nodes name the exec's nodes
@@ -72,7 +72,7 @@ struct swb_ctx {
         cudaKernelNodeParams kp[2] = {};     // their launch shapes
         unsigned char set_args[256] = {};    // the BatchArgs last set on them
         bool args_valid = false;
-        int traced = 0, wide = 0, packed = 0, R = 0, cap = 0, size_class = 0;
+        int traced = 0, wide = 0, packed = 0, segments = 0, R = 0, cap = 0, size_class = 0;
     };
     GraphEntry graphs[16];
     int graph_next = 0;                  // round-robin replacement when all entries are taken
@@ -91,7 +91,7 @@ struct swb_ctx {
         for (swb::DevBuf *b : {&rows, &cols, &hbuf, &wbest, &best, &errf, &srows, &scols, &work, &flags, &lut,
                                &rcode, &ctab, &trace, &b_seq, &b_rcode, &b_ctab, &b_pairs, &b_units, &b_hbuf,
                                &b_gbest, &b_ubest, &b_pbest, &b_ctl, &b_srows, &b_scols, &b_walk, &b_ops, &b_xps,
-                               &b_state, &b_gdir, &g_hdr, &g_in, &g_work, &g_out, &g_dir})
+                               &b_state, &b_gdir, &g_hdr, &g_in, &g_work, &g_out, &g_dir, &g_seg})
             f(*b);
         for (swb::DevBuf &b : tb) f(b);
     }

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <string>
+#include <vector>
 
 #include "swb_internal.h"
 
@@ -82,7 +83,8 @@ struct Scratch {
 enum ScratchSlot {
     kScrOps = 0, kScrXps, kScrState, kScrSrows2, kScrScols2, kScrHbuf, kScrWbest, kScrBest, kScrErr,
     kScrGdir, kScrBlk, kScrMap, kScrWalkErr,
-    kScrL1Pairs, kScrL1Units, kScrL1Hbuf, kScrL1Gbest, kScrL1Ubest, kScrL1Pbest, kScrL1Ctl, kScrSlots
+    kScrL1Pairs, kScrL1Units, kScrL1Hbuf, kScrL1Gbest, kScrL1Ubest, kScrL1Pbest, kScrL1Ctl,
+    kScrSegRec, kScrSegItems, kScrSegOff, kScrSlots
 };
 
 // Walks the path from host_state's cell through the region of `in` (until the
@@ -96,7 +98,7 @@ int walk_region(cudaStream_t st, int sms, const WalkInputs &in, int64_t *host_st
 // int64 (initial states are copied from host_states, final ones back to it),
 // d_dir walk_batch_dir_bytes(sms, n) bytes of direction scratch.
 int walk_batch(cudaStream_t st, int sms, const WalkInputs *in, int64_t n, void *d_args, int64_t *d_states,
-               void *d_dir, int64_t *host_states, const Scratch &scr, std::string &err);
+               void *d_dir, int64_t *host_states, const Scratch &scr, std::string &err, int32_t *launches);
 size_t walk_batch_dir_bytes(int sms, int64_t n);
 
 // Graphed batches (the header's walk_args / walk_states / walk_dir hold every
@@ -106,7 +108,13 @@ size_t walk_batch_dir_bytes(int sms, int64_t n);
 // pairs, up to walk_graph_ctas(sms) CTAs whose direction scratch is
 // walk_batch_dir_bytes(sms, walk_graph_ctas(sms)).
 void pack_walk_args(const WalkInputs *in, int64_t n, int64_t *d_states, void *dst);
-cudaError_t walk_graph_enqueue(const GraphHdr *d_hdr, bool wide, int sms, int64_t max_pairs, cudaStream_t st);
+cudaError_t walk_graph_enqueue(const GraphHdr *d_hdr, bool wide, bool segments, int sms, int64_t max_pairs,
+                               int64_t max_units, cudaStream_t st);
+// Segments (traceback.cu) of n pairs with the given row counts: per pair its first
+// segment's index or -1, and the items (pair, segment); returns their number, 0
+// when the pairs alone fill the GPU.  seg_scratch_bytes: records and outputs.
+int64_t seg_plan(const int64_t *rows, int64_t n, int sms, std::vector<int32_t> &base, std::vector<int32_t> &items);
+size_t seg_scratch_bytes(int64_t nseg);
 int64_t walk_graph_ctas(int sms);
 
 // Canonical traceback from the end cell in `out` (score, end_row, end_col set by
