@@ -1099,8 +1099,6 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
             std::vector<const char *> tO(tr.size());
             std::vector<int64_t> tOc(tr.size()), tXc(tr.size());
             std::vector<int64_t> st;
-            std::vector<char> hops;
-            std::vector<int64_t> hxp;
             if (use_graph && first_stores) {
                 // the graph walked every pair with a positive score already
                 std::vector<int64_t> pos((size_t)npairs, -1);
@@ -1176,55 +1174,79 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
                 int rc = tb::walk_batch(c->stream, c->sms, win.data(), (int64_t)win.size(), c->b_walk.p,
                                         (int64_t *)c->b_state.p, c->b_gdir.p, st.data(), scr, err, &launches);
                 if (rc != SWB_OK) return ctx_fail(c, rc, "%s", err.c_str());
-                hops.resize((size_t)std::max<int64_t>(1, oo));
-                hxp.resize((size_t)std::max<int64_t>(4, 4 * xo));
-                if ((e = ctx_get(c, hops.data(), c->b_ops.p, (size_t)oo)) != cudaSuccess ||
-                    (e = ctx_get(c, hxp.data(), c->b_xps.p, sizeof(int64_t) * 4 * (size_t)xo)) != cudaSuccess)
-                    return ctx_cuda_fail(c, e, "batch traceback copy");
+                std::vector<int64_t> ends(2 * tr.size()), offs;
                 for (size_t k = 0; k < tr.size(); ++k) {
-                    tS[k] = st.data() + (size_t)kS * k;
-                    tO[k] = hops.data() + ops_off[k];
-                    tX[k] = hxp.data() + 4 * xp_off[k];
-                    tOc[k] = win[k].ops_cap;
-                    tXc[k] = win[k].xp_cap;
+                    const int64_t *S = st.data() + (size_t)kS * k;
+                    if (S[tb::slot_nops()] > win[k].ops_cap || S[tb::slot_nxp()] > win[k].xp_cap)
+                        return ctx_fail(c, SWB_ECUDA, "batch traceback output larger than its buffers");
+                    ends[2 * k] = out->items[tr[k]].end_row;
+                    ends[2 * k + 1] = out->items[tr[k]].end_col;
+                }
+                int64_t nops = 0, nxps = 0;
+                char *d_ops = nullptr;
+                swb_xpoint *d_xps = nullptr;
+                rc = tb::pack_results(c->stream, c->b_walk.p, (int64_t)tr.size(), st.data(), ends.data(), offs, &nops,
+                                      &nxps, &d_ops, &d_xps, scr, err);
+                if (rc != SWB_OK) return ctx_fail(c, rc, "%s", err.c_str());
+                launches += 1;
+                out->ops = (char *)std::malloc((size_t)nops + 1);
+                out->xpoints = (swb_xpoint *)std::malloc(sizeof(swb_xpoint) * (size_t)(nxps + 2 * ntrace + 1));
+                if (!out->ops || !out->xpoints) return ctx_fail(c, SWB_ENOMEM, "out of host memory");
+                if ((e = ctx_get(c, out->ops, d_ops, (size_t)nops)) != cudaSuccess ||
+                    (e = ctx_get(c, out->xpoints, d_xps, sizeof(swb_xpoint) * (size_t)nxps)) != cudaSuccess)
+                    return ctx_cuda_fail(c, e, "batch traceback copy");
+                out->ops[nops] = 0;
+                out->ops_bytes = nops;
+                out->n_xpoints = nxps;
+                for (size_t k = 0; k < tr.size(); ++k) {
+                    swb_batch_item &it = out->items[tr[k]];
+                    const int64_t *S = st.data() + (size_t)kS * k;
+                    it.ops_off = offs[4 * k];
+                    it.n_ops = S[tb::slot_nops()];
+                    it.xp_off = offs[4 * k + 1];
+                    it.n_xpoints = S[tb::slot_nxp()] + 2;
+                    it.start_row = S[tb::slot_start_r()];
+                    it.start_col = S[tb::slot_start_c()];
                 }
             }
             ph.mark("walker");
-            // gather: ops (end -> start on the device) and crosspoints
-            int64_t tot_ops = 0, tot_xp = 0;
-            for (size_t k = 0; k < tr.size(); ++k) {
-                const int64_t *S = tS[k];
-                if (S[tb::slot_nops()] > tOc[k] || S[tb::slot_nxp()] > tXc[k])
-                    return ctx_fail(c, SWB_ECUDA, "batch traceback output larger than its buffers");
-                tot_ops += S[tb::slot_nops()];
-                tot_xp += S[tb::slot_nxp()] + 2;
-            }
-            out->ops = (char *)std::malloc((size_t)tot_ops + 1);
-            out->xpoints = (swb_xpoint *)std::malloc(sizeof(swb_xpoint) * (size_t)(tot_xp + 2 * ntrace + 1));
-            if (!out->ops || !out->xpoints) return ctx_fail(c, SWB_ENOMEM, "out of host memory");
-            int64_t po = 0, px = 0;
-            for (size_t k = 0; k < tr.size(); ++k) {
-                swb_batch_item &it = out->items[tr[k]];
-                const int64_t *S = tS[k];
-                const int64_t nops = S[tb::slot_nops()], nxp = S[tb::slot_nxp()];
-                it.ops_off = po;
-                it.n_ops = nops;
-                std::reverse_copy(tO[k], tO[k] + nops, out->ops + po);
-                po += nops;
-                it.start_row = S[tb::slot_start_r()];
-                it.start_col = S[tb::slot_start_c()];
-                it.xp_off = px;
-                out->xpoints[px++] = swb_xpoint{0, 0, it.start_row, it.start_col};
-                for (int64_t q = nxp - 1; q >= 0; --q) {
-                    const int64_t *d = tX[k] + 4 * q;
-                    out->xpoints[px++] = swb_xpoint{(int32_t)d[3], (int32_t)d[2], d[0], d[1]};
+            if (use_graph && first_stores) {
+                // gather: ops (end -> start on the device) and crosspoints
+                int64_t tot_ops = 0, tot_xp = 0;
+                for (size_t k = 0; k < tr.size(); ++k) {
+                    const int64_t *S = tS[k];
+                    if (S[tb::slot_nops()] > tOc[k] || S[tb::slot_nxp()] > tXc[k])
+                        return ctx_fail(c, SWB_ECUDA, "batch traceback output larger than its buffers");
+                    tot_ops += S[tb::slot_nops()];
+                    tot_xp += S[tb::slot_nxp()] + 2;
                 }
-                out->xpoints[px++] = swb_xpoint{0, it.score, it.end_row, it.end_col};
-                it.n_xpoints = px - it.xp_off;
+                out->ops = (char *)std::malloc((size_t)tot_ops + 1);
+                out->xpoints = (swb_xpoint *)std::malloc(sizeof(swb_xpoint) * (size_t)(tot_xp + 2 * ntrace + 1));
+                if (!out->ops || !out->xpoints) return ctx_fail(c, SWB_ENOMEM, "out of host memory");
+                int64_t po = 0, px = 0;
+                for (size_t k = 0; k < tr.size(); ++k) {
+                    swb_batch_item &it = out->items[tr[k]];
+                    const int64_t *S = tS[k];
+                    const int64_t nops = S[tb::slot_nops()], nxp = S[tb::slot_nxp()];
+                    it.ops_off = po;
+                    it.n_ops = nops;
+                    std::reverse_copy(tO[k], tO[k] + nops, out->ops + po);
+                    po += nops;
+                    it.start_row = S[tb::slot_start_r()];
+                    it.start_col = S[tb::slot_start_c()];
+                    it.xp_off = px;
+                    out->xpoints[px++] = swb_xpoint{0, 0, it.start_row, it.start_col};
+                    for (int64_t q = nxp - 1; q >= 0; --q) {
+                        const int64_t *d = tX[k] + 4 * q;
+                        out->xpoints[px++] = swb_xpoint{(int32_t)d[3], (int32_t)d[2], d[0], d[1]};
+                    }
+                    out->xpoints[px++] = swb_xpoint{0, it.score, it.end_row, it.end_col};
+                    it.n_xpoints = px - it.xp_off;
+                }
+                out->ops_bytes = po;
+                out->ops[po] = 0;
+                out->n_xpoints = px;
             }
-            out->ops_bytes = po;
-            out->ops[po] = 0;
-            out->n_xpoints = px;
         }
         // traced pairs with score 0: no alignment; crosspoints [start = end]
         // (pairs with an empty sequence have none, as in swb_align_pair)

@@ -821,6 +821,7 @@ constexpr int kSegXps = 160;
 // A pair alone: below this many segments one corridor of precomputed blocks is as fast.
 constexpr int kSegPairMin = 8;
 constexpr int kSegChain = 32;  // records a batched pair's CTA looks at together
+constexpr int64_t kSegMax = 65536;  // segments of one launch
 constexpr int kSegMin = 3;     // segments a pair must have to be walked in segments
 
 struct SegArgs {
@@ -967,6 +968,27 @@ __global__ void seg_copy_kernel(const SegRec *rec, const char *sops, const int64
     int64_t *px = xps + 4 * off[2 * blockIdx.x + 1];
     for (int i = threadIdx.x; i < nops; i += blockDim.x) po[i] = sops[slot * kSegOps + i];
     for (int i = threadIdx.x; i < nx; i += blockDim.x) px[i] = sxps[slot * kSegXps * 4 + i];
+}
+
+// A walked pair's results in their final form: operations start -> end at
+// ops + off.ops, crosspoints [start, top -> bottom, end] at xps + off.xps.
+struct PackOff {
+    int64_t ops, xps, end_r, end_c;
+};
+__global__ void pack_results_kernel(const WalkArgs *args, const PackOff *offs, char *ops, swb_xpoint *xps) {
+    const WalkArgs &a = args[blockIdx.x];
+    const PackOff o = offs[blockIdx.x];
+    const int64_t nops = a.st[kStNOps], nxp = a.st[kStNXp];
+    for (int64_t i = threadIdx.x; i < nops; i += blockDim.x) ops[o.ops + i] = a.ops[nops - 1 - i];
+    swb_xpoint *x = xps + o.xps;
+    for (int64_t i = threadIdx.x; i < nxp; i += blockDim.x) {
+        const int64_t *d = a.xps + 4 * (nxp - 1 - i);
+        x[1 + i] = swb_xpoint{(int32_t)d[3], (int32_t)d[2], d[0], d[1]};
+    }
+    if (threadIdx.x == 0) {
+        x[0] = swb_xpoint{0, 0, a.st[kStStartR], a.st[kStStartC]};
+        x[1 + nxp] = swb_xpoint{0, a.score, o.end_r, o.end_c};
+    }
 }
 
 // Batched pairs: CTA b walks pairs b, b + gridDim.x, ... (each pair's whole matrix is
@@ -1482,6 +1504,43 @@ int walk_batch(cudaStream_t st, int sms, const WalkInputs *in, int64_t n, void *
     return SWB_OK;
 }
 
+int pack_results(cudaStream_t st, const void *d_args, int64_t n, const int64_t *host_states, const int64_t *ends,
+                 std::vector<int64_t> &offs, int64_t *ops_bytes, int64_t *n_xps, char **d_ops, swb_xpoint **d_xps,
+                 const Scratch &scr, std::string &err) {
+    offs.resize((size_t)(4 * n));
+    int64_t po = 0, px = 0;
+    for (int64_t i = 0; i < n; ++i) {
+        const int64_t *S = host_states + i * kStN;
+        int64_t *o = offs.data() + 4 * i;
+        o[0] = po;
+        o[1] = px;
+        o[2] = ends[2 * i];
+        o[3] = ends[2 * i + 1];
+        po += S[kStNOps];
+        px += S[kStNXp] + 2;
+    }
+    *ops_bytes = po;
+    *n_xps = px;
+    int64_t *d_off = (int64_t *)scr.ensure(scr.owner, kScrSegOff, sizeof(PackOff) * (size_t)n);
+    *d_ops = (char *)scr.ensure(scr.owner, kScrOps, (size_t)po + 1);
+    *d_xps = (swb_xpoint *)scr.ensure(scr.owner, kScrXps, sizeof(swb_xpoint) * (size_t)px);
+    cudaError_t e;
+    if (!d_off || !*d_ops || !*d_xps) {
+        err = "result buffers: out of device memory";
+        return SWB_ENOMEM;
+    }
+    static_assert(sizeof(PackOff) == 4 * sizeof(int64_t), "PackOff layout");
+    if ((e = scr.put(scr.owner, d_off, offs.data(), sizeof(PackOff) * (size_t)n)) == cudaSuccess) {
+        pack_results_kernel<<<(unsigned)n, 256, 0, st>>>((const WalkArgs *)d_args, (const PackOff *)d_off, *d_ops, *d_xps);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        err = std::string("batched results: ") + cudaGetErrorString(e);
+        return SWB_ECUDA;
+    }
+    return SWB_OK;
+}
+
 void pack_walk_args(const WalkInputs *in, int64_t n, int64_t *d_states, void *dst) {
     WalkArgs *out = (WalkArgs *)dst;
     for (int64_t i = 0; i < n; ++i) {
@@ -1516,9 +1575,10 @@ int64_t seg_plan(const int64_t *rows, int64_t n, int sms, std::vector<int32_t> &
     items.clear();
     int64_t total = 0;
     for (int64_t p = 0; p < n; ++p) total += (rows[p] + kBR - 1) / kBR;
-    // beyond two waves of CTAs the pairs themselves fill the GPU, and walking
-    // segments twice only costs
-    if (total > 2 * walk_graph_ctas(sms)) return 0;
+    // (9 KB of records and outputs each.)  Segments pay even where the pairs alone fill
+    // the GPU: few are walked twice, and none is left over at the end (1,000 long
+    // pairs of the 100,000-pair batch: 6.4 ms, against about 15 ms walked pair by pair).
+    if (total > kSegMax) return 0;
     int32_t seg = 0;
     for (int64_t p = 0; p < n; ++p) {
         const int32_t k = (int32_t)((rows[p] + kBR - 1) / kBR);

@@ -100,6 +100,12 @@ int walk_region(cudaStream_t st, int sms, const WalkInputs &in, int64_t *host_st
 int walk_batch(cudaStream_t st, int sms, const WalkInputs *in, int64_t n, void *d_args, int64_t *d_states,
                void *d_dir, int64_t *host_states, const Scratch &scr, std::string &err, int32_t *launches);
 size_t walk_batch_dir_bytes(int sms, int64_t n);
+// Results of n walked pairs (as walk_batch left them; ends: end cell per pair) laid
+// out on the device in their final form, pair after pair: offs holds per pair
+// {first operation, first crosspoint, end row, end column}.
+int pack_results(cudaStream_t st, const void *d_args, int64_t n, const int64_t *host_states, const int64_t *ends,
+                 std::vector<int64_t> &offs, int64_t *ops_bytes, int64_t *n_xps, char **d_ops, swb_xpoint **d_xps,
+                 const Scratch &scr, std::string &err);
 
 // Graphed batches (the header's walk_args / walk_states / walk_dir hold every
 // pair of the batch): writes the walker arguments of n pairs into dst (host
