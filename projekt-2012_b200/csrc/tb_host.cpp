@@ -60,6 +60,8 @@ int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const 
     w.xps = d_xps;
     w.xp_cap = xp_cap;
     w.dstate = d_state;
+    w.rr1 = m;
+    w.cc1 = n;
     int rc;
     if (!plan.level1) {
         w.br = plan.br;
@@ -202,32 +204,24 @@ int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const 
                 err = "level-1 recompute: a bounded wait between strips ran out";
                 return SWB_ETIMEOUT;
             }
-            // walk cell after cell while the path stays in the corridor
-            for (;;) {
-                const int64_t rr = S[slot_r()], ccc = S[slot_c()];
-                if (S[slot_done()] || rr < 0 || ccc < 0) break;
-                const int64_t RR0 = (rr / plan.kr) * plan.kr, CC0 = (ccc / plan.kc) * plan.kc;
-                int64_t q = -1;
-                for (int64_t t = 0; t < ncell; ++t)
-                    if (cells[2 * t] == RR0 && cells[2 * t + 1] == CC0) {
-                        q = t;
-                        break;
-                    }
-                if (q < 0) break;  // left the corridor: next round
+            // walk through the cells while the path stays in the corridor
+            std::vector<WalkInputs> regs((size_t)ncell, w);
+            for (int64_t q = 0; q < ncell; ++q) {
                 const BatchPair &d = bp[(size_t)q];
-                w.srows = s2r + d.sr_off;
-                w.scols = s2c + d.sc_off;
-                w.rr0 = RR0;
-                w.cc0 = CC0;
-                w.rr1 = RR0 + d.m;
-                w.cc1 = CC0 + d.n;
-                w.rtop = d.top;
-                w.rleft = d.left;
-                if ((rc = walk_region(st, sms, w, S.data(), scr, err, launches)) != SWB_OK) return rc;
-                if (S[slot_r()] == rr && S[slot_c()] == ccc && !S[slot_done()]) {
-                    err = "traceback made no progress in a level-1 cell";
-                    return SWB_ECUDA;
-                }
+                WalkInputs &x = regs[(size_t)q];
+                x.srows = s2r + d.sr_off;
+                x.scols = s2c + d.sc_off;
+                x.rr0 = cells[2 * q];
+                x.cc0 = cells[2 * q + 1];
+                x.rr1 = x.rr0 + d.m;
+                x.cc1 = x.cc0 + d.n;
+                x.rtop = d.top;
+                x.rleft = d.left;
+            }
+            if ((rc = walk_cells(st, sms, w, regs, plan.kr, plan.kc, S.data(), scr, err, launches)) != SWB_OK) return rc;
+            if (S[slot_r()] == r && S[slot_c()] == c && !S[slot_done()]) {
+                err = "traceback made no progress in a level-1 cell";
+                return SWB_ECUDA;
             }
         }
         if (!S[slot_done()]) {

@@ -27,13 +27,15 @@
 // halves (four of 128 rows in 32 bits for scoring too wide for them), handing rows
 // down through shared memory with tagged 64-bit words instead of barriers.
 // Pairs whose stores would not fit the HBM budget keep a coarser grid (level 1);
-// each level-1 cell the path enters is recomputed by the stage-1 kernel on that
-// sub-rectangle, which writes the 512 x 256 stores for it (level 2).
+// each level-1 cell near the expected path is recomputed by the batched scoring
+// kernel on that sub-rectangle, which writes the 512 x 256 stores for it (level 2),
+// and the corridors of blocks run across the cells.
 #include <algorithm>
 #include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <unordered_map>
 #include <vector>
 
 #include "batch.h"
@@ -677,6 +679,30 @@ __global__ void __launch_bounds__(WIDE ? kThreadsWide : kThreads) precompute_ker
     if (threadIdx.x == 0 && xc.err) atomicExch(err, 1);
 }
 
+// The same for blocks of several regions (level-1 cells): reg[b] is block b's.
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? kThreadsWide : kThreads)
+    precompute_cells_kernel(const WalkArgs *regs, const int64_t *blk, const int32_t *reg, int64_t nblk, uint32_t *gdir,
+                            int32_t *err) {
+    __shared__ Xchg xc;
+    __shared__ Stage sg;
+    __shared__ WalkArgs a;
+    xchg_init(&xc);
+    uint32_t gen = 0;
+    for (int64_t b = blockIdx.x; b < nblk; b += gridDim.x) {
+        __syncthreads();
+        if (threadIdx.x == 0) a = regs[reg[b]];
+        __syncthreads();
+        const int64_t R0 = blk[2 * b], C0 = blk[2 * b + 1];
+        const int64_t R1 = min(R0 + a.br - 1, a.rr1 - 1), C1 = min(C0 + kBC - 1, a.cc1 - 1);
+        stage_block(a, R0, R1, C0, C1, &sg);
+        __syncthreads();
+        recompute<WIDE>(a, R0, R1, C0, C1, gdir + b * kBlockWords, &xc, &sg, ++gen);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && xc.err) atomicExch(err, 1);
+}
+
 // One warp walks the path through precomputed blocks: block (bi, bj) of the
 // region (relative to rr0, cc0) is slot map[(bi - bi0) * mw + (bj - bj0)] of
 // gdir, or absent (-1).  Stops where the path enters an absent block, at the
@@ -1131,6 +1157,8 @@ cudaError_t walker_configure() {
     cudaError_t e = cudaSuccess;
     for (cudaError_t x : {cudaFuncSetAttribute((const void *)precompute_kernel<false>, A, c),
                           cudaFuncSetAttribute((const void *)precompute_kernel<true>, A, c),
+                          cudaFuncSetAttribute((const void *)precompute_cells_kernel<false>, A, c),
+                          cudaFuncSetAttribute((const void *)precompute_cells_kernel<true>, A, c),
                           cudaFuncSetAttribute((const void *)corridor_walk_kernel, A, c),
                           cudaFuncSetAttribute((const void *)corridor_walk_kernel,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDirTileBytes),
@@ -1385,11 +1413,10 @@ int walk_region(cudaStream_t st, int sms, const WalkInputs &in, int64_t *host_st
     }
     std::vector<int64_t> blk;
     std::vector<int32_t> map;
-    // a whole pair of many blocks: segments at once as long as they continue the path,
-    // a corridor round where they do not
-    const bool whole = in.rr0 == 0 && in.cc0 == 0 && !in.rtop && !in.rleft && in.rr1 == in.m && in.cc1 == in.n;
+    // a pair of many blocks: segments at once as long as they continue the path, a
+    // corridor round where they do not
     for (int round = 0; round < (1 << 26); ++round) {
-        if (whole && !host_state[kStDone] && host_state[kStR] >= kSegPairMin * (int64_t)a.br) {
+        if (!host_state[kStDone] && host_state[kStR] >= kSegPairMin * (int64_t)a.br) {
             int64_t taken = 0;
             const int rc = walk_pair_segments(st, sms, in, a, host_state, scr, err, launches, &taken);
             if (rc != SWB_OK) return rc;
@@ -1421,6 +1448,93 @@ int walk_region(cudaStream_t st, int sms, const WalkInputs &in, int64_t *host_st
         if ((e = cudaGetLastError()) != cudaSuccess ||
             (e = scr.get(scr.owner, host_state, in.dstate, sizeof(int64_t) * kStN)) != cudaSuccess) {
             err = std::string("walker: ") + cudaGetErrorString(e);
+            return SWB_ECUDA;
+        }
+        if (host_state[kStR] == r && host_state[kStC] == c && !host_state[kStDone] && !host_state[kStErr]) {
+            err = "walker: no progress through the current block";
+            return SWB_ECUDA;
+        }
+    }
+    if (host_state[kStErr]) {
+        err = "walker: inconsistent direction data";
+        return SWB_ECUDA;
+    }
+    return SWB_OK;
+}
+
+int walk_cells(cudaStream_t st, int sms, const WalkInputs &whole, const std::vector<WalkInputs> &cells, int64_t kr,
+               int64_t kc, int64_t *host_state, const Scratch &scr, std::string &err, int32_t *launches) {
+    WalkInputs base = whole;
+    base.br = kBR;
+    const WalkArgs a = to_args(base);
+    const int64_t cap = 4LL * std::max(1, sms);
+    std::vector<WalkArgs> regs(cells.size());
+    std::unordered_map<int64_t, int32_t> find;  // (cell row, cell column) -> region
+    for (size_t q = 0; q < cells.size(); ++q) {
+        regs[q] = to_args(cells[q]);
+        find.emplace((cells[q].rr0 / kr << 32) | (cells[q].cc0 / kc), (int32_t)q);
+    }
+    cudaError_t e;
+    uint32_t *gdir = (uint32_t *)scr.ensure(scr.owner, kScrGdir, sizeof(uint32_t) * (size_t)(cap * kBlockWords));
+    WalkArgs *d_regs = (WalkArgs *)scr.ensure(scr.owner, kScrSegItems, sizeof(WalkArgs) * regs.size());
+    int32_t *d_err = (int32_t *)scr.ensure(scr.owner, kScrWalkErr, sizeof(int32_t));
+    if (!gdir || !d_regs || !d_err) {
+        err = "walker buffers: out of device memory";
+        return SWB_ENOMEM;
+    }
+    if ((e = cudaMemsetAsync(d_err, 0, sizeof(int32_t), st)) != cudaSuccess ||
+        (e = scr.put(scr.owner, d_regs, regs.data(), sizeof(WalkArgs) * regs.size())) != cudaSuccess ||
+        (e = scr.put(scr.owner, base.dstate, host_state, sizeof(int64_t) * kStN)) != cudaSuccess) {
+        err = std::string("walker cells: ") + cudaGetErrorString(e);
+        return SWB_ECUDA;
+    }
+    std::vector<int64_t> blk;
+    std::vector<int32_t> map, reg;
+    std::vector<char> up;
+    for (int round = 0; round < (1 << 26); ++round) {
+        const int64_t r = host_state[kStR], c = host_state[kStC];
+        if (host_state[kStDone] || host_state[kStErr] || r < 0 || c < 0) break;
+        if (find.find((r / kr << 32) | (c / kc)) == find.end()) break;  // the path left the cells
+        int64_t bi0, bj0, mh, mw;
+        predict_corridor(base, r, c, cap, blk, bi0, bj0, mh, mw, map);
+        // blocks of cells that are there, their regions and their slots
+        std::vector<int32_t> slot(blk.size() / 2, -1);
+        int32_t kept = 0;
+        reg.clear();
+        for (size_t b = 0; b < slot.size(); ++b) {
+            const auto it = find.find((blk[2 * b] / kr << 32) | (blk[2 * b + 1] / kc));
+            if (it == find.end()) continue;
+            blk[2 * (size_t)kept] = blk[2 * b];
+            blk[2 * (size_t)kept + 1] = blk[2 * b + 1];
+            reg.push_back(it->second);
+            slot[b] = kept++;
+        }
+        for (int32_t &v : map)
+            if (v >= 0) v = slot[(size_t)v];
+        const size_t nb = sizeof(int64_t) * 2 * (size_t)kept, nr = sizeof(int32_t) * (size_t)kept,
+                     nm = sizeof(int32_t) * map.size();
+        up.resize(nb + nr + nm);
+        std::memcpy(up.data(), blk.data(), nb);
+        std::memcpy(up.data() + nb, reg.data(), nr);
+        std::memcpy(up.data() + nb + nr, map.data(), nm);
+        char *d_up = (char *)scr.ensure(scr.owner, kScrMap, up.size());
+        if (!d_up) {
+            err = "walker buffers: out of device memory";
+            return SWB_ENOMEM;
+        }
+        if ((e = scr.put(scr.owner, d_up, up.data(), up.size())) != cudaSuccess) {
+            err = std::string("walker cells: ") + cudaGetErrorString(e);
+            return SWB_ECUDA;
+        }
+        const int64_t *d_blk = (const int64_t *)d_up;
+        const int32_t *d_reg = (const int32_t *)(d_up + nb), *d_map = (const int32_t *)(d_up + nb + nr);
+        if (a.wide) precompute_cells_kernel<true><<<(unsigned)kept, kThreadsWide, 0, st>>>(d_regs, d_blk, d_reg, kept, gdir, d_err);
+        else precompute_cells_kernel<false><<<(unsigned)kept, kThreads, 0, st>>>(d_regs, d_blk, d_reg, kept, gdir, d_err);
+        corridor_walk_kernel<<<1, 32, kDirTileBytes, st>>>(a, gdir, d_map, bi0, bj0, mh, mw, d_err);
+        *launches += 2;
+        if ((e = cudaGetLastError()) != cudaSuccess ||
+            (e = scr.get(scr.owner, host_state, base.dstate, sizeof(int64_t) * kStN)) != cudaSuccess) {
+            err = std::string("walker cells: ") + cudaGetErrorString(e);
             return SWB_ECUDA;
         }
         if (host_state[kStR] == r && host_state[kStC] == c && !host_state[kStDone] && !host_state[kStErr]) {

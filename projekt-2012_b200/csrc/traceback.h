@@ -87,11 +87,17 @@ enum ScratchSlot {
     kScrSegRec, kScrSegItems, kScrSegOff, kScrSlots
 };
 
-// Walks the path from host_state's cell through the region of `in` (until the
-// start cell or the region's top/left edge): rounds of a predicted corridor of
-// whole blocks precomputed in parallel, then walked by one warp.
+// Walks the path of a whole pair from host_state's cell to the start cell: segments
+// walked at the same time, and rounds of a predicted corridor of whole blocks
+// precomputed in parallel, then walked by one warp.
 int walk_region(cudaStream_t st, int sms, const WalkInputs &in, int64_t *host_state, const Scratch &scr,
                 std::string &err, int32_t *launches);
+
+// The same through the recomputed level-1 cells (regions of kr x kc cells of the
+// whole matrix, with their own stores): the corridors run across cells, until the
+// start cell or a cell that is not there.
+int walk_cells(cudaStream_t st, int sms, const WalkInputs &whole, const std::vector<WalkInputs> &cells, int64_t kr,
+               int64_t kc, int64_t *host_state, const Scratch &scr, std::string &err, int32_t *launches);
 
 // Walks n independent pairs (each region is its pair's whole matrix) with one
 // launch; d_args holds n * walk_args_bytes() bytes, d_states n * state_slots()
