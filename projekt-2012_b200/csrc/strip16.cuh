@@ -77,9 +77,10 @@ struct Sub {
 };
 constexpr int kColRing = 128;  // column values kept: 63 behind (the high half of lane 31), 63 ahead
 
-// Runs kept at once (the one in progress included).
+// Runs kept at once (the one in progress included).  Eight instead of three 256-row
+// strips' runs: unrelated 15 kbp pair, stage 1 1.59 -> 1.54 ms.
 template <int RH>
-constexpr int kKept = RH <= 8 ? 3 : 2;
+constexpr int kKept = RH <= 4 ? 8 : (RH <= 8 ? 3 : 2);
 
 // A warp's shared memory.
 template <int RH>
@@ -227,11 +228,40 @@ __device__ __forceinline__ void put_state(WarpMem<RH> *w, int q, int lane, const
     w->save[q][(RH + 1) / 2][lane] = make_uint4(L.inHO, L.inF, L.hod, 0);
 }
 
-// Column value of column c: the table word (TAB) or the byte's code (CMP).
+// What column c is read as: the table word (TAB) or the byte; and its column value.
+template <bool TAB>
+__device__ __forceinline__ uint32_t read_col(const uint32_t *ctab, const uint8_t *cols, int32_t c) {
+    return TAB ? ctab[c] : (uint32_t)cols[c];
+}
+template <bool TAB>
+__device__ __forceinline__ uint32_t col_value(uint32_t v) {
+    return TAB ? v : v << 6;
+}
 template <bool TAB>
 __device__ __forceinline__ uint32_t col2(const uint32_t *ctab, const uint8_t *cols, int32_t c) {
-    if (TAB) return ctab[c];
-    return (uint32_t)cols[c] << 6;
+    return col_value<TAB>(read_col<TAB>(ctab, cols, c));
+}
+
+// The loads that are issued a run before their values are used write the very
+// registers that are carried around the loop, whatever was in them having been used
+// before, and are predicated.  Written as assignments in branches they were given
+// registers of their own, and the moves into the carried ones, put right behind the
+// loads, waited for each: a refill of a lone warp's 256-row strip took 1000 to 1300
+// cycles of a run's 3400, and takes 600 (score only, 61 kbp pair: 4.6 -> 3.75 ms).
+__device__ __forceinline__ void ld_hand(int4 &v, bool on, const int4 *p) {
+    asm volatile("{.reg .pred p; setp.ne.s32 p, %5, 0; @p ld.volatile.global.v4.s32 {%0,%1,%2,%3}, [%4];}"
+                 : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+                 : "l"(p), "r"((int)on));
+}
+template <bool TAB>
+__device__ __forceinline__ void ld_col(uint32_t &v, bool on, const uint32_t *ctab, const uint8_t *cols, int32_t c) {
+    if (TAB)
+        asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p ld.global.u32 %0, [%1];}" : "+r"(v) : "l"(ctab + c), "r"((int)on));
+    else
+        asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p ld.global.u8 %0, [%1];}" : "+r"(v) : "l"(cols + c), "r"((int)on));
+}
+__device__ __forceinline__ void ld_best(int32_t &v, const int32_t *p) {
+    asm volatile("ld.volatile.global.s32 %0, [%1];" : "+r"(v) : "l"(p));
 }
 
 // Row selector (TAB) or code (CMP) of rows r0 + i and r0 + 32 RH + i.
@@ -367,10 +397,10 @@ __device__ __forceinline__ int4 above2(const A &a, int32_t strip, int32_t c) {
 
 // Column c's entry, loaded earlier, as offsets from base (loading it again until
 // the strip above has written it).  Returns false when the wait ran out; clears
-// range when the entry does not fit the window.
+// range when the entry does not fit the window (lo to 32767 - near).
 template <class A>
 __device__ __forceinline__ bool commit2(const A &a, uint32_t *slot, int32_t strip, int32_t c, int4 h, int32_t base,
-                                        int32_t near, bool &range) {
+                                        int32_t lo, int32_t near, bool &range) {
     if (strip > 0 && (h.y != strip - 1 || h.w != strip - 1)) {
         const long long t0 = clock64();
         const long long limit = a.wait_limit > 0 ? a.wait_limit : kWaitLimitCycles;
@@ -382,15 +412,15 @@ __device__ __forceinline__ bool commit2(const A &a, uint32_t *slot, int32_t stri
         }
     }
     const int32_t d = h.z - base, ho = half16((uint32_t)h.x, 0) + d, f = half16((uint32_t)h.x, 1) + d;
-    if (max(ho, f) > 32767 - near || min(ho, f) < (base > 0 ? near : -32768)) range = false;
+    if (max(ho, f) > 32767 - near || min(ho, f) < lo) range = false;
     *slot = ((uint32_t)ho & 0xFFFFu) | ((uint32_t)f << 16);
     return true;
 }
 
-// The value of a column outside the matrix: a mismatch for every row.
+// What a column outside the matrix is read as: a mismatch for every row.
 template <bool TAB>
 __device__ __forceinline__ uint32_t no_column(int32_t mm1) {
-    return TAB ? (uint32_t)(uint8_t)(int8_t)mm1 * 0x01010101u : 257u << 6;
+    return TAB ? (uint32_t)(uint8_t)(int8_t)mm1 * 0x01010101u : 257u;
 }
 
 // Keeps column c's value.
@@ -468,9 +498,6 @@ __device__ __forceinline__ void steps2(Lane2<RH> &L, const uint32_t *ra, const C
     }
 }
 
-// What the lanes agree on before a run.
-enum : uint32_t { kVoteBase = 1, kVoteTimeout = 2, kVoteRange = 4, kVoteTrack = 8 };
-
 // Runs strip s.  (Kernels without STORES serve no launch with a left boundary or a
 // right border.)  w->best_* holds the warp's best cell (kept over strips by the
 // caller).  STORES: the launch keeps special rows or columns or a block's borders.
@@ -544,8 +571,12 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     // column 0's row above, then the first run's (columns 1..32) and column values
     // [0, 64).  From here on both are loaded a run before they are stored, more
     // than the ~800 cycles of an L2 round trip.
-    bool ok = true, range = true;
-    if (lane == 0) ok = commit2(a, w->ring, s, 0, above2(a, s, 0), base, win.near, range);
+    int32_t wlo = base > 0 ? win.lo : -32768, wnear = base > 0 ? win.near : -32768;  // the window's lower ends
+    {
+        bool ok = true, range = true;
+        if (lane == 0) ok = commit2(a, w->ring, s, 0, above2(a, s, 0), base, wnear, win.near, range);
+        if (!__all_sync(0xffffffffu, ok && range)) return __all_sync(0xffffffffu, ok) ? kErrRange : kErrTimeout;
+    }
     __syncwarp();
     {
         // what the shuffles of the step before column 0 would have brought
@@ -568,10 +599,10 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     // a wanted right border needs the predicates.
     const bool exact = a.left != nullptr || a.right != nullptr;
     const uint32_t none = no_column<TAB>(a.mm1);
-    put_col(w->col, lane, lane < n ? col2<TAB>(a.ctab, a.cols, lane) : none);
-    put_col(w->col, lane - 32, none);
-    put_col(w->col, lane - 64, none);
-    uint32_t cv = kRun + lane < n ? col2<TAB>(a.ctab, a.cols, kRun + lane) : none;
+    put_col(w->col, lane, col_value<TAB>(lane < n ? read_col<TAB>(a.ctab, a.cols, lane) : none));
+    put_col(w->col, lane - 32, col_value<TAB>(none));
+    put_col(w->col, lane - 64, col_value<TAB>(none));
+    uint32_t cv = kRun + lane < n ? read_col<TAB>(a.ctab, a.cols, kRun + lane) : none;
     if (a.trace && lane == 0) {  // the strip above has delivered column 0
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
@@ -587,7 +618,6 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     const int32_t kEnd = n + 63;
     for (int32_t k = 0;; k += kRun) {
         const bool end = k >= kEnd;
-        if (end && !__all_sync(0xffffffffu, ok && range)) return __all_sync(0xffffffffu, ok) ? kErrRange : kErrTimeout;
         if (end || kept == kKept<RH>) {
             // the kept runs again, unless a better cell was found elsewhere; in the
             // middle of the strip the lanes' rows wait in shared memory
@@ -631,47 +661,56 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
             L.inF = inF;
             L.hod = hod;
         }
-        // refill: the stored rows of the last run out, the base moved when a bottom
-        // row leaves the window, the next run's row above and the columns of the
-        // run after it in
+        // refill: the next run's row above and the columns of the run after it in.  One
+        // vote says whether every lane is inside its window and every entry is there
+        // and close to the base; the lanes that would wait or move the base are rare.
         const uint32_t bot = L.HO[RH - 1];
         const int32_t vmax = max16(bot), vmin = min(half16(bot, 0), half16(bot, 1));
+        const int32_t q = k + 1 + lane, qc = k + kRun + lane;
+        const int32_t ub = up4.z - base, uho = half16((uint32_t)up4.x, 0) + ub, uf = half16((uint32_t)up4.x, 1) + ub;
         thr = max(thr, gpre + a.open);
-        gpre = ld_volatile(a.gbest);
-        const uint32_t votes = __reduce_or_sync(
-            0xffffffffu, (vmax > win.hi || (base > 0 && vmin < win.lo) ? kVoteBase : 0u) | (ok ? 0u : kVoteTimeout) |
-                             (range ? 0u : kVoteRange) | (vmax + win.reach >= thr - base ? kVoteTrack : 0u));
-        if (votes & (kVoteBase | kVoteTimeout | kVoteRange)) {
-            if (votes & kVoteTimeout) return kErrTimeout;
-            if (votes & kVoteRange) return kErrRange;
-            const int32_t hi = __reduce_max_sync(0xffffffffu, vmax), lo = __reduce_min_sync(0xffffffffu, vmin);
-            const int32_t mid = base + (lo + hi) / 2;
-            const int32_t nb = mid > 16384 ? mid - 16384 : 0;
-            const int32_t d = base - nb;
-            if (hi + d > win.hi || (nb > 0 && lo + d < win.lo)) return kErrRange;
-            const uint32_t d2 = dup16(d);
+        const bool track = __any_sync(0xffffffffu, vmax + win.reach >= thr - base);  // some cell of this run may reach the best known
+        const bool mine = vmax <= win.hi && vmin >= wlo;
+        const bool entry = q >= n || (max(uho, uf) <= 32767 - win.near && min(uho, uf) >= wnear &&
+                                      (s == 0 || (up4.y == s - 1 && up4.w == s - 1)));
+        if (__all_sync(0xffffffffu, mine && entry)) {
+            w->ring[lane] = q < n ? ((uint32_t)uho & 0xFFFFu) | ((uint32_t)uf << 16) : bot;  // past the end any value of the window
+        } else {
+            if (__any_sync(0xffffffffu, !mine)) {
+                // the base moves so that the bottom rows are in the middle of the window
+                const int32_t hi = __reduce_max_sync(0xffffffffu, vmax), lo = __reduce_min_sync(0xffffffffu, vmin);
+                const int32_t mid = base + (lo + hi) / 2;
+                const int32_t nb = mid > 16384 ? mid - 16384 : 0;
+                const int32_t d = base - nb;
+                if (hi + d > win.hi || (nb > 0 && lo + d < win.lo)) return kErrRange;
+                const uint32_t d2 = dup16(d);
 #pragma unroll
-            for (int i = 0; i < RH; ++i) {
-                L.HO[i] = __vadd2(L.HO[i], d2);
-                L.E[i] = __vadd2(L.E[i], d2);
+                for (int i = 0; i < RH; ++i) {
+                    L.HO[i] = __vadd2(L.HO[i], d2);
+                    L.E[i] = __vadd2(L.E[i], d2);
+                }
+                L.inHO = __vadd2(L.inHO, d2);
+                L.inF = __vadd2(L.inF, d2);
+                L.hod = __vadd2(L.hod, d2);
+                base = nb;
+                t.base = base;
+                wlo = base > 0 ? win.lo : -32768;
+                wnear = base > 0 ? win.near : -32768;
             }
-            L.inHO = __vadd2(L.inHO, d2);
-            L.inF = __vadd2(L.inF, d2);
-            L.hod = __vadd2(L.hod, d2);
-            base = nb;
-            t.base = base;
+            bool ok = true, range = true;
+            if (q < n) ok = commit2(a, w->ring + lane, s, q, up4, base, wnear, win.near, range);
+            else w->ring[lane] = L.HO[RH - 1];
+            if (!__all_sync(0xffffffffu, ok && range)) return __all_sync(0xffffffffu, ok) ? kErrRange : kErrTimeout;
         }
-        {
-            const int32_t q = k + 1 + lane, qc = k + kRun + lane;
-            const int4 h = up4;
-            const uint32_t v = cv;
-            if (q + kRun < n) up4 = above2(a, s, q + kRun);
-            cv = qc + kRun < n ? col2<TAB>(a.ctab, a.cols, qc + kRun) : none;
-            put_col(w->col, qc, v);
-            if (q < n) ok = ok && commit2(a, w->ring + lane, s, q, h, base, win.near, range);
-            else w->ring[lane] = dup16(base > 0 ? win.lo : a.open);  // any value of the window
+        put_col(w->col, qc, col_value<TAB>(cv));
+        if (s > 0) {
+            ld_hand(up4, q + kRun < n, a.hbuf + (q + kRun));
+        } else if (a.top && q + kRun < n) {
+            up4 = above2(a, s, q + kRun);
         }
-        const bool track = (votes & kVoteTrack) != 0;  // some cell of this run may reach the best known
+        cv = none;
+        ld_col<TAB>(cv, qc + kRun < n, a.ctab, a.cols, qc + kRun);
+        ld_best(gpre, a.gbest);
         const int32_t rel = thr - base;
         __syncwarp();
 
@@ -720,7 +759,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         }
         // did it reach the best H known?
         const int32_t top = max16(mx);
-        if (__any_sync(0xffffffffu, top >= rel)) {
+        if ((track || mode != kPlain || sc_run) && __any_sync(0xffffffffu, top >= rel)) {
             const int32_t val = __reduce_max_sync(0xffffffffu, top) + base;
             if (lane == 0) {
                 if (val > thr) atomicMax(a.gbest, val - a.open);
