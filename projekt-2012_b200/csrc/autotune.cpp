@@ -13,7 +13,10 @@
 // spacing is the other tuned parameter; it is chosen from the HBM budget by the
 // traceback planner (the densest grid that fits).
 //
-// Batches: the packed 16-bit pass takes 448- or 256-row strips.  Short pairs pad
+// Packed 16-bit strips with stores, and short ones without, follow a rule instead
+// (autotune_rows_per_lane).
+//
+// Batches: the large score-only pass takes 448- or 256-row strips.  Short pairs pad
 // less with 256 rows, long ones run fewer per-strip steps with 448, so the
 // choice depends on the batch's length mix.  Its bucket is the SM count and
 // ceil(log2) of the cells-weighted median rows and columns of the packed pairs;

@@ -6,15 +6,19 @@
 // the single-pair ones (stage1_core.cuh), so a pair scores exactly the same
 // alone or in a batch.
 //
-// Work units.  A pair with m rows has ceil(m / 512) strips of 512 rows (16 rows
-// per lane).  The host lists every strip of every pair as one work unit, pair
+// Strips are the packed 16-bit ones of strip16.cuh, or 32-bit ones (stage1_core.cuh)
+// where the scoring parameters are too wide for them.
+//
+// Work units.  A pair with m rows has ceil(m / H) strips of H rows (256, 448 or
+// 512, the same in a launch).  The host lists every strip of every pair as one work unit, pair
 // after pair (longest pairs first, each pair's strips in order), and warps claim
 // units from a device counter.  A unit's only dependency is the strip above it,
 // which an earlier claim gave to a warp that is already running, so every wait
-// ends whether or not the whole grid is resident at once.  A short pair (<= 512 rows) is one unit: one
-// warp aligns it alone (inter-sequence mapping).  A longer pair's strips run on
-// consecutive warps that pass the strip's bottom row down through the pair's
-// tagged row buffer as in the single-pair kernel (intra-sequence wavefront).
+// ends whether or not the whole grid is resident at once.  A pair of one strip
+// is one unit: one warp aligns it alone (inter-sequence mapping).  A longer pair's
+// strips run on consecutive warps that pass the strip's bottom row down through the
+// pair's tagged row buffer as in the single-pair kernel (intra-sequence wavefront),
+// or, in large launches, strip after strip on one warp (kWholePair).
 //
 // Each unit records the best cell of its strip; a second kernel merges the
 // strips of each pair (a warp per pair) into the pair's record, which may carry

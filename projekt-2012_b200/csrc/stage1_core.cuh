@@ -1,5 +1,7 @@
-// stage1_core.cuh -- device core of the scoring wavefront, shared by the pair
-// kernel (stage1.cu) and the batched kernel (batch.cu).
+// stage1_core.cuh -- device core of the scoring wavefront in 32 bits, shared by
+// the pair kernel (stage1.cu) and the batched kernel (batch.cu).  Both run the
+// packed 16-bit strips of strip16.cuh instead where the scoring parameters allow
+// it; the best-cell and tie-key functions here serve both.
 //
 // Follows the recurrence of the reference's shortPhase/longPhase kernels
 // (src/FindAlignment.cuh:50-104, twin :187-241) with this library's own layout: a
@@ -124,40 +126,6 @@ __device__ __forceinline__ int32_t slow_best(uint32_t mask, int32_t cm, const Ti
             b->key = key;
             b->row = r;
             b->col = j;
-        }
-    }
-    if (b->ho > before) atomicMax(gbest, b->ho - open);
-    return b->ho;
-}
-
-// The same update with the rows past the end masked first and a single
-// strictly-better cell taken without a loop.  The packed batch kernel runs
-// about 5% faster with this form; the single-pair kernels with slow_best
-// (code layout of the two differs; both give the same cell).
-__device__ __forceinline__ int32_t slow_best_single(uint32_t mask, int32_t cm, const TieGeom tie, int64_t m,
-                                                 int64_t r_origin, int64_t c_origin, Best *b, int64_t row0,
-                                                 int32_t j, int32_t *gbest, int32_t open) {
-    const int32_t before = b->ho;
-    if (row0 + 32 > m) mask &= (m - row0 > 0) ? (uint32_t)((1ULL << (m - row0)) - 1ULL) : 0u;
-    if (mask == 0) return b->ho;
-    if (cm > b->ho && (mask & (mask - 1)) == 0) {
-        b->ho = cm;
-        b->keyed = 0;
-        b->row = row0 + __ffs(mask) - 1;
-        b->col = j;
-    } else {
-        key_best(b, tie, r_origin, c_origin);
-        while (mask) {
-            const int i = __ffs(mask) - 1;
-            mask &= mask - 1;
-            const int64_t r = row0 + i;
-            const uint64_t key = tie_key(tie, r_origin + r, c_origin + j);
-            if (better(cm, key, b->ho, b->key)) {
-                b->ho = cm;
-                b->key = key;
-                b->row = r;
-                b->col = j;
-            }
         }
     }
     if (b->ho > before) atomicMax(gbest, b->ho - open);

@@ -21,8 +21,12 @@
 // from the current cell, with the blocks above and to the left as margin), and
 // then one warp walks the path through them (32 cells per ballot along
 // diagonal, row or column runs) until it reaches the start or leaves the
-// corridor, where the next round predicts from.  Batches of pairs use one CTA
-// per pair that recomputes the blocks on its path on demand.  Inside a CTA the
+// corridor, where the next round predicts from.  Before that, a pair of many
+// blocks is cut into segments at special rows: one CTA per segment guesses the
+// cell where the path crosses its lower row (the row's best H near the diagonal)
+// and walks from there on blocks it recomputes on demand; a chain of segments
+// whose ends meet is the path, whatever was guessed.  Batches of pairs use one CTA
+// per pair or segment.  Inside a CTA the
 // block recompute is a pipeline of two warps of 256 rows each in packed 16-bit
 // halves (four of 128 rows in 32 bits for scoring too wide for them), handing rows
 // down through shared memory with tagged 64-bit words instead of barriers.

@@ -81,10 +81,10 @@ struct Scratch {
     void *owner;
 };
 enum ScratchSlot {
-    kScrOps = 0, kScrXps, kScrState, kScrSrows2, kScrScols2, kScrHbuf, kScrWbest, kScrBest, kScrErr,
+    kScrOps = 0, kScrXps, kScrState, kScrSrows2, kScrScols2,
     kScrGdir, kScrBlk, kScrMap, kScrWalkErr,
     kScrL1Pairs, kScrL1Units, kScrL1Hbuf, kScrL1Gbest, kScrL1Ubest, kScrL1Pbest, kScrL1Ctl,
-    kScrSegRec, kScrSegItems, kScrSegOff, kScrSlots
+    kScrSegRec, kScrSegItems, kScrSegOff
 };
 
 // Walks the path of a whole pair from host_state's cell to the start cell: segments
