@@ -109,10 +109,17 @@ int autotune_rows_per_lane(swb_ctx *c, const Stage1Args &base, bool tab, bool st
     // Packed strips (strip16.cuh).  While every 256-row strip has a scheduler to
     // itself the strips' latency decides, and the lowest strips are fastest (90 kbp
     // pair, store pass: 9.8 ms with 256 rows, 10.8 with 448, 11.3 with 512, 17.1 with
-    // 1024); beyond that their fill does, and 448 rows are (172 kbp: 26.8, 20.6, 21.3,
-    // 32.6 ms; 1 Mbp: 341, 298, 322, 323 ms; score only 287, 263, 285, 285 ms).
+    // 1024); beyond that 448 rows are (172 kbp: 26.8, 20.6, 21.3, 32.6 ms; 1 Mbp: 341,
+    // 298, 322, 323 ms; score only 287, 263, 285, 285 ms).  All strips wait for the
+    // scheduler with the most of them, so where 512 rows need one strip fewer on it
+    // they win (store pass, 448 / 512 rows: 262 kbp 31.2 / 31.4 ms, one each; 296 kbp
+    // 52.0 / 35.6, two or one; 310 kbp 54.9 / 56.6, two each; 540 kbp 122 / 105, three
+    // or two; 620 kbp 149 / 150; 830 kbp 243 / 218, four or three).  Past four, what an
+    // SM holds, a scheduler's next strip starts as soon as one ends.
     if (packed) {
-        fallback = base.m <= 256LL * 4 * std::max(1, c->sms) ? 8 : 14;
+        const int64_t sched = 4LL * std::max(1, c->sms);
+        auto most = [&](int64_t rows) { return (base.m + rows * sched - 1) / (rows * sched); };
+        fallback = most(256) <= 1 ? 8 : (most(448) <= 4 && most(512) < most(448) ? 16 : 14);
         if (sr_interval > 0 && sr_interval % (16 * fallback) != 0) fallback = 16;
         if (stores) return fallback;
     }
