@@ -347,7 +347,7 @@ Stage1Plan stage1_plan(int64_t m, int64_t n, int device_sms, int R_hint, bool ta
 }
 
 cudaError_t stage1_launch(Stage1Args &a, const Stage1Plan &p, cudaStream_t st) {
-    const KernelRef k = kernel_of(p.R, p.tab, p.stores || a.srows || a.scols || (p.packed && (a.bottom || a.right || a.left)), p.packed);
+    const KernelRef k = kernel_of(p.R, p.tab, p.stores || a.srows || a.scols || (p.packed && stage1_has_borders(a)), p.packed);
     if (!k.fn) return cudaErrorInvalidValue;
     void *args[] = {&a};
     const cudaError_t e = cudaLaunchCooperativeKernel(k.fn, dim3(p.blocks), dim3(kWarps * 32), args, k.smem, st);

@@ -365,6 +365,37 @@ __device__ __forceinline__ void rerun(const A &a, WarpMem<RH> *w, Lane2<RH> &L, 
     __syncwarp();
 }
 
+// The cells of a block's first row that take H from the top border through F: cells of
+// the block like any other, though no maximum over t holds them.  Their H is F of row
+// 0, known with the border.  Takes the best of the lanes' cells (ho: H + open of (0, col),
+// where the cell's H is higher the steps find that) into the warp's best and returns
+// the threshold after it.
+template <int RH, class A>
+__device__ __forceinline__ int32_t take_border(const A &a, WarpMem<RH> *w, int lane, int32_t ho, int32_t col, int32_t thr) {
+    const int32_t best = __reduce_max_sync(0xffffffffu, ho);
+    if (best < thr) return thr;
+    uint64_t key = ho == best ? tie_key(a.tie, a.r_origin, a.c_origin + col) : ~0ULL;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const uint64_t okey = __shfl_xor_sync(0xffffffffu, key, off);
+        const int32_t ocol = __shfl_xor_sync(0xffffffffu, col, off);
+        if (okey < key) {
+            key = okey;
+            col = ocol;
+        }
+    }
+    if (lane == 0 && (best > w->best_ho || (best == w->best_ho && key < w->best_key))) {
+        if (best > thr) atomicMax(a.gbest, best - a.open);
+        w->best_ho = best;
+        w->best_valid = 1;
+        w->best_key = key;
+        w->best_row = 0;
+        w->best_col = col;
+    }
+    __syncwarp();
+    return best;
+}
+
 // Where a strip's last rows go besides the strip below.
 struct Out2 {
     int2 *row[2];  // per half: special row or the rectangle's last row (column 0), or null
@@ -498,7 +529,7 @@ __device__ __forceinline__ void steps2(Lane2<RH> &L, const uint32_t *ra, const C
     }
 }
 
-// Runs strip s.  (Kernels without STORES serve no launch with a left boundary or a
+// Runs strip s.  (Kernels without STORES serve no launch with a given boundary or a
 // right border.)  w->best_* holds the warp's best cell (kept over strips by the
 // caller).  STORES: the launch keeps special rows or columns or a block's borders.
 // Returns kErrNone, kErrTimeout or kErrRange.
@@ -612,6 +643,8 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     // the best H known anywhere, loaded a run before it is used
     int32_t gpre = ld_volatile(a.gbest);
     int32_t thr = max(w->best_ho, gpre + a.open);
+    const bool first_row = STORES && s == 0 && a.top != nullptr;  // cells take H from a given border through F
+    if (first_row) thr = take_border(a, w, lane, lane == 0 ? half16(L.inF, 0) + base + a.open : INT_MIN, 0, thr);
     // kept runs: slots first, first + 1, ... (cyclic), all with maximum kv
     int first = 0, kept = 0;
     int32_t kv = 0;
@@ -669,6 +702,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         const int32_t q = k + 1 + lane, qc = k + kRun + lane;
         const int32_t ub = up4.z - base, uho = half16((uint32_t)up4.x, 0) + ub, uf = half16((uint32_t)up4.x, 1) + ub;
         thr = max(thr, gpre + a.open);
+        if (first_row) thr = take_border(a, w, lane, q < n ? half16((uint32_t)up4.x, 1) + up4.z + a.open : INT_MIN, q, thr);
         const bool track = __any_sync(0xffffffffu, vmax + win.reach >= thr - base);  // some cell of this run may reach the best known
         const bool mine = vmax <= win.hi && vmin >= wlo;
         const bool entry = q >= n || (max(uho, uf) <= 32767 - win.near && min(uho, uf) >= wnear &&

@@ -70,6 +70,10 @@ struct Stage1Args {
     int2 *right;           // optional: (H, E) of the last column, m entries
 };
 
+// A launch over a block with given boundaries or wanted borders (packed strips run
+// it with the kernels that have stores).
+inline bool stage1_has_borders(const Stage1Args &a) { return a.top || a.left || a.bottom || a.right; }
+
 // Geometry of the reference's launch (src/SWutils.cpp:233-253) and padding
 // (src/FASTA.cpp:107-134).  Returns false when the reference could not launch.
 bool reference_geometry(int64_t rows, int64_t cols, int32_t *G, int32_t *T, int64_t *P1,

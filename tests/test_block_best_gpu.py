@@ -1,0 +1,49 @@
+"""The best cell of one block (swb_score_block_device): only cells of the block
+count, whatever its borders hold, for blocks with a top border, a left border, both,
+any number of rows, and table and compare scores, against the oracle's block."""
+import ctypes as C
+import random
+
+import numpy as np
+import pytest
+
+import oracle_ctypes as O
+import swb200
+
+pytestmark = pytest.mark.gpu
+
+
+def _best(ctx, rows, cols, sc, top, left, corner, r0, c0, full_m, full_n, tie):
+    """The block's best cell (score, row, col, key) on the GPU and from the oracle."""
+    import torch
+    dev = lambda x: None if x is None else torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    ptr = lambda t: None if t is None else C.c_void_p(t.data_ptr())
+    d_rows, d_cols = dev(np.frombuffer(rows, np.uint8).copy()), dev(np.frombuffer(cols, np.uint8).copy())
+    d_top, d_left, out, s = dev(top), dev(left), swb200.BlockBest(), swb200.scoring(*sc)
+    rc = swb200.lib().swb_score_block_device(
+        ctx._h, ptr(d_rows), len(rows), ptr(d_cols), len(cols), ptr(d_top), ptr(d_left), corner, r0, c0, full_m, full_n,
+        C.byref(s), swb200.FLAG_TIE_ROWMAJOR if tie else 0, None, None, C.byref(out))
+    assert rc == 0
+    _, _, e, key = O.block(rows, cols, O.scoring(*sc), top, left, corner, r0, c0, full_m, full_n, tie)
+    want = (e.score, e.row, e.col, key) if e.score > 0 else (0, -1, -1, (1 << 64) - 1)
+    return (out.score, out.row, out.col, out.key), want
+
+
+def _seq(rng, n, alph):
+    return bytes(rng.choices(alph, k=n))
+
+
+@pytest.mark.parametrize("n", [200, 700])
+@pytest.mark.parametrize("m", [1, 40, 512, 700])
+def test_cells_that_take_h_from_the_top_border_count(gpu_ctx, m, n):
+    """A top border with one peak and no match below it, gaps cheaper than mismatches:
+    the best cell is the one below the peak, whose H is its F (200 columns are scored in
+    32-bit strips, 700 in packed ones)."""
+    rng = random.Random(m + n)
+    top = np.zeros((n, 2), dtype=np.int32)
+    top[:, 0] = 300 - np.abs(np.arange(n) - n // 2)
+    top[:, 1] = top[:, 0] - 2
+    for alph in (b"CGT", b"CGTRYKM"):
+        for tie in (O.TIE_REFERENCE, O.TIE_ROWMAJOR):
+            got, want = _best(gpu_ctx, b"A" * m, _seq(rng, n, alph), (1, -3, -2, -2), top, None, 0, 512, 0, 4096, 1024, tie)
+            assert want[:3] == (298, 512, n // 2) and got == want
