@@ -435,7 +435,7 @@ int run_stage1(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_co
     Stage1Plan plan = stage1_plan(m, n, c->sms, R, tab, packed);
     if (c->max_blocks > 0 && plan.blocks > c->max_blocks) plan.blocks = c->max_blocks;
     const int64_t W = (int64_t)plan.blocks * plan.warps_per_block;
-    if ((e = c->wbest.ensure(sizeof(BestRec) * (size_t)W)) != cudaSuccess)
+    if ((e = c->wbest.ensure(sizeof(BestRec) * (size_t)(W + kStage1BorderRecs))) != cudaSuccess)
         return ctx_cuda_fail(c, e, "stage 1 buffers");
     a.nstrips = plan.nstrips;
     a.wbest = (BestRec *)c->wbest.p;

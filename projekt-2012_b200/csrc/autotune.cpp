@@ -173,7 +173,7 @@ int autotune_rows_per_lane(swb_ctx *c, const Stage1Args &base, bool tab, bool st
         p.stores = stores;
         if (c->max_blocks > 0 && p.blocks > c->max_blocks) p.blocks = c->max_blocks;
         const int64_t W = (int64_t)p.blocks * p.warps_per_block;
-        if (c->wbest.ensure(sizeof(BestRec) * (size_t)W) != cudaSuccess) return fallback;
+        if (c->wbest.ensure(sizeof(BestRec) * (size_t)(W + kStage1BorderRecs)) != cudaSuccess) return fallback;
         Stage1Args a = base;
         a.n = np;
         a.nstrips = p.nstrips;

@@ -180,7 +180,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs &g) {
 template <int RH, class S>
 __device__ __forceinline__ void packed_body(const BatchArgs &g, bool tab) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr bool STORES = !std::is_same<S, NoStores>::value;
+    constexpr int KIND = std::is_same<S, NoStores>::value ? kScore : (std::is_same<S, WithBounds>::value ? kBorders : kStores);
     const int lane = threadIdx.x & 31;
     WarpMem<RH> *w = reinterpret_cast<WarpMem<RH> *>(smem) + (threadIdx.x >> 5);
     for (;;) {
@@ -201,7 +201,7 @@ __device__ __forceinline__ void packed_body(const BatchArgs &g, bool tab) {
 #pragma unroll 1
         for (int32_t strip = s0; strip < s1 && rc == kErrNone; ++strip) {
             init_warp(w, lane, g.open);
-            rc = tab ? run_strip2<RH, true, STORES>(v, w, lane, strip) : run_strip2<RH, false, STORES>(v, w, lane, strip);
+            rc = tab ? run_strip2<RH, true, KIND>(v, w, lane, strip) : run_strip2<RH, false, KIND>(v, w, lane, strip);
             if (rc == kErrNone && lane == 0) {
                 BestRec r;
                 r.ho = w->best_ho;

@@ -156,7 +156,7 @@ __global__ void prepare_kernel(const uint8_t *rows, int64_t m, const uint8_t *co
 
 // The same launch with strips in packed 16-bit lanes (strip16.cuh): 2 RH rows per
 // lane, strips of 64 RH rows.  Table or compare scores by the bytes that occur.
-template <int RH, bool STORES>
+template <int RH, int KIND>
 __global__ void __launch_bounds__(kWarps * 32, 4) stage1_packed_kernel(Stage1Args a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) stage1_packed_kernel(Stage1Arg
             asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
             a.trace[3 * s + 2] = (int64_t)smid;
         }
-        rc = tab ? run_strip2<RH, true, STORES>(a, w, lane, (int32_t)s) : run_strip2<RH, false, STORES>(a, w, lane, (int32_t)s);
+        rc = tab ? run_strip2<RH, true, KIND>(a, w, lane, (int32_t)s) : run_strip2<RH, false, KIND>(a, w, lane, (int32_t)s);
         if (a.trace && lane == 0) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -196,6 +196,44 @@ __global__ void __launch_bounds__(kWarps * 32, 4) stage1_packed_kernel(Stage1Arg
     }
 }
 
+// Merges sh[0 .. blockDim.x) into sh[0].
+__device__ __forceinline__ void reduce_block(BestRec *sh) {
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w) {
+            const BestRec r = sh[threadIdx.x + w];
+            BestRec &m = sh[threadIdx.x];
+            if (r.valid && (!m.valid || better(r.ho, r.key, m.ho, m.key))) m = r;
+        }
+        __syncthreads();
+    }
+}
+
+// Before a block with a top border: the cells of its first row that take H from the
+// border through F.  They are cells of the block like any other, though no maximum over
+// t = max(diagonal, E, 0) holds them (inside a matrix such a cell is below the one
+// above it).  Their H is at least F of row 0, known with the border; where it is
+// higher the strips find that.  One record per thread block, and the best H known.
+// (Taken by strip 0 with its entries instead, the 131 kbp block took 2% longer.)
+__global__ void border_best_kernel(Stage1Args a, BestRec *out) {
+    __shared__ BestRec sh[256];
+    BestRec b{a.open, 0, ~0ULL, 0, 0};
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += stride) {
+        const int2 t = a.top[c];
+        const int32_t ho = max(t.y + a.ext, t.x + a.open) + a.open;
+        if (ho <= a.open || ho < b.ho) continue;
+        const uint64_t key = tie_key(a.tie, a.r_origin, a.c_origin + c);
+        if (better(ho, key, b.ho, b.key)) b = BestRec{ho, 1, key, 0, c};
+    }
+    sh[threadIdx.x] = b;
+    reduce_block(sh);
+    if (threadIdx.x == 0) {
+        out[blockIdx.x] = sh[0];
+        if (sh[0].valid) atomicMax(a.gbest, sh[0].ho - a.open);
+    }
+}
+
 __global__ void reduce_best_kernel(const BestRec *in, int64_t count, BestRec *out) {
     __shared__ BestRec sh[256];
     BestRec b;
@@ -209,15 +247,7 @@ __global__ void reduce_best_kernel(const BestRec *in, int64_t count, BestRec *ou
         if (r.valid && (!b.valid || better(r.ho, r.key, b.ho, b.key))) b = r;
     }
     sh[threadIdx.x] = b;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            const BestRec r = sh[threadIdx.x + w];
-            BestRec &m = sh[threadIdx.x];
-            if (r.valid && (!m.valid || better(r.ho, r.key, m.ho, m.key))) m = r;
-        }
-        __syncthreads();
-    }
+    reduce_block(sh);
     if (threadIdx.x == 0) *out = sh[0];
 }
 
@@ -255,23 +285,29 @@ template <int R, bool TAB, bool STORES>
 KernelRef wide_ref() {
     return {(const void *)stage1_kernel<R, TAB, STORES>, 0};
 }
-template <int R, bool STORES>
-KernelRef packed_ref() {
-    return {(const void *)stage1_packed_kernel<R / 2, STORES>, kWarps * sizeof(WarpMem<R / 2>)};
-}
-template <bool TAB, bool STORES>
-KernelRef kernel_ref(int R, bool packed) {
-    switch (R) {
-        case 8: return packed ? packed_ref<8, STORES>() : wide_ref<8, TAB, STORES>();
-        case 14: return packed ? packed_ref<14, STORES>() : wide_ref<14, TAB, STORES>();
-        case 16: return packed ? packed_ref<16, STORES>() : wide_ref<16, TAB, STORES>();
-        case 32: return packed ? packed_ref<32, STORES>() : wide_ref<32, TAB, STORES>();
-        default: return {};
+template <int R>
+KernelRef packed_ref(int kind) {
+    constexpr size_t smem = kWarps * sizeof(WarpMem<R / 2>);
+    switch (kind) {
+        case kScore: return {(const void *)stage1_packed_kernel<R / 2, kScore>, smem};
+        case kStores: return {(const void *)stage1_packed_kernel<R / 2, kStores>, smem};
+        default: return {(const void *)stage1_packed_kernel<R / 2, kBorders>, smem};
     }
 }
-KernelRef kernel_of(int R, bool tab, bool stores, bool packed) {
-    if (tab) return stores ? kernel_ref<true, true>(R, packed) : kernel_ref<true, false>(R, packed);
-    return stores ? kernel_ref<false, true>(R, packed) : kernel_ref<false, false>(R, packed);
+// (the 32-bit kernels without stores serve borders too)
+template <int R>
+KernelRef wide_ref(bool tab, int kind) {
+    if (tab) return kind == kStores ? wide_ref<R, true, true>() : wide_ref<R, true, false>();
+    return kind == kStores ? wide_ref<R, false, true>() : wide_ref<R, false, false>();
+}
+KernelRef kernel_of(int R, bool tab, int kind, bool packed) {
+    switch (R) {
+        case 8: return packed ? packed_ref<8>(kind) : wide_ref<8>(tab, kind);
+        case 14: return packed ? packed_ref<14>(kind) : wide_ref<14>(tab, kind);
+        case 16: return packed ? packed_ref<16>(kind) : wide_ref<16>(tab, kind);
+        case 32: return packed ? packed_ref<32>(kind) : wide_ref<32>(tab, kind);
+        default: return {};
+    }
 }
 
 }  // namespace
@@ -286,14 +322,15 @@ cudaError_t stage1_configure() {
     const auto A = cudaFuncAttributePreferredSharedMemoryCarveout;
     cudaError_t e = cudaSuccess;
     for (int R : {8, 14, 16, 32})
-        for (int v = 0; v < 8; ++v) {
-            const KernelRef k = kernel_of(R, v & 1, v & 2, v & 4);
+        for (int v = 0; v < 12; ++v) {
+            const KernelRef k = kernel_of(R, v & 1, v >> 2, v & 2);
             cudaError_t x = cudaFuncSetAttribute(k.fn, A, c);
             if (x == cudaSuccess && k.smem > 0)
                 x = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
             if (x != cudaSuccess) e = x;
         }
     for (cudaError_t x : {cudaFuncSetAttribute((const void *)reduce_best_kernel, A, c),
+                          cudaFuncSetAttribute((const void *)border_best_kernel, A, c),
                           cudaFuncSetAttribute((const void *)encode_kernel, A, c),
                           cudaFuncSetAttribute((const void *)prepare_kernel, A, c),
                           cudaFuncSetAttribute((const void *)presence_kernel, A, c)})
@@ -303,8 +340,8 @@ cudaError_t stage1_configure() {
 
 int stage1_max_blocks_per_sm(int R, bool tab, bool packed) {
     int least = INT_MAX;
-    for (bool stores : {false, true}) {
-        const KernelRef k = kernel_of(R, tab, stores, packed);
+    for (int kind : {kScore, kStores, kBorders}) {
+        const KernelRef k = kernel_of(R, tab, kind, packed);
         int nb = 0;
         if (!k.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn, kWarps * 32, k.smem) != cudaSuccess)
             return 0;
@@ -347,12 +384,18 @@ Stage1Plan stage1_plan(int64_t m, int64_t n, int device_sms, int R_hint, bool ta
 }
 
 cudaError_t stage1_launch(Stage1Args &a, const Stage1Plan &p, cudaStream_t st) {
-    const KernelRef k = kernel_of(p.R, p.tab, p.stores || a.srows || a.scols || (p.packed && stage1_has_borders(a)), p.packed);
+    const int kind = stage1_has_borders(a) ? kBorders : (p.stores || a.srows || a.scols ? kStores : kScore);
+    const KernelRef k = kernel_of(p.R, p.tab, kind, p.packed);
     if (!k.fn) return cudaErrorInvalidValue;
+    int extra = 0;
+    if (a.top) {
+        extra = (int)std::min<int64_t>(kStage1BorderRecs, (a.n + 255) / 256);
+        border_best_kernel<<<extra, 256, 0, st>>>(a, a.wbest + (int64_t)p.blocks * kWarps);
+    }
     void *args[] = {&a};
     const cudaError_t e = cudaLaunchCooperativeKernel(k.fn, dim3(p.blocks), dim3(kWarps * 32), args, k.smem, st);
     if (e != cudaSuccess) return e;
-    reduce_best_kernel<<<1, 256, 0, st>>>(a.wbest, (int64_t)p.blocks * kWarps, a.best);
+    reduce_best_kernel<<<1, 256, 0, st>>>(a.wbest, (int64_t)p.blocks * kWarps + extra, a.best);
     return cudaGetLastError();
 }
 

@@ -289,20 +289,6 @@ __device__ __forceinline__ void prefetch(const A &a, int32_t strip, int32_t c, P
     }
 }
 
-// A block's top border comes into its first row's F, and a cell that takes H from
-// there is a cell of the block like any other, though no maximum over t holds it (see
-// step).  Its H is F of row 0, known with the border: a candidate if it reaches the
-// lane's threshold (where the cell's H is higher still, the step finds that).
-template <class A>
-__device__ __forceinline__ void border_candidate(const A &a, Best *b, int32_t &bho, int32_t &thr, int32_t strip, int32_t c,
-                                                 const Pre &p) {
-    if (strip != 0 || a.top == nullptr) return;
-    const int32_t ho = p.h.z + a.open;
-    if (ho < max(thr, bho)) return;
-    bho = slow_best(1u, ho, a.tie, a.m, a.r_origin, a.c_origin, b, 0, c, a.gbest, a.open);
-    thr = max(thr, bho);
-}
-
 // Stores the prefetched entry of column c into the ring (re-polling until the
 // strip above has written it).  Returns false on timeout/abort.
 template <class A>
@@ -343,7 +329,7 @@ __device__ __forceinline__ void flush(const A &a, const int4 *stage, int lane, c
 
 template <bool TAB, class A>
 __device__ __forceinline__ bool refill(const A &a, int4 *ring, const int4 *stage, int lane, const StripCtx &sc,
-                                       int32_t n, int32_t k, Pre &pre, int32_t &thr, Best *b, int32_t &bho, int32_t &gpre) {
+                                       int32_t n, int32_t k, Pre &pre, int32_t &thr, int32_t bho, int32_t &gpre) {
     const int32_t strip = sc.strip;
     flush(a, stage, lane, sc, n, k);
     // cells below the best H found anywhere so far can never win: raise the
@@ -354,10 +340,7 @@ __device__ __forceinline__ bool refill(const A &a, int4 *ring, const int4 *stage
     bool ok = true;
     if (lane < kCH) {
         const int32_t c = k + kCH + lane;
-        if (c < n) {
-            ok = commit(a, ring, strip, c, pre);
-            border_candidate(a, b, bho, thr, strip, c, pre);
-        }
+        if (c < n) ok = commit(a, ring, strip, c, pre);
         const int32_t cn = c + kCH;
         if (cn < n) prefetch<TAB>(a, strip, cn, pre);
     }
@@ -419,7 +402,6 @@ __device__ bool run_strip(const A &a, int4 *ring, int4 *stage, int lane, int32_t
             if (c < n) {
                 prefetch<TAB>(a, s, c, pre);
                 ok = commit(a, ring, s, c, pre);
-                border_candidate(a, b, L.bho, L.thr, s, c, pre);
             }
         }
         if (2 * kCH + lane < n) prefetch<TAB>(a, s, 2 * kCH + lane, pre);
@@ -448,13 +430,13 @@ __device__ bool run_strip(const A &a, int4 *ring, int4 *stage, int lane, int32_t
     if (n > 32) kB = 32 + ((n - 32) / kCH) * kCH;
     int32_t k = 0;
     for (; k < kA; ++k) {
-        if (k > 0 && (k % kCH) == 0 && !refill<TAB>(a, ring, stage, lane, sc, n, k, pre, L.thr, b, L.bho, gpre)) return false;
+        if (k > 0 && (k % kCH) == 0 && !refill<TAB>(a, ring, stage, lane, sc, n, k, pre, L.thr, L.bho, gpre)) return false;
         if constexpr (!STORES) step<R, TAB, true, false>(L, a, b, ring, stage, lane, sc, k);
         else if (a.scols) step<R, TAB, true, true>(L, a, b, ring, stage, lane, sc, k);
         else step<R, TAB, true, false>(L, a, b, ring, stage, lane, sc, k);
     }
     while (k < kB) {
-        if (!refill<TAB>(a, ring, stage, lane, sc, n, k, pre, L.thr, b, L.bho, gpre)) return false;
+        if (!refill<TAB>(a, ring, stage, lane, sc, n, k, pre, L.thr, L.bho, gpre)) return false;
         // lane l stores special column j = q*sc_every - 1 at step j + l: a chunk of
         // steps [k, k+kCH) needs the check when some (t + 1) mod sc_every < 32
         const bool sc_window = a.scols != nullptr && ((k + kCH) & (a.sc_every - 1)) < 32 + kCH;
@@ -479,7 +461,7 @@ __device__ bool run_strip(const A &a, int4 *ring, int4 *stage, int lane, int32_t
         k += kCH;
     }
     for (; k < kEnd; ++k) {
-        if ((k % kCH) == 0 && !refill<TAB>(a, ring, stage, lane, sc, n, k, pre, L.thr, b, L.bho, gpre)) return false;
+        if ((k % kCH) == 0 && !refill<TAB>(a, ring, stage, lane, sc, n, k, pre, L.thr, L.bho, gpre)) return false;
         if constexpr (!STORES) step<R, TAB, true, false>(L, a, b, ring, stage, lane, sc, k);
         else if (a.scols) step<R, TAB, true, true>(L, a, b, ring, stage, lane, sc, k);
         else step<R, TAB, true, false>(L, a, b, ring, stage, lane, sc, k);

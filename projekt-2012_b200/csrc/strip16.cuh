@@ -365,37 +365,6 @@ __device__ __forceinline__ void rerun(const A &a, WarpMem<RH> *w, Lane2<RH> &L, 
     __syncwarp();
 }
 
-// The cells of a block's first row that take H from the top border through F: cells of
-// the block like any other, though no maximum over t holds them.  Their H is F of row
-// 0, known with the border.  Takes the best of the lanes' cells (ho: H + open of (0, col),
-// where the cell's H is higher the steps find that) into the warp's best and returns
-// the threshold after it.
-template <int RH, class A>
-__device__ __forceinline__ int32_t take_border(const A &a, WarpMem<RH> *w, int lane, int32_t ho, int32_t col, int32_t thr) {
-    const int32_t best = __reduce_max_sync(0xffffffffu, ho);
-    if (best < thr) return thr;
-    uint64_t key = ho == best ? tie_key(a.tie, a.r_origin, a.c_origin + col) : ~0ULL;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const uint64_t okey = __shfl_xor_sync(0xffffffffu, key, off);
-        const int32_t ocol = __shfl_xor_sync(0xffffffffu, col, off);
-        if (okey < key) {
-            key = okey;
-            col = ocol;
-        }
-    }
-    if (lane == 0 && (best > w->best_ho || (best == w->best_ho && key < w->best_key))) {
-        if (best > thr) atomicMax(a.gbest, best - a.open);
-        w->best_ho = best;
-        w->best_valid = 1;
-        w->best_key = key;
-        w->best_row = 0;
-        w->best_col = col;
-    }
-    __syncwarp();
-    return best;
-}
-
 // Where a strip's last rows go besides the strip below.
 struct Out2 {
     int2 *row[2];  // per half: special row or the rectangle's last row (column 0), or null
@@ -415,10 +384,10 @@ __device__ __forceinline__ void flush2(const WarpMem<RH> *w, int lane, const Out
 
 // The row above the strip at column c as a hand-off entry: the strip above's, a
 // given top boundary or the matrix edge (relative to H + open of that cell).
-template <class A>
+template <bool BORDERS, class A>
 __device__ __forceinline__ int4 above2(const A &a, int32_t strip, int32_t c) {
     if (strip > 0) return ld_ll(a.hbuf + c);
-    if (a.top) {
+    if (BORDERS && a.top) {
         const int2 t = a.top[c];
         const int32_t d = max(t.y + a.ext - t.x - a.open, 0);  // F of row 0 above H + open
         return make_int4((int32_t)((uint32_t)min(d, 32767) << 16), 0, t.x + a.open, 0);
@@ -529,12 +498,21 @@ __device__ __forceinline__ void steps2(Lane2<RH> &L, const uint32_t *ra, const C
     }
 }
 
-// Runs strip s.  (Kernels without STORES serve no launch with a given boundary or a
-// right border.)  w->best_* holds the warp's best cell (kept over strips by the
-// caller).  STORES: the launch keeps special rows or columns or a block's borders.
+// What a launch may keep or be given besides the best cell: nothing; special rows and
+// columns; a block's boundaries and wanted borders.  Each has its own kernels: what
+// they run between the runs of steps is bound by instruction fetch (172 kbp pair 20.5
+// ms with the borders' code in the pairs' kernels, 19.8 without).
+enum : int { kScore = 0, kStores = 1, kBorders = 2 };
+
+// Runs strip s.  w->best_* holds the warp's best cell (kept over strips by the
+// caller).
 // Returns kErrNone, kErrTimeout or kErrRange.
-template <int RH, bool TAB, bool STORES, class A>
+template <int RH, bool TAB, int KIND, class A>
 __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
+    constexpr bool STORES = KIND != kScore, BORDERS = KIND >= kBorders;
+    // (the score-only kernels have no left boundary either; without its code the
+    // compiler's schedule of their steps is worse: score only, 61 kbp 3.79 -> 3.89 ms)
+    constexpr bool LEFT = BORDERS || KIND == kScore;
     Lane2<RH> L;
     uint32_t ra[RH];
     constexpr int64_t HR = 32 * RH;  // rows of a half
@@ -550,13 +528,13 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         for (int h = 0; h < 2; ++h) {
             const int64_t q = 2 * (int64_t)s + h + 1;  // half strips above and including this one
             if (a.srows != nullptr && q % a.sr_every == 0 && q * HR <= a.m) o.row[h] = a.srows + (q / a.sr_every - 1) * a.n;
-            if (a.bottom != nullptr && q * HR == a.m) o.row[h] = a.bottom;
+            if (BORDERS && a.bottom != nullptr && q * HR == a.m) o.row[h] = a.bottom;
         }
     }
 
     // left boundary: the base first, then offsets
     int32_t base = 0;
-    if (a.left) {
+    if (LEFT && a.left) {
         int32_t lo = INT_MAX, hi = INT_MIN;
         for (int64_t i = lane; i < 2 * HR && row0 + i < a.m; i += 32) {
             const int2 lv = a.left[row0 + i];
@@ -575,7 +553,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         for (int h = 0; h < 2; ++h) {
             ho[h] = (uint32_t)a.open;  // H = 0 and E = 0 left of column 0
             ee[h] = 0u;
-            if (a.left) {
+            if (LEFT && a.left) {
                 // rows past the end repeat the last row's boundary
                 const int64_t r = r_lane + h * HR + i;
                 const int2 lv = a.left[r < a.m ? r : a.m - 1];
@@ -588,8 +566,8 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         L.E[i] = (ee[0] & 0xFFFFu) | (ee[1] << 16);
     }
     int32_t corner = a.open;  // H + open above row 0 left of column 0
-    if (s == 0) corner = a.corner + a.open - base;
-    else if (a.left) corner = a.left[row0 - 1].x + a.open - base;
+    if (BORDERS && s == 0) corner = a.corner + a.open - base;
+    else if (BORDERS && a.left) corner = a.left[row0 - 1].x + a.open - base;
     if (corner > 32767 - win.near || corner < (base > 0 ? win.near : -32768)) return kErrRange;
     Turn t;
     t.selH = lane == 31 ? 0x5410u : 0x7654u;
@@ -605,7 +583,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     int32_t wlo = base > 0 ? win.lo : -32768, wnear = base > 0 ? win.near : -32768;  // the window's lower ends
     {
         bool ok = true, range = true;
-        if (lane == 0) ok = commit2(a, w->ring, s, 0, above2(a, s, 0), base, wnear, win.near, range);
+        if (lane == 0) ok = commit2(a, w->ring, s, 0, above2<BORDERS>(a, s, 0), base, wnear, win.near, range);
         if (!__all_sync(0xffffffffu, ok && range)) return __all_sync(0xffffffffu, ok) ? kErrRange : kErrTimeout;
     }
     __syncwarp();
@@ -620,7 +598,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     }
     __syncwarp();
     int4 up4 = make_int4(0, 0, 0, 0);
-    if (1 + lane < n) up4 = above2(a, s, 1 + lane);
+    if (1 + lane < n) up4 = above2<BORDERS>(a, s, 1 + lane);
     // Columns outside the matrix mismatch every row.  Left of it (no left boundary
     // given) H then stays 0 and the steps need no predicate; E is open there where
     // the recurrence starts from 0, which is gone after |open| / |extend| columns and
@@ -628,7 +606,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     // stay below a cell's value that was seen before, and the exact rerun, the
     // stored rows and the special columns leave them out.  A given left boundary or
     // a wanted right border needs the predicates.
-    const bool exact = a.left != nullptr || a.right != nullptr;
+    const bool exact = BORDERS && (a.left != nullptr || a.right != nullptr);
     const uint32_t none = no_column<TAB>(a.mm1);
     put_col(w->col, lane, col_value<TAB>(lane < n ? read_col<TAB>(a.ctab, a.cols, lane) : none));
     put_col(w->col, lane - 32, col_value<TAB>(none));
@@ -643,8 +621,6 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     // the best H known anywhere, loaded a run before it is used
     int32_t gpre = ld_volatile(a.gbest);
     int32_t thr = max(w->best_ho, gpre + a.open);
-    const bool first_row = STORES && s == 0 && a.top != nullptr;  // cells take H from a given border through F
-    if (first_row) thr = take_border(a, w, lane, lane == 0 ? half16(L.inF, 0) + base + a.open : INT_MIN, 0, thr);
     // kept runs: slots first, first + 1, ... (cyclic), all with maximum kv
     int first = 0, kept = 0;
     int32_t kv = 0;
@@ -654,7 +630,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         if (end || kept == kKept<RH>) {
             // the kept runs again, unless a better cell was found elsewhere; in the
             // middle of the strip the lanes' rows wait in shared memory
-            if constexpr (STORES) {
+            if constexpr (BORDERS) {
                 if (end && a.right != nullptr) {
                     // after its last column a half's registers hold H + open and E of column n - 1
 #pragma unroll
@@ -702,7 +678,6 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         const int32_t q = k + 1 + lane, qc = k + kRun + lane;
         const int32_t ub = up4.z - base, uho = half16((uint32_t)up4.x, 0) + ub, uf = half16((uint32_t)up4.x, 1) + ub;
         thr = max(thr, gpre + a.open);
-        if (first_row) thr = take_border(a, w, lane, q < n ? half16((uint32_t)up4.x, 1) + up4.z + a.open : INT_MIN, q, thr);
         const bool track = __any_sync(0xffffffffu, vmax + win.reach >= thr - base);  // some cell of this run may reach the best known
         const bool mine = vmax <= win.hi && vmin >= wlo;
         const bool entry = q >= n || (max(uho, uf) <= 32767 - win.near && min(uho, uf) >= wnear &&
@@ -739,8 +714,8 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         put_col(w->col, qc, col_value<TAB>(cv));
         if (s > 0) {
             ld_hand(up4, q + kRun < n, a.hbuf + (q + kRun));
-        } else if (a.top && q + kRun < n) {
-            up4 = above2(a, s, q + kRun);
+        } else if (BORDERS && a.top && q + kRun < n) {
+            up4 = above2<BORDERS>(a, s, q + kRun);
         }
         cv = none;
         ld_col<TAB>(cv, qc + kRun < n, a.ctab, a.cols, qc + kRun);
@@ -775,7 +750,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
             else if (STORES && mode == kPlain)
                 steps2<Sub<RH>::edge, RH, TAB, true, kPlain, STORES, STORES>(L, ra, c, pa, pb, w->ring, hb, w->stage, w->spec, lane,
                                                                       t, spec, k, n, mx);
-            else if (!STORES || mode == kEdge)
+            else if (!BORDERS || mode == kEdge)
                 steps2<Sub<RH>::edge, RH, TAB, true, kEdge, STORES, STORES>(L, ra, c, pa, pb, w->ring, hb, w->stage, w->spec, lane,
                                                                        t, spec, k, n, mx);
             else

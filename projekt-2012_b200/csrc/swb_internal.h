@@ -26,6 +26,9 @@ struct BestRec {
     int64_t col;
 };
 
+// Best cells found in a block's top border before the launch (one per thread block).
+constexpr int kStage1BorderRecs = 256;
+
 enum TieMode : int32_t { kTieReference = 0, kTieRowMajor = 1 };
 
 struct TieGeom {
@@ -58,7 +61,7 @@ struct Stage1Args {
     int32_t corner;        // H above-left of the rectangle
     int64_t r_origin, c_origin;  // rectangle origin in the whole matrix (tie key)
     int64_t nstrips;
-    BestRec *wbest;        // one per warp of the grid
+    BestRec *wbest;        // one per warp of the grid, and kStage1BorderRecs more with a top border
     BestRec *best;         // final reduced record
     int32_t *err;          // [0] error code, [1] abort flag, [2] best H seen so far (device-wide)
     int32_t *gbest;        // best H seen so far in this matrix (err + 2 for a single pair)
@@ -70,8 +73,8 @@ struct Stage1Args {
     int2 *right;           // optional: (H, E) of the last column, m entries
 };
 
-// A launch over a block with given boundaries or wanted borders (packed strips run
-// it with the kernels that have stores).
+// A launch over a block with given boundaries or wanted borders (it keeps no special
+// rows or columns).
 inline bool stage1_has_borders(const Stage1Args &a) { return a.top || a.left || a.bottom || a.right; }
 
 // Geometry of the reference's launch (src/SWutils.cpp:233-253) and padding
