@@ -604,9 +604,10 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
     // the recurrence starts from 0, which is gone after |open| / |extend| columns and
     // never positive.  Right of it the values belong to no cell and reach none: they
     // stay below a cell's value that was seen before, and the exact rerun, the
-    // stored rows and the special columns leave them out.  A given left boundary or
-    // a wanted right border needs the predicates.
-    const bool exact = BORDERS && (a.left != nullptr || a.right != nullptr);
+    // stored rows and the special columns leave them out.  A given boundary (they
+    // would go on from it, and it is no cell) or a wanted right border needs the
+    // predicates.
+    const bool exact = BORDERS && (a.top != nullptr || a.left != nullptr || a.right != nullptr);
     const uint32_t none = no_column<TAB>(a.mm1);
     put_col(w->col, lane, col_value<TAB>(lane < n ? read_col<TAB>(a.ctab, a.cols, lane) : none));
     put_col(w->col, lane - 32, col_value<TAB>(none));

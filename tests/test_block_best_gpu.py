@@ -47,3 +47,22 @@ def test_cells_that_take_h_from_the_top_border_count(gpu_ctx, m, n):
         for tie in (O.TIE_REFERENCE, O.TIE_ROWMAJOR):
             got, want = _best(gpu_ctx, b"A" * m, _seq(rng, n, alph), (1, -3, -2, -2), top, None, 0, 512, 0, 4096, 1024, tie)
             assert want[:3] == (298, 512, n // 2) and got == want
+
+
+@pytest.mark.parametrize("alph", [b"ACGT", b"ACGTRYKM"])
+@pytest.mark.parametrize("last", [1, 24, 257, 512, 700])
+def test_columns_right_of_the_block_do_not_count(gpu_ctx, alph, last):
+    """The last rows of a matrix whose alignment ends in the row above the block, at
+    the last column: the border is higher than every cell of the block, and a column
+    past the last one would continue from it."""
+    rng = random.Random(last + len(alph))
+    n, above = 700, 1536
+    cols = _seq(rng, n, alph)
+    rows = _seq(rng, above - 500, alph) + cols[-500:] + _seq(rng, last, alph)
+    m, sc = len(rows), (1, -3, -5, -2)
+    for tie in (O.TIE_REFERENCE, O.TIE_ROWMAJOR):
+        top = O.block(rows[:above], cols, O.scoring(*sc), None, None, 0, 0, 0, m, n, tie)[0]
+        high = int(top[-1, 0])
+        assert high >= 500
+        got, want = _best(gpu_ctx, rows[above:], cols, sc, top, None, 0, above, 0, m, n, tie)
+        assert want[0] == high - 5 and got == want
