@@ -180,6 +180,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs &g) {
 template <int RH, class S>
 __device__ __forceinline__ void packed_body(const BatchArgs &g, bool tab) {
     extern __shared__ __align__(16) unsigned char smem[];
+    // (nothing reads the best cells of a launch with boundaries: kBorders serves every height)
     constexpr int KIND = std::is_same<S, NoStores>::value ? kScore : (std::is_same<S, WithBounds>::value ? kBorders : kStores);
     const int lane = threadIdx.x & 31;
     WarpMem<RH> *w = reinterpret_cast<WarpMem<RH> *>(smem) + (threadIdx.x >> 5);

@@ -291,7 +291,8 @@ KernelRef packed_ref(int kind) {
     switch (kind) {
         case kScore: return {(const void *)stage1_packed_kernel<R / 2, kScore>, smem};
         case kStores: return {(const void *)stage1_packed_kernel<R / 2, kStores>, smem};
-        default: return {(const void *)stage1_packed_kernel<R / 2, kBorders>, smem};
+        case kBorders: return {(const void *)stage1_packed_kernel<R / 2, kBorders>, smem};
+        default: return {(const void *)stage1_packed_kernel<R / 2, kRagged>, smem};
     }
 }
 // (the 32-bit kernels without stores serve borders too)
@@ -322,7 +323,7 @@ cudaError_t stage1_configure() {
     const auto A = cudaFuncAttributePreferredSharedMemoryCarveout;
     cudaError_t e = cudaSuccess;
     for (int R : {8, 14, 16, 32})
-        for (int v = 0; v < 12; ++v) {
+        for (int v = 0; v < 16; ++v) {
             const KernelRef k = kernel_of(R, v & 1, v >> 2, v & 2);
             cudaError_t x = cudaFuncSetAttribute(k.fn, A, c);
             if (x == cudaSuccess && k.smem > 0)
@@ -340,7 +341,7 @@ cudaError_t stage1_configure() {
 
 int stage1_max_blocks_per_sm(int R, bool tab, bool packed) {
     int least = INT_MAX;
-    for (int kind : {kScore, kStores, kBorders}) {
+    for (int kind : {kScore, kStores, kBorders, kRagged}) {
         const KernelRef k = kernel_of(R, tab, kind, packed);
         int nb = 0;
         if (!k.fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k.fn, kWarps * 32, k.smem) != cudaSuccess)
@@ -384,7 +385,8 @@ Stage1Plan stage1_plan(int64_t m, int64_t n, int device_sms, int R_hint, bool ta
 }
 
 cudaError_t stage1_launch(Stage1Args &a, const Stage1Plan &p, cudaStream_t st) {
-    const int kind = stage1_has_borders(a) ? kBorders : (p.stores || a.srows || a.scols ? kStores : kScore);
+    const int kind = stage1_has_borders(a) ? (a.left && a.m % p.strip_rows != 0 ? kRagged : kBorders)
+                                           : (p.stores || a.srows || a.scols ? kStores : kScore);
     const KernelRef k = kernel_of(p.R, p.tab, kind, p.packed);
     if (!k.fn) return cudaErrorInvalidValue;
     int extra = 0;

@@ -235,7 +235,19 @@ __device__ __forceinline__ void step(Lane<R> &L, const A &a, Best *b, const int4
         uint32_t mask = 0;
 #pragma unroll
         for (int i = 0; i < R; ++i) mask |= (L.HO[i] == cm ? 1u : 0u) << i;
-        L.bho = slow_best(mask, cm, a.tie, a.m, a.r_origin, a.c_origin, b, sc.row0, j, a.gbest, a.open);
+        if (a.left != nullptr && sc.row0 + __ffs(mask) > a.m) {
+            // only rows past the end hold it, which go on from the left border: the
+            // maximum of the rectangle's rows
+            cm = L.thr - 1;
+            mask = 0;
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                if (sc.row0 + i < a.m && L.HO[i] >= cm) {
+                    mask = (L.HO[i] > cm ? 0u : mask) | (1u << i);
+                    cm = L.HO[i];
+                }
+        }
+        if (cm >= L.thr) L.bho = slow_best(mask, cm, a.tie, a.m, a.r_origin, a.c_origin, b, sc.row0, j, a.gbest, a.open);
         L.thr = max(L.thr, L.bho);
     }
     if (SC && act && ((j + 1) & (a.sc_every - 1)) == 0) {

@@ -157,18 +157,19 @@ struct Turn {
 // column's row above; hb: hand-off entry of lane 31's column, st: its place in the
 // stage.  TRACK: fold t + open of every row into mx (packed maxima).  EDGE: lane
 // 31's column may be outside [0, n): `inside` says.  PRED: halves outside [0, n)
-// keep their values: mask has 0xFFFF in each half that is inside.
+// keep their values: mask has 0xFFFF in each half that is inside.  PRED with ROWS: mx
+// takes only the rectangle's rows: bits i and 16 + i of rows for row i of the halves.
 //
 // A warp issues in order, and alone on its scheduler it is bound by latencies.
 // Phase 1 (scores, E, t: 8 issue cycles a row) needs only the previous step's H
 // and E and covers the shuffle of H and F from the lane above; phase 2 is the F
 // chain, whose two ops a row issue in the 4 cycles that one of them takes.
-enum : int { kPlain = 0, kEdge = 1, kPred = 2 };
+enum : int { kPlain = 0, kEdge = 1, kPred = 2, kPredRows = 3 };
 template <int RH, bool TAB, bool TRACK, int MODE, bool STORES, bool SC>
 __device__ __forceinline__ void step2(Lane2<RH> &L, const uint32_t *ra, const Consts2 &c, uint32_t ca, uint32_t cb,
                                       uint32_t rv, int4 *hb, int2 *st, uint4 (*sp)[32], int v, int lane, const Turn &t,
-                                      bool inside, uint32_t mask, uint32_t &mx) {
-    constexpr bool PRED = MODE == kPred;
+                                      bool inside, uint32_t mask, uint32_t rows, uint32_t &mx) {
+    constexpr bool PRED = MODE == kPred || MODE == kPredRows, ROWS = MODE == kPredRows;
     uint32_t to[RH];
     if (!TAB) ca = cb * 65536u + ca;
     uint32_t hod = L.hod;
@@ -182,9 +183,17 @@ __device__ __forceinline__ void step2(Lane2<RH> &L, const uint32_t *ra, const Co
     }
     if (TRACK) {
         uint32_t m = PRED ? 0x80008000u : mx;
+        if (ROWS) {
 #pragma unroll
-        for (int i = 0; i + 1 < RH; i += 2) m = __vimax3_s16x2(m, to[i], to[i + 1]);
-        if (RH & 1) m = __vmaxs2(m, to[RH - 1]);
+            for (int i = 0; i < RH; ++i) {
+                const uint32_t in = ((rows >> i) & 0x00010001u) * 0xFFFFu;
+                m = __vmaxs2(m, (to[i] & in) | (0x80008000u & ~in));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i + 1 < RH; i += 2) m = __vimax3_s16x2(m, to[i], to[i + 1]);
+            if (RH & 1) m = __vmaxs2(m, to[RH - 1]);
+        }
         mx = PRED ? __vmaxs2(mx, (m & mask) | (0x80008000u & ~mask)) : m;
     }
     uint32_t f = L.inF, flast = 0;
@@ -212,6 +221,14 @@ __device__ __forceinline__ void step2(Lane2<RH> &L, const uint32_t *ra, const Co
             sp[i / 2][lane] = make_uint4(L.HO[i], L.HO[i1], L.E[i], L.E[i1]);
         }
     }
+}
+
+// The rows of a lane (first rows r and r + 32 RH) above row m, as step2 takes them.
+template <int RH>
+__device__ __forceinline__ uint32_t rows_in(int64_t r, int64_t m) {
+    const int64_t l = m - r, h = l - 32 * RH;
+    const uint32_t nl = (uint32_t)max((int64_t)0, min(l, (int64_t)RH)), nh = (uint32_t)max((int64_t)0, min(h, (int64_t)RH));
+    return ((1u << nl) - 1u) | (((1u << nh) - 1u) << 16);
 }
 
 // 0xFFFF in each half whose column at step k lies in [0, n).
@@ -286,7 +303,7 @@ __device__ __forceinline__ uint32_t row2(const uint8_t *rcode, const uint8_t *ro
 
 // Does the kept run of slot q again (L is overwritten), finds the cells that hold
 // its maximum and merges the one with the smallest tie key into the warp's best.
-template <int RH, bool TAB, class A>
+template <int RH, bool TAB, bool RAGGED, class A>
 __device__ __forceinline__ void rerun(const A &a, WarpMem<RH> *w, Lane2<RH> &L, const uint32_t *ra, const Consts2 &c, int q,
                                       int lane, int64_t r_lane) {
     __syncwarp();
@@ -311,6 +328,7 @@ __device__ __forceinline__ void rerun(const A &a, WarpMem<RH> *w, Lane2<RH> &L, 
     }
     const int32_t k0 = w->kept_k[q], target = w->kept_val[q] - w->kept_base[q], n = (int32_t)a.n;
     const Turn t{lane == 31 ? 0x5410u : 0x7654u, lane == 31 ? 0x5432u : 0x7654u, false, false, 0, 0, 0};
+    const uint32_t rows = RAGGED ? rows_in<RH>(r_lane, a.m) : 0u;
     uint64_t bkey = ~0ULL;
     int64_t brow = 0, bcol = 0;
 #pragma unroll 1
@@ -319,18 +337,18 @@ __device__ __forceinline__ void rerun(const A &a, WarpMem<RH> *w, Lane2<RH> &L, 
         uint32_t mx = 0x80008000u;
         const uint32_t ca = (mask & 1u) ? col2<TAB>(a.ctab, a.cols, k0 + u - lane) : 0u;
         const uint32_t cb = (mask >> 16) ? col2<TAB>(a.ctab, a.cols, k0 + u - lane - 32) : 0u;
-        step2<RH, TAB, true, kPred, false, false>(L, ra, c, ca, cb, w->sring[q][u], nullptr, nullptr, nullptr, 0, lane, t,
-                                                  false, mask, mx);
+        step2<RH, TAB, true, RAGGED ? kPredRows : kPred, false, false>(L, ra, c, ca, cb, w->sring[q][u], nullptr, nullptr, nullptr, 0, lane, t,
+                                                  false, mask, rows, mx);
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
             if (half16(mx, h) != target || !((mask >> (16 * h)) & 1u)) continue;
             const int64_t r0 = r_lane + h * 32 * RH;
             const int64_t j = (int64_t)(k0 + u - lane - 32 * h);
-            uint32_t rows = 0;
+            uint32_t hold = 0;
 #pragma unroll
-            for (int i = 0; i < RH; ++i) rows |= (half16(L.HO[i], h) == target ? 1u : 0u) << i;
-            for (; rows; rows &= rows - 1) {
-                const int64_t r = r0 + __ffs(rows) - 1;
+            for (int i = 0; i < RH; ++i) hold |= (half16(L.HO[i], h) == target ? 1u : 0u) << i;
+            for (; hold; hold &= hold - 1) {
+                const int64_t r = r0 + __ffs(hold) - 1;
                 if (r >= a.m) break;
                 const uint64_t key = tie_key(a.tie, a.r_origin + r, a.c_origin + j);
                 if (key < bkey) {
@@ -430,6 +448,33 @@ __device__ __forceinline__ void put_col(uint32_t *col, int32_t c, uint32_t v) {
     if (q < kRun) col[kColRing + q] = v;
 }
 
+// A strip that reaches past the rectangle's last row, after every lane has passed column
+// 0 (step 64): its rows past the end, which went on from the left border (no cell of
+// the rectangle, so the predicated steps before kept them out of the maxima), start
+// again a gap below the lane's last row, or below a cell of the strip.  From here on
+// they come from cells alone, a mismatch or a gap below them, and the steps need not
+// tell them apart.
+template <int RH>
+__device__ __forceinline__ void drop_past_rows(Lane2<RH> &L, uint32_t rows, int64_t r_lane, int64_t m, uint32_t open2) {
+    int32_t low = INT_MAX;  // the lowest H + open of the halves' first rows
+    if (rows & 1u) low = half16(L.HO[0], 0);
+    if (rows & 0x10000u) low = min(low, half16(L.HO[0], 1));
+    const uint32_t low2 = dup16(__reduce_min_sync(0xffffffffu, low));
+    uint32_t past = low2;
+#pragma unroll
+    for (int i = 0; i < RH; ++i) {
+        const uint32_t in = ((rows >> i) & 0x00010001u) * 0xFFFFu;
+        L.E[i] = (L.E[i] & in) | (past & ~in);
+        L.HO[i] = (L.HO[i] & in) | (past & ~in);
+        past = (__vadd2(L.HO[i], open2) & in) | (past & ~in);
+    }
+    // the row above the half is past the end too
+    const uint32_t up = (r_lane <= m ? 0xFFFFu : 0u) | (r_lane + 32 * RH <= m ? 0xFFFF0000u : 0u);
+    L.inHO = (L.inHO & up) | (low2 & ~up);
+    L.inF = (L.inF & up) | (low2 & ~up);
+    L.hod = (L.hod & up) | (low2 & ~up);
+}
+
 // The window of the bottom rows' offsets: the margin covers the rows above them
 // and the columns until the next check (both neighbours' included).
 struct Window2 {
@@ -475,10 +520,11 @@ __device__ __forceinline__ void put_special(const A &a, const Lane2<RH> &L, cons
 
 // The kRun steps from step k in a loop of SUB unrolled ones; the next step's inputs
 // are loaded ahead.  spec: SC, the step after which my rows go to the special column.
+// rows: ROWS, see step2.
 template <int SUB, int RH, bool TAB, bool TRACK, int MODE, bool STORES, bool SC>
 __device__ __forceinline__ void steps2(Lane2<RH> &L, const uint32_t *ra, const Consts2 &c, const uint32_t *pa,
                                        const uint32_t *pb, const uint32_t *rg, int4 *hb, int2 *st, uint4 (*sp)[32],
-                                       int lane, Turn t, int spec, int32_t k, int32_t n, uint32_t &mx) {
+                                       int lane, Turn t, int spec, int32_t k, int32_t n, uint32_t rows, uint32_t &mx) {
     uint32_t ca = pa[0], cb = pb[0], rv = rg[0];
 #pragma unroll 1
     for (int v = 0; v < kRun; v += SUB) {
@@ -487,10 +533,10 @@ __device__ __forceinline__ void steps2(Lane2<RH> &L, const uint32_t *ra, const C
         for (int u = 0; u < SUB; ++u) {
             // the entry past the run's last is not used (it is inside the warp's memory)
             const uint32_t na = pa[v + u + 1], nb = pb[v + u + 1], nv = rg[v + u + 1];
-            const uint32_t mask = MODE == kPred ? active2(k + v + u, lane, n) : ~0u;
+            const uint32_t mask = MODE >= kPred ? active2(k + v + u, lane, n) : ~0u;
             const bool inside = MODE == kPlain || (uint32_t)(k + v + u - 63) < (uint32_t)n;
             step2<RH, TAB, TRACK, MODE, STORES, SC>(L, ra, c, ca, cb, rv, hb + v + u, st + v + u, sp, u, lane, t, inside,
-                                                    mask, mx);
+                                                    mask, rows, mx);
             ca = na;
             cb = nb;
             rv = nv;
@@ -499,17 +545,20 @@ __device__ __forceinline__ void steps2(Lane2<RH> &L, const uint32_t *ra, const C
 }
 
 // What a launch may keep or be given besides the best cell: nothing; special rows and
-// columns; a block's boundaries and wanted borders.  Each has its own kernels: what
-// they run between the runs of steps is bound by instruction fetch (172 kbp pair 20.5
-// ms with the borders' code in the pairs' kernels, 19.8 without).
-enum : int { kScore = 0, kStores = 1, kBorders = 2 };
+// columns; a block's boundaries and wanted borders; a block with a left boundary whose
+// last strip reaches past its last row.  Each has its own kernels: what they run
+// between the runs of steps is bound by instruction fetch, and compiled into the
+// pairs' kernels the blocks' code cost 2 to 6% (172 kbp pair 21.0 ms with all of it in,
+// 20.5 with what it had of it before, 19.8 with none; 131 kbp block 12.6 ms with the
+// last kind's code in, 12.3 without).
+enum : int { kScore = 0, kStores = 1, kBorders = 2, kRagged = 3 };
 
 // Runs strip s.  w->best_* holds the warp's best cell (kept over strips by the
 // caller).
 // Returns kErrNone, kErrTimeout or kErrRange.
 template <int RH, bool TAB, int KIND, class A>
 __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
-    constexpr bool STORES = KIND != kScore, BORDERS = KIND >= kBorders;
+    constexpr bool STORES = KIND != kScore, BORDERS = KIND >= kBorders, RAGGED = KIND == kRagged;
     // (the score-only kernels have no left boundary either; without its code the
     // compiler's schedule of their steps is worse: score only, 61 kbp 3.79 -> 3.89 ms)
     constexpr bool LEFT = BORDERS || KIND == kScore;
@@ -619,6 +668,9 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         a.trace[3 * s] = (int64_t)now;
     }
 
+    const bool past_end = RAGGED && row0 + 2 * HR > a.m;
+    const uint32_t rows_here = RAGGED ? rows_in<RH>(r_lane, a.m) : 0u;
+
     // the best H known anywhere, loaded a run before it is used
     int32_t gpre = ld_volatile(a.gbest);
     int32_t thr = max(w->best_ho, gpre + a.open);
@@ -654,7 +706,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
             if (kv >= __shfl_sync(0xffffffffu, ld_volatile(a.gbest), 0) + a.open) {
 #pragma unroll 1
                 for (int q = 0; q < kept; ++q)
-                    rerun<RH, TAB>(a, w, L, ra, c, first + q < kKept<RH> ? first + q : first + q - kKept<RH>, lane, r_lane);
+                    rerun<RH, TAB, RAGGED>(a, w, L, ra, c, first + q < kKept<RH> ? first + q : first + q - kKept<RH>, lane, r_lane);
             }
             kept = 0;
             if (end) break;
@@ -671,6 +723,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
             L.inF = inF;
             L.hod = hod;
         }
+        if (past_end && k == 64) drop_past_rows(L, rows_here, r_lane, a.m, c.open2);
         // refill: the next run's row above and the columns of the run after it in.  One
         // vote says whether every lane is inside its window and every entry is there
         // and close to the base; the lanes that would wait or move the base are rare.
@@ -736,7 +789,7 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         const int cur = first + kept < kKept<RH> ? first + kept : first + kept - kKept<RH>;
         if (!track && mode == kPlain && !sc_run) {
             steps2<Sub<RH>::plain, RH, TAB, false, kPlain, STORES, false>(L, ra, c, pa, pb, w->ring, hb, w->stage, w->spec, lane, t,
-                                                                 -1, k, n, mx);
+                                                                 -1, k, n, rows_here, mx);
         } else {
             if (sc_run && lane == 0) {
                 const int h = (k & (a.sc_every - 1)) == 0 ? 0 : 1;
@@ -747,16 +800,19 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
             const int spec = sc_run ? lane - 1 : -1;
             if (mode == kPlain && !sc_run)
                 steps2<Sub<RH>::plain, RH, TAB, true, kPlain, STORES, false>(L, ra, c, pa, pb, w->ring, hb, w->stage, w->spec, lane,
-                                                                    t, -1, k, n, mx);
+                                                                    t, -1, k, n, rows_here, mx);
             else if (STORES && mode == kPlain)
                 steps2<Sub<RH>::edge, RH, TAB, true, kPlain, STORES, STORES>(L, ra, c, pa, pb, w->ring, hb, w->stage, w->spec, lane,
-                                                                      t, spec, k, n, mx);
+                                                                      t, spec, k, n, rows_here, mx);
             else if (!BORDERS || mode == kEdge)
                 steps2<Sub<RH>::edge, RH, TAB, true, kEdge, STORES, STORES>(L, ra, c, pa, pb, w->ring, hb, w->stage, w->spec, lane,
-                                                                       t, spec, k, n, mx);
+                                                                       t, spec, k, n, rows_here, mx);
+            else if (RAGGED && past_end)
+                steps2<1, RH, TAB, true, kPredRows, STORES, STORES>(L, ra, c, pa, pb, w->ring, hb, w->stage, w->spec, lane,
+                                                                       t, spec, k, n, rows_here, mx);
             else
                 steps2<1, RH, TAB, true, kPred, STORES, STORES>(L, ra, c, pa, pb, w->ring, hb, w->stage, w->spec, lane,
-                                                                       t, spec, k, n, mx);
+                                                                       t, spec, k, n, rows_here, mx);
         }
         // the run's stored rows and special column out
         if constexpr (STORES) {

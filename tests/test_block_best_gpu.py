@@ -66,3 +66,19 @@ def test_columns_right_of_the_block_do_not_count(gpu_ctx, alph, last):
         assert high >= 500
         got, want = _best(gpu_ctx, rows[above:], cols, sc, top, None, 0, above, 0, m, n, tie)
         assert want[0] == high - 5 and got == want
+
+
+@pytest.mark.parametrize("alph", [b"ACGT", b"ACGTRYKM"])
+@pytest.mark.parametrize("m", [3, 63, 255, 505, 520, 1000])
+def test_rows_below_the_block_do_not_count(gpu_ctx, alph, m):
+    """A left border that is highest at the block's last row, with mismatches cheaper
+    than gaps: a row past the last one would continue from it along the diagonal."""
+    rng = random.Random(m + len(alph))
+    n = 600
+    left = np.zeros((m, 2), dtype=np.int32)
+    left[:, 0] = 40 + np.arange(m)
+    left[:, 1] = left[:, 0] - 5
+    for sc in ((1, -1, -5, -2), (2, -3, -9, -4)):
+        got, want = _best(gpu_ctx, b"A" * m, _seq(rng, n, alph[1:]), sc, None, left, 0, 0, 256, 4096, 1024,
+                          O.TIE_REFERENCE)
+        assert got == want, sc
