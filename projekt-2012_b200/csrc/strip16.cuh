@@ -36,7 +36,8 @@
 //
 // Best cell.  The step itself does not look for it.  Before each run of 32 steps
 // the warp asks whether any cell of the run could reach the best H known (bottom
-// rows + the bound above): if not, the steps run without a column maximum.  If
+// rows + the bound above, and the row above where a given border need not keep the
+// bound): if not, the steps run without a column maximum.  If
 // so, the state is kept in shared memory, the steps fold a running maximum, and
 // only when that reaches the best known does the warp remember the run (instead
 // of the ones remembered before, which it beats: along an alignment path that is
@@ -732,7 +733,15 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
         const int32_t q = k + 1 + lane, qc = k + kRun + lane;
         const int32_t ub = up4.z - base, uho = half16((uint32_t)up4.x, 0) + ub, uf = half16((uint32_t)up4.x, 1) + ub;
         thr = max(thr, gpre + a.open);
-        const bool track = __any_sync(0xffffffffu, vmax + win.reach >= thr - base);  // some cell of this run may reach the best known
+        bool near = vmax + win.reach >= thr - base;  // some cell of this run may reach the best known
+        if (BORDERS && a.top != nullptr) {
+            // a given top border may rise from column to column as no matrix does, and
+            // with it the strips' rows above: what they bring into this run counts too
+            // (the entries not there yet: below)
+            const int32_t up = max16(__vimax3_s16x2(L.inHO, L.hod, L.inF));
+            near |= max(up, q < n ? max(uho, uf) : up) + win.reach >= thr - base;
+        }
+        bool track = __any_sync(0xffffffffu, near);
         const bool mine = vmax <= win.hi && vmin >= wlo;
         const bool entry = q >= n || (max(uho, uf) <= 32767 - win.near && min(uho, uf) >= wnear &&
                                       (s == 0 || (up4.y == s - 1 && up4.w == s - 1)));
@@ -764,6 +773,9 @@ __device__ int32_t run_strip2(const A &a, WarpMem<RH> *w, int lane, int32_t s) {
             if (q < n) ok = commit2(a, w->ring + lane, s, q, up4, base, wnear, win.near, range);
             else w->ring[lane] = L.HO[RH - 1];
             if (!__all_sync(0xffffffffu, ok && range)) return __all_sync(0xffffffffu, ok) ? kErrRange : kErrTimeout;
+            if (BORDERS && a.top != nullptr) {
+                track |= __any_sync(0xffffffffu, max16(w->ring[lane]) + win.reach >= thr - base);
+            }
         }
         put_col(w->col, qc, col_value<TAB>(cv));
         if (s > 0) {

@@ -82,3 +82,24 @@ def test_rows_below_the_block_do_not_count(gpu_ctx, alph, m):
         got, want = _best(gpu_ctx, b"A" * m, _seq(rng, n, alph[1:]), sc, None, left, 0, 0, 256, 4096, 1024,
                           O.TIE_REFERENCE)
         assert got == want, sc
+
+
+@pytest.mark.parametrize("alph", [b"ACGT", b"ACGTRYKM"])
+@pytest.mark.parametrize("base", [0, 20_000])
+@pytest.mark.parametrize("high", [5_000, 9_000, 20])
+def test_a_top_border_that_jumps_up(gpu_ctx, alph, base, high):
+    """A top border with one high value, and a slightly higher one far behind it
+    followed by a match: no cell before it comes near the block's best."""
+    rng = random.Random(high + base)
+    m, n = 512, 700
+    rows, cols = bytearray(_seq(rng, m, alph)), bytearray(_seq(rng, n, alph))
+    cols[51] = ord("A") if rows[0] != ord("A") else ord("C")
+    cols[401] = rows[0]
+    top = np.zeros((n, 2), dtype=np.int32)
+    top[:, 0] = base
+    top[50, 0] = base + high
+    top[400, 0] = base + high + 200
+    top[:, 1] = np.maximum(top[:, 0] - 5, 0)
+    got, want = _best(gpu_ctx, bytes(rows), bytes(cols), (1, -3, -5, -2), top, None, 0, 512, 0, 4096, 1024,
+                      O.TIE_REFERENCE)
+    assert want[:3] == (base + high + 201, 512, 401) and got == want
