@@ -198,7 +198,7 @@ __device__ __forceinline__ void packed_body(const BatchArgs &g, bool tab) {
         // complete, so no wait spins)
         const int32_t first = g.unit_strip ? g.unit_strip[u] : u - d.unit0;
         const int32_t s0 = first == kWholePair ? 0 : first, s1 = first == kWholePair ? d.nstrips : first + 1;
-        int32_t rc = kErrNone;
+        int32_t rc = g.test_range != 0 && u == 0 ? kErrRange : kErrNone;
 #pragma unroll 1
         for (int32_t strip = s0; strip < s1 && rc == kErrNone; ++strip) {
             init_warp(w, lane, g.open);

@@ -57,6 +57,7 @@ struct BatchArgs {
     int32_t *ctl;              // [0] unit counter, [1] error code, [2] abort flag
     int2 *srows, *scols;       // store pass: special rows (H, F) / columns (H, E) of every pair
     int64_t wait_limit;        // bound of each wait for the strip above, in SM clock cycles; 0 = default
+    int32_t test_range;        // test hook (SWB_FLAG_TEST_PACK_ANY): packed strips' first unit reports kStage1Range
 };
 
 // Rows per lane of the large score-only pass's strips: 14 (448 rows) unless the

@@ -1107,7 +1107,10 @@ __global__ void __launch_bounds__(WIDE ? kThreadsWide : kThreads) walk_batch_ker
 }
 
 // Graphed batches: every pair's walk starts at the best cell the scoring kernel
-// merged into pbest (a pair without a positive score is marked done at once).
+// merged into pbest (a pair without a positive score is marked done at once).  After a
+// scoring kernel that gave up (an error code in the control words) neither the best
+// cells nor the stores are all written: every pair is marked done, so that nothing
+// walks, and the host reads the code.
 __global__ void walk_graph_init_kernel(const GraphHdr *h) {
     const int64_t np = h->npairs;
     WalkArgs *args = (WalkArgs *)h->walk_args;
@@ -1116,7 +1119,7 @@ __global__ void walk_graph_init_kernel(const GraphHdr *h) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride) {
         const BestRec b = h->pbest[p];
-        const int32_t score = b.valid ? b.ho - open : 0;
+        const int32_t score = b.valid && h->out[1] == 0 ? b.ho - open : 0;
         args[p].score = score;
         int64_t *S = st + p * kStN;
 #pragma unroll
