@@ -71,9 +71,10 @@ typedef struct {
  * returns SWB_ETIMEOUT with the context still usable.  Pairs of one strip (at
  * most 448 rows) have no wait and are unaffected. */
 #define SWB_FLAG_TEST_WITHHOLD 0x80000000u
-/* Test hook of swb_batch_align[_device]: a pass in packed strips (32-bit scores as
- * a base and 16-bit offsets) reports that its offsets did not fit, which no batch
- * of pairs does by itself, so the batch runs again in 32-bit strips.  Results do
+/* Test hook of swb_batch_align[_device], and of swb_align_pair[_device] where the
+ * traceback recomputes cells of a coarse grid: a pass in packed strips (32-bit
+ * scores as a base and 16-bit offsets) reports that its offsets did not fit, which
+ * no whole pair does by itself, so the pass runs again in 32-bit strips.  Results do
  * not change. */
 #define SWB_FLAG_TEST_PACK_ANY 0x40000000u
 

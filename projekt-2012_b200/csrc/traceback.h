@@ -132,9 +132,10 @@ int64_t walk_graph_ctas(int sms);
 // Canonical traceback from the end cell in `out` (score, end_row, end_col set by
 // stage 1), using the stage-1 stores laid out by `plan`.  Fills out->ops,
 // out->n_ops, start_*, xpoints.  Returns SWB_OK or an SWB_E* code with `err`.
+// test_range: level-1 recomputes in packed strips report kStage1Range.
 int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const uint8_t *d_cols, int64_t n,
               const swb_scoring *sc, const Plan &plan, const int2 *d_srows, const int2 *d_scols, swb_result *out,
-              const Scratch &scr, std::string &err, int32_t *launches);
+              const Scratch &scr, std::string &err, int32_t *launches, bool test_range = false);
 
 }  // namespace tb
 }  // namespace swb

@@ -41,3 +41,19 @@ def test_batch_redone_in_32_bits(gpu_ctx, monkeypatch, count, graph, frac):
         wide = gpu_ctx.batch_align(buf, refs, sc, trace_frac=frac)
         monkeypatch.delenv("SWB_BATCH_PACK")
         assert redone.kernel_launches == wide.kernel_launches  # what ran last were 32-bit strips
+
+
+def test_level1_recompute_redone_in_32_bits():
+    """A small HBM budget keeps the coarse grid; the first round of recomputed cells is
+    done again, which shows in the launches."""
+    rng = random.Random(5)
+    a = bytes(rng.choices(b"ACGT", k=6000))
+    b = bytes(c if rng.random() > 0.08 else rng.choice(b"ACGT") for c in a[300:5600])
+    sc = swb200.scoring(1, -3, -5, -2)
+    with swb200.Context(device=0, hbm_budget_bytes=1 << 20) as ctx:
+        plain = ctx.align(a, b, sc)
+        redone = ctx.align(a, b, sc, swb200.FLAG_TEST_PACK_ANY)
+    assert plain.score > 3000 and redone.kernel_launches == plain.kernel_launches + 2
+    for f in ("score", "end_row", "end_col", "start_row", "start_col", "ops"):
+        assert getattr(plain, f) == getattr(redone, f), f
+    assert [tuple(x) for x in plain.xpoints] == [tuple(x) for x in redone.xpoints]
