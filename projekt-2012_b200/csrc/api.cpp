@@ -595,11 +595,14 @@ int align_device(swb_ctx *c, const uint8_t *d_rows, int64_t m, const uint8_t *d_
             return swb::ctx_put((swb_ctx *)owner, dst, src, bytes);
         };
         int32_t launches = 0;
+        // what the stores leave of the budget
+        const uint64_t kept = (uint64_t)(out->special_bytes - out->host_bytes);
+        const uint64_t seg_bytes = c->opts.hbm_budget_bytes > kept ? c->opts.hbm_budget_bytes - kept : 0;
         // a capped context (the serving loop's long lane) sizes its stage-2 grids
         // to the same share of the GPU as its stage 1 (4 scoring blocks per SM)
         const int tb_sms = c->max_blocks > 0 ? std::max(1, std::min(c->sms, c->max_blocks / 4)) : c->sms;
         rc = tb::traceback(c->stream, tb_sms, d_rows, m, d_cols, n, sc, plan, c->last_srows, c->last_scols, out, scr,
-                           c->err, &launches, (flags & SWB_FLAG_TEST_PACK_ANY) != 0);
+                           c->err, &launches, seg_bytes, (flags & SWB_FLAG_TEST_PACK_ANY) != 0);
         if (rc != SWB_OK) return ctx_fail(c, rc, "%s", c->err.c_str());
         out->kernel_launches += launches;
         out->stage2_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t1).count();

@@ -659,7 +659,15 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
     if (traced) {
         std::vector<int64_t> rows((size_t)np);
         for (int64_t k = 0; k < np; ++k) rows[(size_t)k] = gp.bp[(size_t)k].m;
-        nseg = tb::seg_plan(rows.data(), np, c->sms, seg_base, seg_items);
+        nseg = tb::seg_plan(rows.data(), np, c->opts.hbm_budget_bytes - (uint64_t)(srn + scn) * sizeof(int2), seg_base,
+                            seg_items);
+        // whole MiB, so that batches of about the same size share it; without it the
+        // pairs are walked in one piece
+        const size_t mib = (size_t)1 << 20;
+        if (nseg > 0 && c->g_seg.ensure((tb::seg_scratch_bytes(nseg) + mib - 1) / mib * mib) != cudaSuccess) {
+            cudaGetLastError();
+            nseg = 0;
+        }
     }
     // device layouts (16-byte aligned sections)
     const size_t wa_bytes = tb::walk_args_bytes();
@@ -686,7 +694,6 @@ int graph_pass(swb_ctx *c, const uint8_t *h_seq, int64_t seq_bytes, const std::v
     if ((e = c->g_hdr.ensure(hdr_all)) != cudaSuccess || (e = c->g_in.ensure(in_bytes)) != cudaSuccess ||
         (e = c->g_work.ensure(work_bytes)) != cudaSuccess || (e = c->g_out.ensure(out_bytes)) != cudaSuccess ||
         (traced && (e = c->g_dir.ensure(tb::walk_batch_dir_bytes(c->sms, tb::walk_graph_ctas(c->sms)))) != cudaSuccess) ||
-        (nseg > 0 && (e = c->g_seg.ensure(pow2_at_least(tb::seg_scratch_bytes(nseg)))) != cudaSuccess) ||
         (e = c->h_gin.ensure(pow2_at_least(hdr_bytes + in_bytes))) != cudaSuccess ||
         (e = c->h_gout.ensure(pow2_at_least(out_bytes))) != cudaSuccess)
         return ctx_cuda_fail(c, e, "graphed batch buffers");
@@ -1122,8 +1129,7 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
                 if ((e = c->b_ops.ensure((size_t)std::max<int64_t>(1, ops_total))) != cudaSuccess ||
                     (e = c->b_xps.ensure(sizeof(int64_t) * 4 * (size_t)std::max<int64_t>(1, xp_total))) != cudaSuccess ||
                     (e = c->b_state.ensure(sizeof(int64_t) * kS * std::max<size_t>(1, tr.size()))) != cudaSuccess ||
-                    (e = c->b_walk.ensure(tb::walk_args_bytes() * std::max<size_t>(1, tr.size()))) != cudaSuccess ||
-                    (e = c->b_gdir.ensure(tb::walk_batch_dir_bytes(c->sms, (int64_t)tr.size()))) != cudaSuccess)
+                    (e = c->b_walk.ensure(tb::walk_args_bytes() * std::max<size_t>(1, tr.size()))) != cudaSuccess)
                     return ctx_cuda_fail(c, e, "batch traceback buffers");
                 std::vector<tb::WalkInputs> win(tr.size());
                 st.assign((size_t)kS * tr.size(), 0);
@@ -1173,8 +1179,9 @@ int batch_run_strips(swb_ctx *c, const uint8_t *h_seq, const uint8_t *d_seq_in, 
                     swb_ctx *cx = (swb_ctx *)owner;
                     return cx->tb[which].ensure(bytes) == cudaSuccess ? cx->tb[which].p : nullptr;
                 };
+                const uint64_t seg_bytes = c->opts.hbm_budget_bytes - (uint64_t)(srn + scn) * sizeof(int2);
                 int rc = tb::walk_batch(c->stream, c->sms, win.data(), (int64_t)win.size(), c->b_walk.p,
-                                        (int64_t *)c->b_state.p, c->b_gdir.p, st.data(), scr, err, &launches);
+                                        (int64_t *)c->b_state.p, seg_bytes, st.data(), scr, err, &launches);
                 if (rc != SWB_OK) return ctx_fail(c, rc, "%s", err.c_str());
                 std::vector<int64_t> ends(2 * tr.size()), offs;
                 for (size_t k = 0; k < tr.size(); ++k) {

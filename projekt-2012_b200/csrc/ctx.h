@@ -54,7 +54,7 @@ struct swb_ctx {
     swb::DevBuf tb[32];  // traceback scratch (ops, crosspoints, state, level-2 stores, recompute and walker buffers)
     // batched path: sequences, encodings, descriptors, per-unit / per-pair records, stores
     swb::DevBuf b_seq, b_rcode, b_ctab, b_pairs, b_units, b_hbuf, b_gbest, b_ubest, b_pbest, b_ctl, b_srows,
-        b_scols, b_walk, b_ops, b_xps, b_state, b_gdir;
+        b_scols, b_walk, b_ops, b_xps, b_state;
     swb::MappedBuf srows_h, scols_h;  // special rows / columns spilled to pinned host memory
     int2 *last_srows = nullptr, *last_scols = nullptr;  // where the last stage 1 kept them
     int64_t last_host_bytes = 0;
@@ -91,7 +91,7 @@ struct swb_ctx {
         for (swb::DevBuf *b : {&rows, &cols, &hbuf, &wbest, &best, &errf, &srows, &scols, &work, &flags, &lut,
                                &rcode, &ctab, &trace, &b_seq, &b_rcode, &b_ctab, &b_pairs, &b_units, &b_hbuf,
                                &b_gbest, &b_ubest, &b_pbest, &b_ctl, &b_srows, &b_scols, &b_walk, &b_ops, &b_xps,
-                               &b_state, &b_gdir, &g_hdr, &g_in, &g_work, &g_out, &g_dir, &g_seg})
+                               &b_state, &g_hdr, &g_in, &g_work, &g_out, &g_dir, &g_seg})
             f(*b);
         for (swb::DevBuf &b : tb) f(b);
     }

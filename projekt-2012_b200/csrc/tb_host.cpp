@@ -27,7 +27,7 @@ int64_t level1_cell_store_bytes(const Plan &plan) {
 
 int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const uint8_t *d_cols, int64_t n,
               const swb_scoring *sc, const Plan &plan, const int2 *d_srows, const int2 *d_scols, swb_result *out,
-              const Scratch &scr, std::string &err, int32_t *launches, bool test_range) {
+              const Scratch &scr, std::string &err, int32_t *launches, uint64_t seg_bytes, bool test_range) {
     const int kBR = block_rows(), kBC = block_cols();
     const int64_t ops_cap = m + n + 8;
     int32_t G = 0, T = 0;
@@ -65,6 +65,7 @@ int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const 
     int rc;
     if (!plan.level1) {
         w.br = plan.br;
+        w.seg_bytes = seg_bytes;
         w.srows = d_srows;
         w.scols = d_scols;
         w.rr0 = 0;

@@ -851,7 +851,9 @@ constexpr int kSegXps = 160;
 // A pair alone: below this many segments one corridor of precomputed blocks is as fast.
 constexpr int kSegPairMin = 8;
 constexpr int kSegChain = 32;  // records a batched pair's CTA looks at together
-constexpr int64_t kSegMax = 65536;  // segments of one launch
+// Segments of one launch (9.4 KB of records and outputs each): of a batch, and of a
+// pair walked alone, which takes its segments in windows from its current row up.
+constexpr int64_t kSegMax = 65536, kSegWindow = 4096;
 constexpr int kSegMin = 3;     // segments a pair must have to be walked in segments
 
 struct SegArgs {
@@ -1320,25 +1322,33 @@ static void launch_segments(const SegArgs &g, bool wide, int64_t grid, cudaStrea
     }
 }
 
-// Segments of a pair from host_state's cell up: takes over the ones that continue the
-// path and returns their number in *taken.  in.dstate holds host_state.
+// Segments of a pair from host_state's cell up, a window of them: takes over the ones
+// that continue the path and returns their number in *taken, or -1 when there are too
+// few of them or no memory for them (the pair is walked without).  in.dstate holds
+// host_state; gdir: blocks of walk_graph_ctas(sms) CTAs.
 static int walk_pair_segments(cudaStream_t st, int sms, const WalkInputs &in, const WalkArgs &a, int64_t *host_state,
-                              const Scratch &scr, std::string &err, int32_t *launches, int64_t *taken) {
+                              uint32_t *gdir, const Scratch &scr, std::string &err, int32_t *launches, int64_t *taken) {
     cudaError_t e;
-    *taken = 0;
-    const int64_t nseg = host_state[kStR] / a.br + 1, grid = std::min<int64_t>(nseg, walk_graph_ctas(sms));
+    *taken = -1;
+    // up to the rows for which guess_column still looks inside the matrix
+    const int64_t top = host_state[kStR] / a.br, reach = (host_state[kStC] + 512) * 16 / 15 / a.br + 2;
+    const int64_t nseg = std::min({top + 1, reach, kSegWindow, (int64_t)(in.seg_bytes / seg_scratch_bytes(1))});
+    if (nseg < kSegPairMin) return SWB_OK;
+    const int64_t q0 = top + 1 - nseg, grid = std::min<int64_t>(nseg, walk_graph_ctas(sms));
     SegRec *rec = (SegRec *)scr.ensure(scr.owner, kScrSegRec, seg_scratch_bytes(nseg));
     char *d_items = (char *)scr.ensure(scr.owner, kScrSegItems, sizeof(WalkArgs) + 16 + sizeof(int2) * (size_t)nseg);
     int64_t *d_off = (int64_t *)scr.ensure(scr.owner, kScrSegOff, sizeof(int64_t) * 2 * (size_t)nseg);
-    uint32_t *gdir = (uint32_t *)scr.ensure(scr.owner, kScrGdir, sizeof(uint32_t) * (size_t)(grid * kBlockWords));
-    if (!rec || !d_items || !d_off || !gdir) {
-        err = "walker buffers: out of device memory";
-        return SWB_ENOMEM;
+    if (!rec || !d_items || !d_off) {
+        cudaGetLastError();
+        return SWB_OK;
     }
+    *taken = 0;
     std::vector<char> up(sizeof(WalkArgs) + 16 + sizeof(int2) * (size_t)nseg, 0);
-    std::memcpy(up.data(), &a, sizeof a);  // then the pair's first segment index (0) and the items
+    std::memcpy(up.data(), &a, sizeof a);
+    const int32_t base = (int32_t)-q0;  // segment q's record is base + q
+    std::memcpy(up.data() + sizeof(WalkArgs), &base, sizeof base);
     int2 *items = (int2 *)(up.data() + sizeof(WalkArgs) + 16);
-    for (int64_t q = 0; q < nseg; ++q) items[q] = make_int2(0, (int)q);
+    for (int64_t k = 0; k < nseg; ++k) items[k] = make_int2(0, (int)(q0 + k));
     if ((e = scr.put(scr.owner, d_items, up.data(), up.size())) != cudaSuccess) {
         err = std::string("walker segments: ") + cudaGetErrorString(e);
         return SWB_ECUDA;
@@ -1363,8 +1373,8 @@ static int walk_pair_segments(cudaStream_t st, int sms, const WalkInputs &in, co
     }
     std::vector<int64_t> off;
     int64_t *S = host_state;
-    for (int64_t q = nseg - 1; q >= 0 && !S[kStDone]; --q) {
-        const SegRec &r = h[(size_t)q];
+    for (int64_t k = nseg - 1; k >= 0 && !S[kStDone]; --k) {
+        const SegRec &r = h[(size_t)k];
         if (!r.valid || r.er != S[kStR] || r.ec != S[kStC] || r.est != S[kStState] || r.val != a.score - S[kStSuffix]) break;
         off.push_back(S[kStNOps]);
         off.push_back(S[kStNXp]);
@@ -1404,9 +1414,16 @@ int walk_region(cudaStream_t st, int sms, const WalkInputs &in, int64_t *host_st
     const WalkArgs a = to_args(in);
     cudaError_t e;
     const int64_t cap = 4LL * std::max(1, sms);  // blocks per round: one wave at four CTAs per SM
-    // (as large as the segments need it, so that it stays where it is)
-    uint32_t *gdir = (uint32_t *)scr.ensure(scr.owner, kScrGdir,
-                                            sizeof(uint32_t) * (size_t)(std::max(cap, walk_graph_ctas(sms)) * kBlockWords));
+    // as large as segments need it, so that it stays where it is, or without them
+    bool segments = host_state[kStR] >= kSegPairMin * (int64_t)a.br;
+    uint32_t *gdir = nullptr;
+    if (segments) {
+        gdir = (uint32_t *)scr.ensure(scr.owner, kScrGdir,
+                                      sizeof(uint32_t) * (size_t)(std::max(cap, walk_graph_ctas(sms)) * kBlockWords));
+        if (!gdir) cudaGetLastError();
+        segments = gdir != nullptr;
+    }
+    if (!gdir) gdir = (uint32_t *)scr.ensure(scr.owner, kScrGdir, sizeof(uint32_t) * (size_t)(cap * kBlockWords));
     int64_t *d_blk = (int64_t *)scr.ensure(scr.owner, kScrBlk, sizeof(int64_t) * 2 * (size_t)cap);
     int32_t *d_err = (int32_t *)scr.ensure(scr.owner, kScrWalkErr, sizeof(int32_t));
     if (!gdir || !d_blk || !d_err) {
@@ -1423,10 +1440,11 @@ int walk_region(cudaStream_t st, int sms, const WalkInputs &in, int64_t *host_st
     // a pair of many blocks: segments at once as long as they continue the path, a
     // corridor round where they do not
     for (int round = 0; round < (1 << 26); ++round) {
-        if (!host_state[kStDone] && host_state[kStR] >= kSegPairMin * (int64_t)a.br) {
+        if (segments && !host_state[kStDone] && host_state[kStR] >= kSegPairMin * (int64_t)a.br) {
             int64_t taken = 0;
-            const int rc = walk_pair_segments(st, sms, in, a, host_state, scr, err, launches, &taken);
+            const int rc = walk_pair_segments(st, sms, in, a, host_state, gdir, scr, err, launches, &taken);
             if (rc != SWB_OK) return rc;
+            segments = taken >= 0;
             if (taken > 0 && (e = scr.put(scr.owner, in.dstate, host_state, sizeof(int64_t) * kStN)) != cudaSuccess) {
                 err = std::string("walker state: ") + cudaGetErrorString(e);
                 return SWB_ECUDA;
@@ -1562,7 +1580,7 @@ size_t walk_batch_dir_bytes(int sms, int64_t n) {
 }
 
 int walk_batch(cudaStream_t st, int sms, const WalkInputs *in, int64_t n, void *d_args, int64_t *d_states,
-               void *d_dir, int64_t *host_states, const Scratch &scr, std::string &err, int32_t *launches) {
+               uint64_t seg_bytes, int64_t *host_states, const Scratch &scr, std::string &err, int32_t *launches) {
     if (n <= 0) return SWB_OK;
     std::vector<WalkArgs> args((size_t)n);
     std::vector<int64_t> rows((size_t)n);
@@ -1581,16 +1599,30 @@ int walk_batch(cudaStream_t st, int sms, const WalkInputs *in, int64_t n, void *
     }
     SegArgs g{};
     std::vector<int32_t> base, items;
-    const int64_t nseg = scr.ensure ? seg_plan(rows.data(), n, sms, base, items) : 0;
+    int64_t nseg = seg_plan(rows.data(), n, seg_bytes, base, items);
+    const int64_t sgrid = std::min<int64_t>(walk_graph_ctas(sms), nseg);
+    auto blocks = [&](int64_t ctas) {
+        return (uint32_t *)scr.ensure(scr.owner, kScrGdir, sizeof(uint32_t) * (size_t)(ctas * kBlockWords));
+    };
+    // segments and walk run one after the other on the same direction blocks; where
+    // there is no memory for segments, the pairs are walked in one piece
+    uint32_t *gdir = nullptr;
+    SegRec *rec = nullptr;
+    int32_t *d_items = nullptr;
     if (nseg > 0) {
-        const int64_t sgrid = std::min<int64_t>(walk_graph_ctas(sms), nseg);
-        SegRec *rec = (SegRec *)scr.ensure(scr.owner, kScrSegRec, seg_scratch_bytes(nseg));
-        int32_t *d_items = (int32_t *)scr.ensure(scr.owner, kScrSegItems, sizeof(int32_t) * (items.size() + base.size()));
-        uint32_t *gdir = (uint32_t *)scr.ensure(scr.owner, kScrGdir, sizeof(uint32_t) * (size_t)(sgrid * kBlockWords));
-        if (!rec || !d_items || !gdir) {
-            err = "walker buffers: out of device memory";
-            return SWB_ENOMEM;
+        rec = (SegRec *)scr.ensure(scr.owner, kScrSegRec, seg_scratch_bytes(nseg));
+        d_items = (int32_t *)scr.ensure(scr.owner, kScrSegItems, sizeof(int32_t) * (items.size() + base.size()));
+        if (rec && d_items) gdir = blocks(std::max(grid, sgrid));
+        if (!gdir) {
+            cudaGetLastError();
+            nseg = 0;
         }
+    }
+    if (!gdir && !(gdir = blocks(grid))) {
+        err = "walker buffers: out of device memory";
+        return SWB_ENOMEM;
+    }
+    if (nseg > 0) {
         std::vector<int32_t> up(items);
         up.insert(up.end(), base.begin(), base.end());
         if ((e = scr.put(scr.owner, d_items, up.data(), sizeof(int32_t) * up.size())) != cudaSuccess) {
@@ -1609,8 +1641,8 @@ int walk_batch(cudaStream_t st, int sms, const WalkInputs *in, int64_t n, void *
         launch_segments(g, wide, sgrid, st);
         *launches += 2;
     }
-    if (wide) walk_batch_kernel<true><<<(unsigned)grid, kThreadsWide, 0, st>>>((const WalkArgs *)d_args, n, (uint32_t *)d_dir, g);
-    else walk_batch_kernel<false><<<(unsigned)grid, kThreads, 0, st>>>((const WalkArgs *)d_args, n, (uint32_t *)d_dir, g);
+    if (wide) walk_batch_kernel<true><<<(unsigned)grid, kThreadsWide, 0, st>>>((const WalkArgs *)d_args, n, gdir, g);
+    else walk_batch_kernel<false><<<(unsigned)grid, kThreads, 0, st>>>((const WalkArgs *)d_args, n, gdir, g);
     *launches += 1;
     if ((e = cudaGetLastError()) != cudaSuccess ||
         (e = scr.get(scr.owner, host_states, d_states, sizeof(int64_t) * kStN * (size_t)n)) != cudaSuccess) {
@@ -1691,15 +1723,16 @@ cudaError_t walk_graph_enqueue(const GraphHdr *d_hdr, bool wide, bool segments, 
     return cudaGetLastError();
 }
 
-int64_t seg_plan(const int64_t *rows, int64_t n, int sms, std::vector<int32_t> &base, std::vector<int32_t> &items) {
+int64_t seg_plan(const int64_t *rows, int64_t n, uint64_t max_bytes, std::vector<int32_t> &base,
+                 std::vector<int32_t> &items) {
     base.assign((size_t)n, -1);
     items.clear();
     int64_t total = 0;
     for (int64_t p = 0; p < n; ++p) total += (rows[p] + kBR - 1) / kBR;
-    // (9 KB of records and outputs each.)  Segments pay even where the pairs alone fill
+    // Segments pay even where the pairs alone fill
     // the GPU: few are walked twice, and none is left over at the end (1,000 long
     // pairs of the 100,000-pair batch: 6.4 ms, against about 15 ms walked pair by pair).
-    if (total > kSegMax) return 0;
+    if (total > kSegMax || seg_scratch_bytes(total) > max_bytes) return 0;
     int32_t seg = 0;
     for (int64_t p = 0; p < n; ++p) {
         const int32_t k = (int32_t)((rows[p] + kBR - 1) / kBR);
@@ -1717,6 +1750,13 @@ int64_t seg_plan(const int64_t *rows, int64_t n, int sms, std::vector<int32_t> &
 size_t seg_scratch_bytes(int64_t nseg) {
     return (size_t)nseg * (2 * sizeof(SegRec) + kSegOps + sizeof(int64_t) * 4 * kSegXps);
 }
+
+uint64_t seg_pair_bytes(int64_t rows) {
+    const int64_t k = (rows + kBR - 1) / kBR;
+    return k < kSegMin ? 0 : (uint64_t)seg_scratch_bytes(k);
+}
+
+int64_t seg_window() { return kSegWindow; }
 
 int64_t walk_graph_ctas(int sms) { return 8LL * std::max(1, sms); }
 

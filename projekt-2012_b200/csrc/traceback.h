@@ -55,6 +55,7 @@ struct WalkInputs {
     int64_t xp_cap;
     int64_t *dstate;              // device copy of the walker state
     int64_t br;                   // block rows of the region's grid (0: 512)
+    uint64_t seg_bytes;           // device memory that segments may take (walk_region)
 };
 
 
@@ -101,10 +102,10 @@ int walk_cells(cudaStream_t st, int sms, const WalkInputs &whole, const std::vec
 
 // Walks n independent pairs (each region is its pair's whole matrix) with one
 // launch; d_args holds n * walk_args_bytes() bytes, d_states n * state_slots()
-// int64 (initial states are copied from host_states, final ones back to it),
-// d_dir walk_batch_dir_bytes(sms, n) bytes of direction scratch.
+// int64 (initial states are copied from host_states, final ones back to it).
+// seg_bytes: device memory that segments may take.
 int walk_batch(cudaStream_t st, int sms, const WalkInputs *in, int64_t n, void *d_args, int64_t *d_states,
-               void *d_dir, int64_t *host_states, const Scratch &scr, std::string &err, int32_t *launches);
+               uint64_t seg_bytes, int64_t *host_states, const Scratch &scr, std::string &err, int32_t *launches);
 size_t walk_batch_dir_bytes(int sms, int64_t n);
 // Results of n walked pairs (as walk_batch left them; ends: end cell per pair) laid
 // out on the device in their final form, pair after pair: offs holds per pair
@@ -124,18 +125,24 @@ cudaError_t walk_graph_enqueue(const GraphHdr *d_hdr, bool wide, bool segments, 
                                int64_t max_units, cudaStream_t st);
 // Segments (traceback.cu) of n pairs with the given row counts: per pair its first
 // segment's index or -1, and the items (pair, segment); returns their number, 0
-// when the pairs alone fill the GPU.  seg_scratch_bytes: records and outputs.
-int64_t seg_plan(const int64_t *rows, int64_t n, int sms, std::vector<int32_t> &base, std::vector<int32_t> &items);
+// (walk without them) past 65,536 or when their records and outputs
+// (seg_scratch_bytes) take more than max_bytes.  seg_pair_bytes: those of one pair.
+int64_t seg_plan(const int64_t *rows, int64_t n, uint64_t max_bytes, std::vector<int32_t> &base,
+                 std::vector<int32_t> &items);
 size_t seg_scratch_bytes(int64_t nseg);
+uint64_t seg_pair_bytes(int64_t rows);
+// Most segments of one launch of a pair walked alone.
+int64_t seg_window();
 int64_t walk_graph_ctas(int sms);
 
 // Canonical traceback from the end cell in `out` (score, end_row, end_col set by
 // stage 1), using the stage-1 stores laid out by `plan`.  Fills out->ops,
 // out->n_ops, start_*, xpoints.  Returns SWB_OK or an SWB_E* code with `err`.
-// test_range: level-1 recomputes in packed strips report kStage1Range.
+// seg_bytes: device memory that segments may take.  test_range: level-1 recomputes in
+// packed strips report kStage1Range.
 int traceback(cudaStream_t st, int sms, const uint8_t *d_rows, int64_t m, const uint8_t *d_cols, int64_t n,
               const swb_scoring *sc, const Plan &plan, const int2 *d_srows, const int2 *d_scols, swb_result *out,
-              const Scratch &scr, std::string &err, int32_t *launches, bool test_range = false);
+              const Scratch &scr, std::string &err, int32_t *launches, uint64_t seg_bytes, bool test_range = false);
 
 }  // namespace tb
 }  // namespace swb
