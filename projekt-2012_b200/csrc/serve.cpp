@@ -59,8 +59,10 @@ struct Request {
     int32_t batch_size = 0;
 };
 
-// Device bytes a short request holds while it runs (batched path with stores).
-uint64_t short_footprint(int64_t m, int64_t n) {
+// Device bytes a short request holds while it runs (batched path with stores), and what
+// it may take beyond them (more: stage 2 does without where there is no room).
+uint64_t short_footprint(int64_t m, int64_t n, uint64_t *more) {
+    *more = swb::tb::seg_pair_bytes(m);
     const uint64_t seq = 6ULL * (uint64_t)(m + n);                       // bytes, codes, table words
     const uint64_t hbuf = 16ULL * (uint64_t)n;
     const uint64_t stores = 8ULL * ((uint64_t)(m / 512) * n + (uint64_t)(n / 256) * m);
@@ -69,8 +71,8 @@ uint64_t short_footprint(int64_t m, int64_t n) {
 }
 
 // Device bytes a long request holds: the pair path's buffers with its special
-// rows / columns sized to `store_budget`.
-uint64_t long_footprint(int64_t m, int64_t n, uint64_t store_budget, int sms) {
+// rows / columns sized to `store_budget`; more: as above.
+uint64_t long_footprint(int64_t m, int64_t n, uint64_t store_budget, int sms, uint64_t *more) {
     swb_options o;
     swb_options_default(&o);
     o.hbm_budget_bytes = store_budget;
@@ -79,7 +81,9 @@ uint64_t long_footprint(int64_t m, int64_t n, uint64_t store_budget, int sms) {
     const uint64_t level2 = p.level1 ? (uint64_t)swb::tb::level1_corridor_cells(p, sms) *
                                            (uint64_t)swb::tb::level1_cell_store_bytes(p)
                                      : 0;
-    const uint64_t walker = (uint64_t)8 * 148 * 81920;  // direction blocks of the walker's CTAs
+    const uint64_t block = 81920;  // direction words of a block
+    const uint64_t walker = (uint64_t)4 * sms * block;  // a corridor's blocks; segments have as many again
+    *more = walker + (uint64_t)swb::tb::seg_scratch_bytes(swb::tb::seg_window());
     return 6ULL * (uint64_t)(m + n) + 16ULL * (uint64_t)n + stores + level2 + walker + (uint64_t)(m + n + 8) +
            (64ULL << 20);
 }
@@ -366,7 +370,8 @@ int swb_server_submit(swb_server *s, const uint8_t *a, int64_t la, const uint8_t
     r->m = std::max(la, lb);
     r->n = std::min(la, lb);
     r->is_long = r->m * r->n > s->o.long_cells;
-    r->foot = r->is_long ? long_footprint(r->m, r->n, s->long_store_budget, s->sms) : short_footprint(r->m, r->n);
+    uint64_t more = 0;
+    r->foot = r->is_long ? long_footprint(r->m, r->n, s->long_store_budget, s->sms, &more) : short_footprint(r->m, r->n, &more);
     r->t_submit = Clock::now();
     if (r->foot > s->o.hbm_budget_bytes) {
         const uint64_t f = r->foot;
@@ -374,6 +379,7 @@ int swb_server_submit(swb_server *s, const uint8_t *a, int64_t la, const uint8_t
         return swb::ctx_fail(nullptr, SWB_ENOMEM_BUDGET, "request needs %llu bytes > server budget %llu",
                              (unsigned long long)f, (unsigned long long)s->o.hbm_budget_bytes);
     }
+    r->foot = std::min<uint64_t>(r->foot + more, s->o.hbm_budget_bytes);
     {
         std::lock_guard<std::mutex> lk(s->mu);
         if (s->stop) {

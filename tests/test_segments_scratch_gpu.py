@@ -71,3 +71,24 @@ def test_a_tall_pair_takes_no_scratch_for_rows_its_path_cannot_reach():
     # codes (1), operations (1), crosspoints (1.6) and special rows (2.1) are about 6
     # bytes a row, the walker's blocks 97 MB; a segment for every 448 rows is 21 more
     assert used < 16 * m
+
+
+def test_the_server_admits_requests_with_their_segments():
+    """A request's reservation holds its segments, but a budget that only holds the
+    request without them takes it all the same."""
+    rng = random.Random(4)
+    a, b = _pair(rng, 5000)
+    m = n = 5000
+    plain = 6 * (m + n) + 16 * n + 8 * (m // 512 * n + n // 256 * m) + (m + n + 8) + 32 * (m // 4 + 8) + 4096
+    segments = 10 * (2 * 80 + 4096 + 8 * 4 * 160)
+    sc = swb200.scoring(1, -3, -5, -2)
+    results = []
+    for budget, reserved in ((1 << 30, plain + segments), (plain + 1000, plain + 1000)):
+        with swb200.Server(sc, hbm_budget_bytes=budget) as srv:
+            results.append(srv.wait(srv.submit(a, b))[0])
+            assert srv.stats()["peak_reserved_bytes"] == reserved
+        with pytest.raises(swb200.SwbError) as ei:
+            with swb200.Server(sc, hbm_budget_bytes=plain - 1) as srv:
+                srv.submit(a, b)
+        assert ei.value.code == swb200.SWB_ENOMEM_BUDGET
+    assert _same(*results)
