@@ -726,6 +726,17 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
     }
 }
 
+// The aligned word at p of the sequence bytes [lo, hi); bytes outside are not read.
+__device__ __forceinline__ uint32_t seq_word(const uint8_t *lo, const uint8_t *hi, const uint32_t *p) {
+    const uint8_t *b = reinterpret_cast<const uint8_t *>(p);
+    if (b >= lo && b + 4 <= hi) return *p;
+    uint32_t v = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (b + k >= lo && b + k < hi) v |= (uint32_t)b[k] << (8 * k);
+    return v;
+}
+
 // The walk of each block reads the block's direction words from shared memory:
 // on entering a block the warp copies the part the path can still reach (the
 // 256-row chunks at or above the current row, the steps up to the current
@@ -790,10 +801,12 @@ __global__ void __launch_bounds__(32) corridor_walk_kernel(WalkArgs a, const uin
             constexpr int kNR = kBR / 128 + 1, kNC = kBC / 128 + 1;
 #pragma unroll
             for (int q = 0; q < kNR; ++q)
-                if (lane + 32 * q < nr) v[q] = reinterpret_cast<const uint32_t *>(pr & ~(uintptr_t)3)[lane + 32 * q];
+                if (lane + 32 * q < nr)
+                    v[q] = seq_word(a.rows, a.rows + a.m, reinterpret_cast<const uint32_t *>(pr & ~(uintptr_t)3) + lane + 32 * q);
 #pragma unroll
             for (int q = 0; q < kNC; ++q)
-                if (lane + 32 * q < nc) v[kNR + q] = reinterpret_cast<const uint32_t *>(pc & ~(uintptr_t)3)[lane + 32 * q];
+                if (lane + 32 * q < nc)
+                    v[kNR + q] = seq_word(a.cols, a.cols + a.n, reinterpret_cast<const uint32_t *>(pc & ~(uintptr_t)3) + lane + 32 * q);
 #pragma unroll
             for (int q = 0; q < kNR; ++q)
                 if (lane + 32 * q < nr) seq_r[lane + 32 * q] = v[q];
