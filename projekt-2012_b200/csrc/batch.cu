@@ -485,6 +485,10 @@ cudaError_t batch_configure() {
                 if (x != cudaSuccess) e = x;
             }
     for (cudaError_t x : {cudaFuncSetAttribute((const void *)batch_reduce_kernel, A, c),
+                          cudaFuncSetAttribute((const void *)graph_prepare_kernel, A, c),
+                          cudaFuncSetAttribute((const void *)graph_decide_kernel, A, c),
+                          cudaFuncSetAttribute((const void *)graph_encode_kernel, A, c),
+                          cudaFuncSetAttribute((const void *)graph_reduce_kernel, A, c),
                           cudaFuncSetAttribute((const void *)batch_encode_kernel, A, c)})
         if (x != cudaSuccess) e = x;
     return e;

@@ -1187,7 +1187,18 @@ cudaError_t walker_configure() {
                           cudaFuncSetAttribute((const void *)walk_batch_kernel<false>, A, c),
                           cudaFuncSetAttribute((const void *)walk_batch_kernel<true>, A, c),
                           cudaFuncSetAttribute((const void *)walk_graph_kernel<false>, A, c),
-                          cudaFuncSetAttribute((const void *)walk_graph_kernel<true>, A, c)})
+                          cudaFuncSetAttribute((const void *)walk_graph_kernel<true>, A, c),
+                          cudaFuncSetAttribute((const void *)walk_graph_init_kernel, A, c),
+                          cudaFuncSetAttribute((const void *)seg_kernel<false, false>, A, c),
+                          cudaFuncSetAttribute((const void *)seg_kernel<false, true>, A, c),
+                          cudaFuncSetAttribute((const void *)seg_kernel<true, false>, A, c),
+                          cudaFuncSetAttribute((const void *)seg_kernel<true, true>, A, c),
+                          cudaFuncSetAttribute((const void *)seg_graph_kernel<false, false>, A, c),
+                          cudaFuncSetAttribute((const void *)seg_graph_kernel<false, true>, A, c),
+                          cudaFuncSetAttribute((const void *)seg_graph_kernel<true, false>, A, c),
+                          cudaFuncSetAttribute((const void *)seg_graph_kernel<true, true>, A, c),
+                          cudaFuncSetAttribute((const void *)seg_copy_kernel, A, c),
+                          cudaFuncSetAttribute((const void *)pack_results_kernel, A, c)})
         if (x != cudaSuccess) e = x;
     return e;
 }
