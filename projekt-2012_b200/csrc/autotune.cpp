@@ -7,8 +7,8 @@
 // R = 16 is 25% faster than R = 8).  So the first pair of a shape bucket times
 // every candidate on a slice of that pair (all its rows, up to 2^18 columns, the
 // same kernel mode), keeps the fastest, and later pairs of the bucket reuse it.
-// Buckets: SM count, store mode, substitution mode, ceil(log2) of rows and of
-// columns.  With SWB_AUTOTUNE_CACHE=<file> the table is read at first use and
+// Buckets: SM count, store mode, kernel (packed strips, or 32-bit ones with table or
+// compare scores), ceil(log2) of rows and of columns.  With SWB_AUTOTUNE_CACHE=<file> the table is read at first use and
 // every new entry appended, so later processes skip the probes.  The special-row
 // spacing is the other tuned parameter; it is chosen from the HBM budget by the
 // traceback planner (the densest grid that fits).
@@ -47,10 +47,12 @@ int log2ceil(int64_t x) {
     return b;
 }
 
-std::string key_of(int sms, bool stores, bool tab, int64_t m, int64_t n) {
+// The kernel is part of the bucket: packed strips ("pk", table or compare scores
+// alike) and 32-bit ones differ in which height is fastest, and so do a packed launch's
+// kinds.
+std::string key_of(int sms, const char *kind, const char *strips, int64_t m, int64_t n) {
     char k[96];
-    snprintf(k, sizeof k, "sms%d %s %s r%d c%d", sms, stores ? "stores" : "score", tab ? "tab" : "cmp",
-             log2ceil(m), log2ceil(n));
+    snprintf(k, sizeof k, "sms%d %s %s r%d c%d", sms, kind, strips, log2ceil(m), log2ceil(n));
     return k;
 }
 
@@ -85,7 +87,8 @@ void store_locked(const std::string &key, int R) {
 
 std::string batch_tune_key(int sms, const char *pass, int64_t m, int64_t n) {
     char k[96];
-    snprintf(k, sizeof k, "sms%d %s tab r%d c%d", sms, pass, log2ceil(m), log2ceil(n));
+    // (p: strips of one pair; entries without it are another kernel's)
+    snprintf(k, sizeof k, "sms%d %s tab r%d c%dp", sms, pass, log2ceil(m), log2ceil(n));
     return k;
 }
 
@@ -126,7 +129,8 @@ int autotune_rows_per_lane(swb_ctx *c, const Stage1Args &base, bool tab, bool st
     // pairs below this many cells are not worth a probe
     constexpr double kMinCells = 2e10;
     if ((double)base.m * (double)base.n < kMinCells) return fallback;
-    const std::string key = key_of(c->sms, stores, tab, base.m, base.n) + (strip_rows ? "|strip" : "") +
+    const char *kind = stores ? "stores" : (packed && stage1_has_borders(base) ? "borders" : "score");
+    const std::string key = key_of(c->sms, kind, packed ? "pk" : (tab ? "tab" : "cmp"), base.m, base.n) + (strip_rows ? "|strip" : "") +
                             (sr_interval > 0 ? "|sr" + std::to_string(sr_interval) : "");
     {
         std::lock_guard<std::mutex> lk(g_mu);
