@@ -37,8 +37,8 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
-// A burst of 48 requests in one or two iterations instead of three or more: see
-// short_lane.
+// A burst of 48 requests in one or two iterations instead of three or more, without a
+// delay for requests whose clients wait already: see short_lane.
 constexpr int64_t kGatherUs = 100, kGatherMaxUs = 500;
 
 double ms_since(Clock::time_point t0, Clock::time_point t1) {
@@ -57,6 +57,7 @@ struct Request {
     swb_result res{};
     Clock::time_point t_submit, t_start, t_end;
     int32_t batch_size = 0;
+    bool waited = false;    // a swb_server_wait has begun
 };
 
 // Device bytes a short request holds while it runs (batched path with stores), and what
@@ -102,6 +103,7 @@ struct swb_server {
     std::unordered_map<uint64_t, Request *> reqs;
     uint64_t next_id = 1;
     uint64_t reserved = 0;
+    int64_t unwaited = 0;  // requests in qs that no client waits for yet
     bool stop = false;
     bool long_active = false;
     std::thread ts, tl;
@@ -133,9 +135,11 @@ struct swb_server {
                 if (stop && qs.empty()) return;
                 // An iteration of one or two pairs costs about as much as one of fifty, so
                 // while requests keep coming in, a moment's wait serves them together: up to
-                // kGatherUs after the newest request, kGatherMaxUs in all.
+                // kGatherUs after the newest request, kGatherMaxUs in all, and only while
+                // some queued request's client is not waiting for it yet (one that waits
+                // sends nothing more, and would only get its result later).
                 const auto gather_end = Clock::now() + std::chrono::microseconds(kGatherMaxUs);
-                while (!stop && (int)qs.size() < o.max_batch) {
+                while (!stop && unwaited > 0 && (int)qs.size() < o.max_batch) {
                     const auto until = std::min(gather_end, qs.back()->t_submit + std::chrono::microseconds(kGatherUs));
                     if (Clock::now() >= until) break;
                     cv_work.wait_until(lk, until);
@@ -149,6 +153,7 @@ struct swb_server {
                         if (stop) return;
                     }
                     qs.pop_front();
+                    if (!r->waited) --unwaited;
                     reserved += r->foot;
                     stats.peak_reserved_bytes = std::max<uint64_t>(stats.peak_reserved_bytes, reserved);
                     r->state = 1;
@@ -389,6 +394,7 @@ int swb_server_submit(swb_server *s, const uint8_t *a, int64_t la, const uint8_t
         r->id = s->next_id++;
         s->reqs[r->id] = r;
         (r->is_long ? s->ql : s->qs).push_back(r);
+        if (!r->is_long) s->unwaited += 1;
         s->stats.submitted += 1;
         *id = r->id;
     }
@@ -403,6 +409,10 @@ int swb_server_wait(swb_server *s, uint64_t id, int64_t timeout_ms, swb_result *
     auto it = s->reqs.find(id);
     if (it == s->reqs.end()) return swb::ctx_fail(nullptr, SWB_ENOTFOUND, "unknown request %llu", (unsigned long long)id);
     Request *r = it->second;
+    if (!r->waited) {
+        r->waited = true;
+        if (!r->is_long && r->state == 0 && --s->unwaited == 0) s->cv_work.notify_all();
+    }
     auto done = [&] { return r->state == 2; };
     if (timeout_ms < 0) s->cv_done.wait(lk, done);
     else if (!s->cv_done.wait_for(lk, std::chrono::milliseconds(timeout_ms), done)) return SWB_ETIMEOUT;
