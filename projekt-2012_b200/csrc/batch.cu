@@ -217,6 +217,7 @@ __device__ __forceinline__ void packed_body(const BatchArgs &g, bool tab) {
         if (rc != kErrNone) {
             if (lane == 0) {
                 atomicCAS(&g.ctl[1], kErrNone, rc);
+                __threadfence();  // a warp that stops for the abort flag reports a timeout: the code first
                 atomicExch(&g.ctl[2], 1);
             }
             break;
