@@ -215,9 +215,10 @@ __device__ __forceinline__ void packed_body(const BatchArgs &g, bool tab) {
             __syncwarp();
         }
         if (rc != kErrNone) {
-            if (lane == 0) {
+            // (a warp that stopped for the abort flag comes here with a timeout: the code is
+            // the other warp's to report)
+            if (lane == 0 && (rc == kErrRange || ld_volatile(&g.ctl[2]) == 0)) {
                 atomicCAS(&g.ctl[1], kErrNone, rc);
-                __threadfence();  // a warp that stops for the abort flag reports a timeout: the code first
                 atomicExch(&g.ctl[2], 1);
             }
             break;

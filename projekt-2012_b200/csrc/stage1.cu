@@ -182,9 +182,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4) stage1_packed_kernel(Stage1Arg
         }
     }
     if (lane == 0) {
-        if (rc != kErrNone) {
+        // (a warp that stopped for the abort flag comes here with a timeout: the code is the
+        // other warp's to report)
+        if (rc == kErrRange || (rc != kErrNone && ld_volatile(&a.err[1]) == 0)) {
             atomicCAS(&a.err[0], kErrNone, rc);
-            __threadfence();  // a warp that stops for the abort flag reports a timeout: the code first
             atomicExch(&a.err[1], 1);
         }
         BestRec r;
