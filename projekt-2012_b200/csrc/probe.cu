@@ -1,5 +1,6 @@
-// probe.cu -- the cell-update roofline: the stage-1 per-cell DPX/INT32 mix run
-// at full occupancy with no memory traffic, and the single-op rates.
+// probe.cu -- the cell-update rooflines: the per-cell op mixes of stage 1's 32-bit and
+// packed 16-bit steps run at full occupancy with no memory traffic, and the single-op
+// rates.
 #include <cstdio>
 
 #include "swb_internal.h"
@@ -46,6 +47,43 @@ __global__ void cell_mix_kernel(const int32_t *in, int32_t *out, int iters) {
 #pragma unroll
     for (int c = 0; c < kChains; ++c) acc ^= HO[c] ^ E[c] ^ f[c] ^ cm[c] ^ hod[c];
     out[tid] = acc;
+}
+
+// Two cells of strip16.cuh's step2() per chain and iteration: PRMT score, E, t, t + open,
+// H + open and F' (runs that look for no best cell have no more).
+__global__ void packed_mix_kernel(const int32_t *in, int32_t *out, int iters) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t HO[kChains], E[kChains], f[kChains], hod[kChains], sel[kChains];
+    const uint32_t ext = (uint32_t)in[0], open = (uint32_t)in[1], gx = (uint32_t)in[2];
+#pragma unroll
+    for (int c = 0; c < kChains; ++c) {
+        HO[c] = (uint32_t)in[3] + c + tid;
+        E[c] = (uint32_t)in[4] + c;
+        f[c] = (uint32_t)in[5] + c;
+        hod[c] = (uint32_t)in[6] + tid;
+        sel[c] = (uint32_t)in[7 + c];  // all different, so that no chain shares another's score
+    }
+    uint32_t ca = (uint32_t)in[15] + tid, cb = ~ca;
+    for (int it = 0; it < iters; ++it) {
+#pragma unroll
+        for (int c = 0; c < kChains; ++c) {
+            uint32_t s1;
+            asm("prmt.b32 %0, %1, %2, %3;" : "=r"(s1) : "r"(ca), "r"(cb), "r"(sel[c]));
+            const uint32_t e = __viaddmax_s16x2(E[c], ext, HO[c]);
+            const uint32_t to = __vadd2(__viaddmax_s16x2_relu(hod[c], s1, e), open);
+            const uint32_t ho = __viaddmax_s16x2(f[c], open, to);
+            f[c] = __viaddmax_s16x2(f[c], gx, to);
+            hod[c] = HO[c];
+            HO[c] = ho;
+            E[c] = e;
+        }
+        ca += 0x01010101u;  // another column: the scores are not the loop's constants
+        cb += ca;
+    }
+    uint32_t acc = 0;
+#pragma unroll
+    for (int c = 0; c < kChains; ++c) acc ^= HO[c] ^ E[c] ^ f[c] ^ hod[c];
+    out[tid] = (int32_t)acc;
 }
 
 // op: 0 = IADD, 1 = __viaddmax_s32, 2 = __vimax3_s32; 8 independent chains.
@@ -121,6 +159,47 @@ extern "C" int swb_probe_latency(int32_t device, double *cycles_per_op, int32_t 
     cudaFree(din);
     cudaFree(dout);
     cudaFree(dcyc);
+    return cudaGetLastError() == cudaSuccess ? SWB_OK : SWB_ECUDA;
+}
+
+extern "C" int swb_probe_packed_peak(int32_t device, double *cells_per_s, double *elapsed_ms) {
+    using namespace swb;
+    if (cudaSetDevice(device) != cudaSuccess) return SWB_ECUDA;
+    int sms = 0, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int threads = 256, iters = 4096;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, packed_mix_kernel, threads, 0);
+    const int blocks = sms * (per_sm > 0 ? per_sm : 1);
+    // -2, -5, max(-5, -2) in both halves; selectors of two rows' codes; a table word
+    const int32_t hin[16] = {(int32_t)0xFFFEFFFEu, (int32_t)0xFFFBFFFBu, (int32_t)0xFFFEFFFEu, 0x00070007, 0, 0, 0x00010001,
+                             0xC480, 0xD591, 0xE6A2, 0xF7B3, 0xD580, 0xE691, 0xF7A2, 0xC4B3, 0x02020206};
+    int32_t *din = nullptr, *dout = nullptr;
+    if (cudaMalloc(&din, sizeof hin) != cudaSuccess) return SWB_ENOMEM;
+    if (cudaMalloc(&dout, sizeof(int32_t) * (size_t)blocks * threads) != cudaSuccess) {
+        cudaFree(din);
+        return SWB_ENOMEM;
+    }
+    cudaMemcpy(din, hin, sizeof hin, cudaMemcpyHostToDevice);
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    packed_mix_kernel<<<blocks, threads>>>(din, dout, iters / 4);
+    float best = 1e30f;
+    for (int rep = 0; rep < 3; ++rep) {
+        float ms = 0.f;
+        cudaEventRecord(e0);
+        packed_mix_kernel<<<blocks, threads>>>(din, dout, iters);
+        cudaEventRecord(e1);
+        cudaEventSynchronize(e1);
+        cudaEventElapsedTime(&ms, e0, e1);
+        if (ms < best) best = ms;
+    }
+    if (cells_per_s) *cells_per_s = 2.0 * blocks * threads * iters * kChains / (best * 1e-3);
+    if (elapsed_ms) *elapsed_ms = best;
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    cudaFree(din);
+    cudaFree(dout);
     return cudaGetLastError() == cudaSuccess ? SWB_OK : SWB_ECUDA;
 }
 

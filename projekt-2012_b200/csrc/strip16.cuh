@@ -29,10 +29,10 @@
 //     (flooring t at base changes no H >= base, and F and E of the next cell are
 //     at least H + open either way).
 //
-// What bounds it: the ALU pipe, where each packed op (and LOP3, PRMT) issues at
-// 64 lanes per SM and cycle: 6 per row pair (PRMT score, E, t, t + open, H, F')
-// = 12 cycles per warp and sub-partition for 64 cells, against 10.3 for 32 cells
-// of the 32-bit step.
+// What bounds it: the ALU pipe, where each packed op (and LOP3, PRMT) alone issues at
+// 64 lanes per SM and cycle: 6 per row pair (PRMT score, E, t, t + open, H, F'), which
+// together take 10.8 cycles per warp and sub-partition for 64 cells
+// (swb_probe_packed_peak), against 10.3 for 32 cells of the 32-bit step.
 //
 // Best cell.  The step itself does not look for it.  Before each run of 32 steps
 // the warp asks whether any cell of the run could reach the best H known (bottom

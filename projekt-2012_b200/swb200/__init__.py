@@ -171,6 +171,8 @@ def lib():
         L.swb_server_destroy.argtypes = [C.c_void_p]
         L.swb_probe_cell_peak.argtypes = [C.c_int32] + [C.POINTER(C.c_double)] * 5
         L.swb_probe_cell_peak.restype = C.c_int
+        L.swb_probe_packed_peak.argtypes = [C.c_int32] + [C.POINTER(C.c_double)] * 2
+        L.swb_probe_packed_peak.restype = C.c_int
         L.swb_probe_latency.argtypes = [C.c_int32, C.POINTER(C.c_double), C.c_int32]
         L.swb_probe_latency.restype = C.c_int
         L.swb_gap_lists.argtypes = [C.POINTER(Result), C.c_void_p, C.c_int64, C.POINTER(C.c_int64), C.c_void_p,
@@ -559,7 +561,7 @@ def version() -> str:
 
 
 def probe_cell_peak(device: int = 0) -> dict:
-    """Measured peak cell-update rate of the stage-1 per-cell instruction mix
+    """Measured peak cell-update rate of the 32-bit strips' per-cell instruction mix
     (swb_probe_cell_peak) and single-op rates."""
     v = [C.c_double() for _ in range(5)]
     rc = lib().swb_probe_cell_peak(device, *[C.byref(x) for x in v])
@@ -567,6 +569,16 @@ def probe_cell_peak(device: int = 0) -> dict:
         raise SwbError(rc, "probe failed")
     return {"cells_per_s": v[0].value, "iadd_per_s": v[1].value, "viaddmax_per_s": v[2].value,
             "vimax3_per_s": v[3].value, "probe_ms": v[4].value}
+
+
+def probe_packed_peak(device: int = 0) -> dict:
+    """Measured peak cell-update rate of the packed strips' instruction mix
+    (swb_probe_packed_peak)."""
+    v = [C.c_double() for _ in range(2)]
+    rc = lib().swb_probe_packed_peak(device, *[C.byref(x) for x in v])
+    if rc != SWB_OK:
+        raise SwbError(rc, "probe failed")
+    return {"cells_per_s": v[0].value, "probe_ms": v[1].value}
 
 
 def probe_latency(device: int = 0) -> dict:
