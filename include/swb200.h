@@ -68,8 +68,9 @@ typedef struct {
 #define SWB_FLAG_NO_SPECIAL    0x4u  /* stage 1 without special-row checkpoints    */
 /* Test hook of swb_align_pair[_device]: strip 0 never hands its bottom row to
  * strip 1, so strip 1's first wait runs out after wait_limit_ms and the call
- * returns SWB_ETIMEOUT with the context still usable.  Pairs of one strip (at
- * most 448 rows) have no wait and are unaffected. */
+ * returns SWB_ETIMEOUT with the context still usable.  Pairs of one strip (any
+ * of at most 256 rows; strips are up to 1,024 rows high) have no wait and are
+ * unaffected. */
 #define SWB_FLAG_TEST_WITHHOLD 0x80000000u
 /* Test hook of swb_batch_align[_device], and of swb_align_pair[_device] where the
  * traceback recomputes cells of a coarse grid: a pass in packed strips (32-bit
@@ -106,7 +107,8 @@ typedef struct {
 
 typedef struct {
     int32_t  device;                /* CUDA device ordinal                           */
-    uint64_t hbm_budget_bytes;      /* cap on special rows/columns; 0 = 64 GiB      */
+    uint64_t hbm_budget_bytes;      /* cap on special rows/columns, and on what stage 2's
+                                       segments add to them; 0 = 64 GiB            */
     int32_t  special_interval;      /* special-row spacing in rows; 0 = autotune    */
     int32_t  verbose;               /* bit 0: progress lines on stderr; bit 1: record
                                        the stage-1 strip trace (swb_trace_copy)     */
@@ -295,7 +297,9 @@ void swb_batch_result_free(swb_batch_result *res);
  * an HBM budget for their sequences and special rows/columns.  Short requests
  * run in iterations: each iteration batches every admitted short request into
  * one scoring launch plus one batched traceback, and requests that arrive during
- * an iteration join the next one.  Long requests (rows * cols above long_cells)
+ * an iteration join the next one.  An iteration starts at once when some client
+ * waits for every queued short request; else it stays open for requests that are
+ * still coming in, up to 0.1 ms after the newest and 0.5 ms in all.  Long requests (rows * cols above long_cells)
  * run one at a time in a second lane on their own stream.  Their scoring grid
  * leaves reserve_sms SMs for the short iterations, so both lanes' work overlaps
  * on the device.  A request's result (score, end and start cells, alignment,
