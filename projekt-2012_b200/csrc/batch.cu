@@ -143,7 +143,7 @@ __device__ __forceinline__ void batch_body(const BatchArgs &g) {
         init_best(b, g.open);
         int32_t bho = b.ho;
         const int32_t strip = g.unit_strip ? g.unit_strip[u] : u - d.unit0;
-        if (!run_strip<R, TAB, !std::is_same<S, NoStores>::value, false>(v, ring, stage, lane, strip, &b, bho)) {
+        if (!run_strip<R, TAB, !std::is_same<S, NoStores>::value, false, false>(v, ring, stage, lane, strip, &b, bho)) {
             if (lane == 0) {
                 atomicCAS(&g.ctl[1], kErrNone, kErrTimeout);
                 atomicExch(&g.ctl[2], 1);

@@ -57,7 +57,7 @@ namespace swb {
 
 namespace {
 
-template <int R, bool TAB, bool STORES>
+template <int R, bool TAB, bool STORES, bool RAGGED>
 __global__ void __launch_bounds__(kWarps * 32, (R <= 16 ? 4 : 2)) stage1_kernel(Stage1Args a) {
     __shared__ int4 ring_all[kWarps][kRing + kStage];
     const int lane = threadIdx.x & 31;
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kWarps * 32, (R <= 16 ? 4 : 2)) stage1_kernel(
             asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
             a.trace[3 * s + 2] = (int64_t)smid;
         }
-        if (!run_strip<R, TAB, STORES, !STORES>(a, ring, stage, lane, (int32_t)s, &b, bho)) failed = true;
+        if (!run_strip<R, TAB, STORES, !STORES, RAGGED>(a, ring, stage, lane, (int32_t)s, &b, bho)) failed = true;
         if (a.trace && lane == 0) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -283,10 +283,6 @@ struct KernelRef {
     const void *fn = nullptr;
     size_t smem = 0;
 };
-template <int R, bool TAB, bool STORES>
-KernelRef wide_ref() {
-    return {(const void *)stage1_kernel<R, TAB, STORES>, 0};
-}
 template <int R>
 KernelRef packed_ref(int kind) {
     constexpr size_t smem = kWarps * sizeof(WarpMem<R / 2>);
@@ -298,10 +294,15 @@ KernelRef packed_ref(int kind) {
     }
 }
 // (the 32-bit kernels without stores serve borders too)
+template <int R, bool TAB>
+KernelRef wide_ref(int kind) {
+    if (kind == kStores) return {(const void *)stage1_kernel<R, TAB, true, false>, 0};
+    if (kind == kRagged) return {(const void *)stage1_kernel<R, TAB, false, true>, 0};
+    return {(const void *)stage1_kernel<R, TAB, false, false>, 0};
+}
 template <int R>
 KernelRef wide_ref(bool tab, int kind) {
-    if (tab) return kind == kStores ? wide_ref<R, true, true>() : wide_ref<R, true, false>();
-    return kind == kStores ? wide_ref<R, false, true>() : wide_ref<R, false, false>();
+    return tab ? wide_ref<R, true>(kind) : wide_ref<R, false>(kind);
 }
 KernelRef kernel_of(int R, bool tab, int kind, bool packed) {
     switch (R) {
